@@ -226,10 +226,9 @@ int64_t macko_compress_workspace_bytes(int64_t padded_count);
  *   row_indices   output of macko_compress_count for the same `dense`
  *   padded_count  P = ceil(ri[rows]/8)*8
  *   workspace     device scratch of macko_compress_workspace_bytes(P) bytes,
- *                 8-byte aligned; contents undefined afterwards. The fp16 and
- *                 bf16 calls check it and leave it alone (they pack the deltas
- *                 in the same pass, after clearing `deltas` on `stream`); the
- *                 int8 call writes one delta per byte into it and packs after.
+ *                 8-byte aligned. The calls check it and leave it alone
+ *                 (they pack the deltas in the same pass, after clearing
+ *                 `deltas` on `stream`).
  */
 int macko_compress_emit(const void *dense, int64_t rows, int64_t cols,
                         const int32_t *row_indices, int64_t padded_count,
@@ -264,18 +263,12 @@ int macko_compress_emit_int8(const void *dense, int64_t rows, int64_t cols,
  * macko_compress_emit without a workspace argument, for hosts that cannot hand the library any
  * scratch memory: a plug-in running inside an application that has already given every byte of
  * device memory to its own pool, or a code path on which a cudaMalloc (which may stall the whole
- * device) is not acceptable. The one-delta-per-byte scratch of phase 2 lives in an array built into
- * the library instead (16 MiB of device memory per GPU that loads the library, held until the
- * process exits), so padded_count may not exceed macko_compress_static_capacity() = 16 777 216
- * stored elements (a dense 4096x4096 matrix just fits); larger counts are refused with
+ * device) is not acceptable. Phase 2 needs no scratch any more; the limit of the scratch that this
+ * entry point once carried stays: padded_count may not exceed macko_compress_static_capacity() =
+ * 16 777 216 stored elements (a dense 4096x4096 matrix just fits); larger counts are refused with
  * MACKO_ERR_WORKSPACE. Same inputs, outputs and bit-exact result as macko_compress_emit. The
- * function calls no cudaMalloc/cudaFree and no allocating library routine.
- *
- * The first call on each device looks up the device address of the built-in array; make that
- * first call outside any stream capture. All calls on a device share the array and it keeps what
- * the previous call left in it (nothing in it needs clearing between calls), so two calls whose
- * kernels can overlap on the GPU - different streams without an ordering between them - race:
- * order them, or use macko_compress_emit with separate workspaces.
+ * function calls no cudaMalloc/cudaFree and no allocating library routine, may be captured, and
+ * calls on different streams do not share anything.
  *
  * This entry point has no counterpart in the reference.
  */
@@ -289,7 +282,7 @@ int64_t macko_compress_static_capacity(void);
 /*
  * Both emit entry points check every store on the device against padded_count: a call whose row_indices
  * do not belong to the padded_count it passes (a stale P, or a matrix that changed between count and
- * emit) writes nothing outside values[0, P) / the scratch, leaves the outputs incomplete and counts the
+ * emit) writes nothing outside values[0, P) / deltas[0, P/2), leaves the outputs incomplete and counts the
  * warps that had to drop a store in a per-device counter. This call copies that counter to *count
  * (0 = every emit since the last call was complete) and clears it; it synchronises `stream`.
  * The reference over-allocates rows*cols + 8 slots for the same purpose (cpu_compressor.cuh:13-14).

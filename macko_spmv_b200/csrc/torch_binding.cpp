@@ -247,8 +247,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> compress_cuda(const at::Tensor &M
     const int64_t padded = (n + 7) / 8 * 8;
     at::Tensor values = at::empty({padded}, M.options());
     at::Tensor deltas = at::empty({padded / 2}, M.options().dtype(at::kByte));
+    // the emit calls check a workspace and leave it alone: the values buffer, never smaller, stands in for it
     const int64_t ws_bytes = macko_compress_workspace_bytes(padded);
-    at::Tensor ws = at::empty({ws_bytes}, M.options().dtype(at::kByte));
+    const at::Tensor &ws = values;
     if (int8)
         check_status(macko_compress_emit_int8(M.data_ptr(), rows, cols, ri.data_ptr<int32_t>(), padded,
                                               values.data_ptr(), deltas.data_ptr(), ws.data_ptr(), ws_bytes, stream),
