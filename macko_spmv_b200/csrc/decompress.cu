@@ -11,97 +11,139 @@
 namespace macko {
 namespace {
 
-constexpr int kWarps = 8;        // warps (rows in flight) per CTA
-// A step decodes 256 stored elements; consecutive stored elements are at most 16 columns apart, so the
-// columns a step covers (from the end of the previous step) fit 15 + 256 * 16 slots; 7 more for alignment.
-constexpr int kStage = 4128;     // fp16 slots of a warp's staging buffer (a multiple of 8)
-
-// dense[g0 .. g0 + n) = stage[off .. off + n) with 16-byte stores wherever source and destination allow.
-// `stage` index 0 corresponds to global index g0 - off, which is a multiple of 8, so aligned 8-element
-// chunks of the destination are aligned chunks of the buffer. src == nullptr writes zeros.
-__device__ __forceinline__ void flush_span(unsigned short *__restrict__ dense, long long g0, int n, const unsigned short *src,
-                                           int off, bool vec_ok, int lane)
+// Zero the deltas and the 16-bit values of one 8-element unit outside element range [lo, hi).
+__device__ __forceinline__ void keep_elements(uint4 &v, unsigned &w, int lo, int hi)
 {
-    if (n <= 0) return;
-    int head = vec_ok ? min(n, (8 - off) & 7) : n;   // elements before the first aligned chunk
-    for (int i = lane; i < head; i += 32) dense[g0 + i] = src ? src[off + i] : (unsigned short)0;
-    if (!vec_ok) return;
-    const int chunks = (n - head) >> 3;
-    uint4 *dst = reinterpret_cast<uint4 *>(dense + g0 + head);
-    const uint4 *s4 = src ? reinterpret_cast<const uint4 *>(src + off + head) : nullptr;
-    for (int c = lane; c < chunks; c += 32) dst[c] = s4 ? s4[c] : make_uint4(0u, 0u, 0u, 0u);
-    const int done = head + (chunks << 3);
-    for (int i = done + lane; i < n; i += 32) dense[g0 + i] = src ? src[off + i] : (unsigned short)0;
+    const int l = min(max(lo, 0), 8), h = min(max(hi, 0), 8);
+    unsigned m = l >= 8 ? 0u : (0xffffffffu << (4 * l));
+    if (h < 8) m &= ~(0xffffffffu << (4 * h));
+    w &= m;
+    unsigned *vw = reinterpret_cast<unsigned *>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        vw[j] &= (((m >> (8 * j)) & 1u) * 0xffffu) | (((m >> (8 * j + 4)) & 1u) * 0xffff0000u);
 }
 
-// One warp per row. Each step's columns are assembled in the warp's shared-memory buffer (zeros, then the
-// stored elements scattered to their columns) and written out with coalesced 16-byte stores, so the dense
-// matrix is written exactly once and no separate clearing pass is needed.
-__global__ void __launch_bounds__(kWarps * 32)
+constexpr int kWarps = 8;        // warps (rows in flight) per CTA
+constexpr int kWin = 1024;       // fp16 slots of a warp's window of the dense row (a multiple of 256)
+
+// One warp per row, no barrier wider than the warp. The row is assembled window by window in shared memory (zeros,
+// then the stored elements scattered to their columns) and leaves as one bulk copy, which costs the load/store pipe
+// nothing, while the warp clears and fills a second window; every byte of the dense matrix is written exactly once
+// and no clearing pass is needed. Windows start on 128-byte lines of the matrix; the up to 7 slots at either end of a
+// row that share 16 bytes with a neighbouring row go one by one. A step decodes 256 stored elements, 8 per lane: the column
+// offsets of a unit come from byte-wise prefix sums of its deltas (as in the product kernel: byte j of `ce` / `co`
+// is twice the column of element 2j / 2j+1 relative to the unit's base, and the top byte of `co` plus 2 is twice the
+// columns the unit advances), the units' bases from a warp scan. A step that reaches beyond the window stays in
+// registers: what lies inside is stored, the window leaves, and the rest goes to the next one. Pads and everything
+// else that is +-0 stay +0. The loads of the next step are issued before a step is scattered.
+// Bound by the load/store pipe (a 2-byte shared store of 32 elements takes 3.8 passes: random columns, random banks) and
+// close behind it HBM: 11003x4093 at density 0.2 (113 MB) in 21.5 us = 5.2 TB/s, 4096x11008 at 0.5 (146 MB) in 29.3 us
+// = 5.0 TB/s; a CTA per row takes 32.8 and 31.8 us. With the window flushed and cleared by the same 16-byte loads and
+// stores instead of a bulk copy 22.7 and 32.5 us; with six CTAs per SM instead of five 23.3 and 30.3 us.
+__global__ void __launch_bounds__(kWarps * 32, 5)
 decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
                        const int *__restrict__ ri, int rows, int cols, int stored,
                        unsigned short *__restrict__ dense, bool vec_ok)
 {
-    extern __shared__ __align__(16) unsigned short stage_all[];
+    __shared__ __align__(16) unsigned short window_s[kWarps][2][kWin];
     const int lane = threadIdx.x & 31;
-    unsigned short *stage = stage_all + (threadIdx.x >> 5) * kStage;
-    const long long n_warps = (long long)gridDim.x * kWarps;
-    for (long long row = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5); row < rows; row += n_warps) {
-        // offsets clamped into [0, stored]: a corrupt row_indices cannot send loads outside the buffers
-        const int begin = min(max(__ldg(ri + row), 0), stored);
-        const int end = min(__ldg(ri + row + 1), stored);
-        const long long row0 = row * (long long)cols;
-        int col_base = 0;   // (sum of deltas) + (number of elements) of the row before this step
-        int written = 0;    // columns of the row already written
-        for (int pos = begin & ~7; pos < end && written < cols; pos += 256) {
-            const int first = pos + lane * 8;   // first element of the lane's unit
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            unsigned w = 0u;
-            if (first < end) {
-                v = __ldg(values + (first >> 3));
-                w = __ldg(deltas + (first >> 3));
-            }
-            const unsigned short *vh = reinterpret_cast<const unsigned short *>(&v);
-            // columns relative to the lane's start: inclusive delta prefix + index, for elements inside the row
-            int rel[8];
-            int sum = 0;
+    const int row = blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
+    if (row >= rows) return;
+    unsigned short *window = window_s[threadIdx.x >> 5][0], *other = window_s[threadIdx.x >> 5][1];
+    // offsets clamped into [0, stored]: a corrupt row_indices cannot send loads outside the buffers
+    const int begin = min(max(__ldg(ri + row), 0), stored);
+    const int end = min(__ldg(ri + row + 1), stored);
+    auto clear = [&]() {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const bool inside = first + j >= begin && first + j < end;
-                if (inside) sum += (int)((w >> (4 * j)) & 15u) + 1;
-                rel[j] = inside ? sum - 1 : -1;
-            }
-            int inc = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += u;
-            }
-            const int lane_base = col_base + inc - sum;
-            col_base += __shfl_sync(0xffffffffu, inc, 31);
-            // this step delivers columns [written, step_end): the gap since the last step, then its elements
-            const int step_end = min(col_base, cols);
-            const int n = step_end - written;
-            if (n <= 0 || n > kStage - 8) continue;   // nothing new, or deltas that no compressor can produce
-            const long long g0 = row0 + written;
-            const int off = (int)(g0 & 7);
-            uint4 *z = reinterpret_cast<uint4 *>(stage);
-            for (int c = lane; c < (off + n + 7) >> 3; c += 32) z[c] = make_uint4(0u, 0u, 0u, 0u);
+        for (int c = lane; c < kWin / 8; c += 32) reinterpret_cast<uint4 *>(window)[c] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+    };
+    clear();
+    const long long row0 = row * (long long)cols;
+    const int lo = vec_ok ? (int)(row0 & 63) : 0;   // the row takes slots [lo, hi) from the line that holds its start
+    const int hi = lo + cols;
+    unsigned short *out = dense + (row0 - lo);
+    int start = 0;                          // first slot of the window
+    int col2 = 2 * lo - 2 * (begin & 7);    // byte offset in the window of the column in front of the next step
+    auto flush = [&]() {
+        const int a = max(lo, start), b = min(hi, start + kWin);               // the row's slots in this window
+        const int a8 = vec_ok ? (a + 7) & ~7 : b, b8 = vec_ok ? b & ~7 : b;    // the whole 16-byte chunks among them
+        if (a8 < b8) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int col = lane_base + rel[j];
-                if (rel[j] >= 0 && col >= written && col < step_end && (vh[j] & 0x7fffu) != 0u) stage[off + col - written] = vh[j];
+            if (lane == 0) {
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out + a8),
+                             "r"((unsigned)__cvta_generic_to_shared(window + (a8 - start))), "r"(2 * (b8 - a8)) : "memory");
             }
+            if (a + lane < a8) out[a + lane] = window[a + lane - start];
+            if (b8 + lane < b) out[b8 + lane] = window[b8 + lane - start];
+        } else {
             __syncwarp();
-            flush_span(dense, g0, n, stage, off, vec_ok, lane);
-            __syncwarp();
-            written = step_end;
+            for (int e = a + lane; e < b; e += 32) out[e] = window[e - start];
         }
-        flush_span(dense, row0 + written, cols - written, nullptr, (int)((row0 + written) & 7), vec_ok, lane);   // zeros behind the last stored element
+        // the other window is free once its copy has been read
+        if (lane == 0) asm volatile("cp.async.bulk.commit_group; cp.async.bulk.wait_group.read 1;" ::: "memory");
+        unsigned short *t = window;
+        window = other;
+        other = t;
+        start += kWin;
+        col2 -= 2 * kWin;
+        __syncwarp();
+        clear();
+    };
+    auto fetch = [&](int first, uint4 &v, unsigned &w) {
+        v = make_uint4(0u, 0u, 0u, 0u);
+        w = 0u;
+        if (first < end) {
+            v = __ldcs(values + (first >> 3));
+            w = __ldcs(deltas + (first >> 3));
+        }
+    };
+    int first = (begin & ~7) + lane * 8;   // first element of the lane's unit
+    uint4 v;
+    unsigned w;
+    fetch(first, v, w);
+    for (int pos = begin & ~7; pos < end && start < hi; pos += 256, first += 256) {
+        uint4 v_next;
+        unsigned w_next;
+        fetch(first + 256, v_next, w_next);
+        if (first < begin || (first < end && first + 8 > end)) keep_elements(v, w, begin - first, end - first);
+        const unsigned ev = w & 0x0f0f0f0fu, od = (w >> 4) & 0x0f0f0f0fu;
+        const unsigned pe = ev * 0x02020202u + 0x0c080400u, po = od * 0x02020202u;
+        const unsigned ce = po * 256u + pe, co = pe + po + 0x02020202u;
+        const int mine = first < end ? (int)(co >> 24) + 2 : 0;   // twice the columns this unit advances
+        int inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+            asm("{.reg .pred p; .reg .b32 t; shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff; @p add.s32 %0, %0, t;}" : "+r"(inc) : "r"(o));
+        const int total = __shfl_sync(0xffffffffu, inc, 31);
+        int at = col2 + inc - mine;   // byte offset in the window of the unit's base column
+        const unsigned vw[4] = {v.x, v.y, v.z, v.w};
+        for (;;) {
+            const unsigned window_addr = (unsigned)__cvta_generic_to_shared(window);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned be = (unsigned)__dp4a(ce, 1u << (8 * j), (unsigned)at);
+                const unsigned bo = (unsigned)__dp4a(co, 1u << (8 * j), (unsigned)at);
+                // predicated, not branched over; offsets in front of the window (already stored) are huge as unsigned numbers
+                asm volatile("{.reg .pred p, q; .reg .b16 l, h; mov.b32 {l, h}, %4; setp.ne.u32 p, %5, 0; setp.ne.u32 q, %6, 0;"
+                             "setp.lt.and.u32 p, %0, %7, p; setp.lt.and.u32 q, %2, %7, q; @p st.shared.u16 [%1], l; @q st.shared.u16 [%3], h;}"
+                             ::"r"(be), "r"(window_addr + be), "r"(bo), "r"(window_addr + bo), "r"(vw[j]), "r"(vw[j] & 0x7fffu), "r"(vw[j] & 0x7fff0000u),
+                               "n"(2 * kWin) : "memory");
+            }
+            if (col2 + total <= 2 * kWin) break;
+            flush();
+            at -= 2 * kWin;
+            if (start >= hi) break;   // only deltas that no compressor can produce reach beyond the row
+        }
+        col2 += total;
+        v = v_next;
+        w = w_next;
     }
+    while (start < hi) flush();   // the last elements and the zeros behind them
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
-
 
 constexpr int kRowThreads = 256;   // threads of a CTA of the row kernel: 256 units (2048 stored elements) per pass
 
@@ -143,17 +185,8 @@ decompress_row_cta_kernel(const uint4 *__restrict__ values, const unsigned *__re
             if (active) {
                 v = __ldg(values + (first >> 3));
                 w = __ldg(deltas + (first >> 3));
-                const int lo = begin - first, hi = end - first;
-                if (lo > 0 || hi < 8) {   // the unit straddles an end of the row: drop what lies outside
-                    const int l = min(max(lo, 0), 8), h = min(max(hi, 0), 8);
-                    unsigned m = l >= 8 ? 0u : (0xffffffffu << (4 * l));
-                    if (h < 8) m &= ~(0xffffffffu << (4 * h));
-                    w &= m;
-                    unsigned *vw = reinterpret_cast<unsigned *>(&v);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        vw[j] &= (((m >> (8 * j)) & 1u) * 0xffffu) | (((m >> (8 * j + 4)) & 1u) * 0xffff0000u);
-                }
+                // a unit that straddles an end of the row: drop what lies outside
+                if (first < begin || first + 8 > end) keep_elements(v, w, begin - first, end - first);
             }
             const unsigned ev = w & 0x0f0f0f0fu, od = (w >> 4) & 0x0f0f0f0fu;
             const unsigned pe = ev * 0x02020202u + 0x0c080400u, po = od * 0x02020202u;
@@ -232,28 +265,30 @@ extern "C" int macko_decompress_fp16(const void *values, const void *deltas, con
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t row_smem = ((size_t)cols + 16) * sizeof(unsigned short);
     cudaError_t e;
-    if (row_smem + 1024 <= (size_t)dev->max_smem_optin) {
+    // CTAs of the kernel that holds a whole row in shared memory (0: the row does not fit)
+    long long per_sm = (long long)((size_t)dev->max_smem_optin / (row_smem + 1024));
+    if (per_sm > 2048 / kRowThreads) per_sm = 2048 / kRowThreads;
+    // A CTA per row where a warp per row would leave three quarters of the warps idle that the CTAs bring, or where rows
+    // are so long that the last wave of the warp kernel (40 rows per SM at a time) weighs more than the CTA kernel's
+    // barriers. Measured (B200, us, CTA per row / warp per row, density 0.5): 512x49152 36.6 / 62.8, 1024x16384
+    // 16.9 / 24.1, 1600x8192 12.6 / 14.7, 8192x11000 65.5 / 71.5, 3000x20000 48.9 / 51.3; 4096x11008 in front of a GEMM
+    // 31.8 / 29.3, 2048x32000 66.2 / 61.8, 2960x8192 20.9 / 18.8, 4096x4096 18.9 / 13.2, 11008x4096 44.8 / 31.7,
+    // 32000x512 71.3 / 18.9.
+    const bool few_rows = rows < 2LL * dev->sm_count * per_sm;
+    const bool long_rows = per_sm >= 4 && (cols >= 16384 || (cols >= 10240 && rows > 40LL * dev->sm_count));
+    if (per_sm > 0 && (few_rows || long_rows)) {
         // a CTA per row with the row in shared memory; as many CTAs per SM as threads and shared memory allow
         if (row_smem > 48 * 1024) {
             e = cudaFuncSetAttribute(decompress_row_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem);
             if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         }
-        long long per_sm = (long long)((size_t)dev->max_smem_optin / (row_smem + 1024));
-        if (per_sm > 2048 / kRowThreads) per_sm = 2048 / kRowThreads;
         long long grid = (long long)dev->sm_count * per_sm;
         if (grid > rows) grid = rows;
         decompress_row_cta_kernel<<<(unsigned)grid, kRowThreads, row_smem, s>>>(
             static_cast<const uint4 *>(values), static_cast<const unsigned *>(deltas), row_indices, (int)rows, (int)cols,
             (int)padded_count, static_cast<unsigned short *>(dense), aligned(dense, 16));
     } else {
-        // rows too wide for shared memory: a warp per row with a window of the row
-        const int smem = kWarps * kStage * (int)sizeof(unsigned short);
-        e = cudaFuncSetAttribute(decompress_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-        long long grid = (rows + kWarps - 1) / kWarps;
-        const long long cap = (long long)dev->sm_count * 3;   // three CTAs per SM fit by shared memory
-        if (grid > cap) grid = cap;
-        decompress_rows_kernel<<<(unsigned)grid, kWarps * 32, smem, s>>>(
+        decompress_rows_kernel<<<(unsigned)((rows + kWarps - 1) / kWarps), kWarps * 32, 0, s>>>(
             static_cast<const uint4 *>(values), static_cast<const unsigned *>(deltas), row_indices, (int)rows, (int)cols,
             (int)padded_count, static_cast<unsigned short *>(dense), aligned(dense, 16));
     }

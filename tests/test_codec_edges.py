@@ -1,12 +1,14 @@
-"""GPU tests of the compressor at the sizes where its kernels change what they do, bit for bit against the oracle: steps of
-256 (count) and 512 (emit) columns, output rings of 512 waiting slots, pad batches of 512 (runs of more than 8192
-zeros), rows at every offset from a 16-byte boundary, the row scan's 16384 entries."""
+"""GPU tests of the compressor and the decompressor at the sizes where their kernels change what they do, bit for bit
+against the oracle: steps of 256 (count) and 512 (emit) columns, output rings of 512 waiting slots, pad batches of 512
+(runs of more than 8192 zeros), rows at every offset from a 16-byte boundary, the row scan's 16384 entries; and for the
+decompressor windows of 1024 columns, steps that reach over several windows, and both of its kernels."""
 import numpy as np
 import pytest
 import torch
 
 import oracle
 import macko_spmv_b200 as macko_spmv
+from macko_spmv_b200 import cabi
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +62,22 @@ def test_row_scan_of_many_rows(rows):
     m[::3, 1] = 1.0
     m[5::7, 2] = 2.0
     _check_compress(m, m.to(DEV))
+
+
+# 2400 rows and more, or more columns than shared memory holds: a warp per row; fewer rows: a CTA per row
+@pytest.mark.parametrize("density", [0.02, 0.5, 1.0])
+@pytest.mark.parametrize("rows,cols", [(2400, 1), (2400, 33), (2401, 1023), (2400, 1024), (2400, 1025), (2401, 2111), (2370, 4096),
+                                       (40, 1025), (40, 4099), (4, 130003)])
+def test_decompress_edges(rows, cols, density):
+    m = _matrix(rows, cols, density, rows + cols)
+    comp = macko_spmv.compress(m.to(DEV))
+    exp = oracle.decompress((_u16(comp[0]), comp[1].cpu().numpy(), comp[2].cpu().numpy(), rows, cols))
+    assert np.array_equal(_u16(macko_spmv.decompress(comp)).reshape(rows, cols), exp)
+    # a destination two bytes behind a 16-byte boundary, with guards on both sides
+    lib = cabi.load()
+    out = torch.full((rows * cols + 64,), 0x5A5A, dtype=torch.int16, device=DEV)
+    cabi.check(lib, lib.macko_decompress_fp16(comp[0].data_ptr(), comp[1].data_ptr(), comp[2].data_ptr(), rows, cols, comp[0].numel(),
+                                              out.data_ptr() + 2, torch.cuda.current_stream().cuda_stream))
+    got = out.cpu().numpy().view(np.uint16)
+    assert np.array_equal(got[1 : 1 + rows * cols].reshape(rows, cols), exp)
+    assert got[0] == 0x5A5A and (got[1 + rows * cols :] == 0x5A5A).all()
