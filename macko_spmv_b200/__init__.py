@@ -16,6 +16,7 @@ Use ``import macko_spmv_b200 as macko_spmv`` to switch an existing program over.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 import torch
@@ -41,10 +42,14 @@ def _load_native():
             )
     core = ctypes.CDLL(_CORE_PATH, mode=ctypes.RTLD_GLOBAL)
     torch.ops.load_library(_OPS_PATH)
-    return core
+    # the same library as a Python module: `multiply` for calls that only want the product
+    spec = importlib.util.spec_from_file_location(__name__ + "._torch_ops", _OPS_PATH)
+    direct = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(direct)
+    return core, direct
 
 
-_core = _load_native()
+_core, _direct = _load_native()
 _core.macko_version.restype = ctypes.c_int
 _core.macko_last_error.restype = ctypes.c_char_p
 _core.macko_status_string.restype = ctypes.c_char_p
@@ -169,6 +174,11 @@ class FrozenMatrix(tuple):
         return self
 
 
+_direct.set_frozen_type(FrozenMatrix)
+_direct_multiply = _direct.multiply
+_is_compiling = torch.compiler.is_compiling
+
+
 def freeze(compressed_M, plan="auto", segment_elements=0):
     """Declare a compressed CUDA matrix immutable and, if it pays, build its launch plan.
 
@@ -194,6 +204,10 @@ def multiply(compressed_M, V, out=None):
 
     `out` (not in the reference): a contiguous CUDA vector of M_rows elements that receives y, for callers
     that keep their results in one buffer; without it a new tensor is returned, as in the reference."""
+    if out is None and not _is_compiling():
+        y = _direct_multiply(compressed_M, V)   # None: not a plain call, or not a valid one
+        if y is not None:
+            return y
     assert compressed_M[0].is_cuda
     assert compressed_M[1].is_cuda
     assert compressed_M[2].is_cuda

@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
@@ -85,7 +86,7 @@ def build_torch_ops(force: bool = False, verbose: bool = False) -> str:
     import torch
     from torch.utils import cpp_extension as ce
 
-    inc = []
+    inc = ["-isystem", sysconfig.get_paths()["include"]]
     for p in ce.include_paths("cuda"):
         inc += ["-isystem", p]
     lib_dirs = ce.library_paths("cuda")
@@ -94,7 +95,7 @@ def build_torch_ops(force: bool = False, verbose: bool = False) -> str:
         "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
         "-DTORCH_API_INCLUDE_EXTENSION_H", "-I", INCLUDE, *inc, src, "-o", LIB_TORCH,
         *[f"-L{d}" for d in lib_dirs], "-L", PKG_DIR,
-        "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-l:libmacko_b200.so",
+        "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-l:libmacko_b200.so",
         "-Wl,-rpath,$ORIGIN", *[f"-Wl,-rpath,{d}" for d in lib_dirs],
     ]
     _run(cmd, verbose)
