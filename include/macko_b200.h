@@ -134,7 +134,7 @@ int macko_spmv_shape(int64_t rows, int64_t cols, int64_t padded_count, int sm_co
  * Planned launch, for matrices whose rows are very long or very uneven. A plan is side metadata built once
  * per matrix on the GPU from row_indices and deltas; the three MACKO buffers are not modified and stay what
  * the reference format defines. It cuts every row into virtual rows of at most `segment_elements` stored
- * elements (0 = default 1536; a multiple of 256, at most 3840), records for each where the decode has to
+ * elements (0 = by the size of the matrix, 512 to 1536; a multiple of 256, at most 3840), records for each where the decode has to
  * resume (the column sum in front of the segment), sorts them by length and deals them to the warps longest
  * first, so that every warp gets about the same number of stored elements whatever the row lengths are. The
  * segments of a cut row leave fp32 partial sums inside the plan; a second, tiny kernel enqueued right behind
@@ -148,7 +148,7 @@ int macko_spmv_shape(int64_t rows, int64_t cols, int64_t padded_count, int sm_co
  *                          cols must fit shared memory (about 116 000). Calls that use one plan must not
  *                          overlap on the GPU (they share the partial sums inside it).
  * info->recommended is 1 when the row statistics say that the planned launch should beat macko_spmv_fp16
- * (rows cut into several segments and much longer than the average row).
+ * (rows cut into several segments and much longer than the average row, in a matrix of some size).
  * No counterpart in the reference: its kernel gives every row one warp (kernels_torch_launchers.cuh:15-16),
  * which is what makes uneven rows slow there.
  */

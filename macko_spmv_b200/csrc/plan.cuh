@@ -17,7 +17,7 @@ namespace macko {
 
 constexpr int kPlanLenBits = 12;                         // a virtual row holds fewer than 4096 stored elements
 constexpr int kPlanMaxSegment = 3840;                    // largest segment length (a multiple of 256)
-constexpr int kPlanDefaultSegment = 1536;
+constexpr long long kPlanGroups = 148LL * 32 * 4;        // rows that a planned launch walks at once on a B200: 4 per resident warp
 constexpr int kPlanBuckets = 64;                         // length classes: 64-element sub-steps spanned, 0..60
 constexpr unsigned kPlanPartialBit = 0x80000000u;        // destination word: a partial-sum slot, not a row of y
 
@@ -63,6 +63,26 @@ inline PlanLayout plan_layout(long long rows, long long padded, int seg)
     l.total = at;
     return l;
 }
+
+// Segment length where the caller names none. A group of lanes gets a share of padded / kPlanGroups elements: a
+// segment a little longer than the share leaves one long segment per group and the short rows to even the ends out,
+// a much longer one leaves groups without work while others walk it, a much shorter one costs a hand-over and a
+// partial sum each time. Above about 1088 elements per group a fixed 1536 is as good as any choice. Skewed matrices of
+// mean density 0.2 (B200, graph of products, us, this rule / always 1536): 4879x7688 (share 474) 13.8 / 19.5,
+// 12000x4096 (617) 14.5 / 19.9, 16000x4096 (822) 16.8 / 20.7, 4096x16384 (858) 20.9 / 23.7, 9000x9000 (1032)
+// 20.6 / 22.5.
+inline int plan_default_segment(long long padded)
+{
+    const long long share = padded / kPlanGroups;
+    if (share > 1088) return 1536;
+    const long long seg = (share + 16 + 255) / 256 * 256;
+    return (int)(seg < 512 ? 512 : seg);
+}
+
+// Fewest elements per group for which a plan is recommended: below, the launch is over before the balance pays for the
+// hand-overs and the second kernel. Default launch / plan (us): 5504x3200 (share 221) 8.4 / 10.5, 2500x9000 (287)
+// 11.7 / 13.2, 3000x9000 (346) 10.7 / 12.8; 7436x4034 (382) 11.4 / 11.0, 6000x6000 (458) 14.3 / 13.0.
+constexpr long long kPlanMinShare = 365;
 
 // Length class of a virtual row: 64-element sub-steps between the unit its first element sits in and its end.
 __host__ __device__ inline int plan_length_class(int begin, int len)

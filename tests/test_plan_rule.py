@@ -1,0 +1,40 @@
+"""The segment length and the recommendation that a plan gets when the caller names none, at the lines of the rule, and
+the product through such a plan against float64."""
+import pytest
+import torch
+
+import macko_spmv_b200 as macko_spmv
+from macko_spmv_b200 import cabi
+
+DEV = "cuda:0"
+GROUPS = 148 * 32 * 4
+
+
+def test_plan_bytes_follow_the_default_segment():
+    lib = cabi.load()
+    for share, seg in ((0, 512), (496, 512), (497, 768), (752, 768), (1008, 1024), (1009, 1280), (1088, 1280), (1089, 1536), (9000, 1536)):
+        padded = share * GROUPS
+        assert lib.macko_spmv_plan_bytes(5000, 8192, padded, 0) == lib.macko_spmv_plan_bytes(5000, 8192, padded, seg), share
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,dense_rows,cols,planned,seg", [
+    (900, 200, 30000, False, 512),     # 317 elements per group: too small for a plan
+    (900, 240, 30000, True, 512),      # 380
+    (2000, 400, 30000, True, 768),     # 634
+    (900, 800, 30000, False, 1536),    # 1267, but no row is far longer than the mean
+    (4000, 640, 30000, True, 1280),    # 1014
+])
+def test_default_plans(rows, dense_rows, cols, planned, seg):
+    M = torch.zeros(rows, cols, dtype=torch.float16, device=DEV)
+    M[:dense_rows] = torch.randn(dense_rows, cols, device=DEV).half()
+    M = M[torch.randperm(rows, device=DEV)].contiguous()
+    comp = macko_spmv.compress(M)
+    frozen = macko_spmv.freeze(comp)
+    assert (frozen.plan is not None) == planned and frozen.plan_meta[1] == seg
+    x = torch.randn(cols, device=DEV).half()
+    for fz in (frozen, macko_spmv.freeze(comp, plan=True)):
+        y = macko_spmv.multiply(fz, x).double()
+        ref, l1 = M.double() @ x.double(), M.double().abs() @ x.double().abs()
+        # half a unit in the last place of y, and 2^-23 of the absolute sum per addition of the fp32 sums
+        assert bool(((y - ref).abs() <= 2.0 ** -11 * ref.abs() + cols * 2.0 ** -23 * l1 + 2.0 ** -24).all())
