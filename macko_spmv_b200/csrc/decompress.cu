@@ -268,14 +268,19 @@ extern "C" int macko_decompress_fp16(const void *values, const void *deltas, con
     // CTAs of the kernel that holds a whole row in shared memory (0: the row does not fit)
     long long per_sm = (long long)((size_t)dev->max_smem_optin / (row_smem + 1024));
     if (per_sm > 2048 / kRowThreads) per_sm = 2048 / kRowThreads;
-    // A CTA per row where a warp per row would leave three quarters of the warps idle that the CTAs bring, or where rows
-    // are so long that the last wave of the warp kernel (40 rows per SM at a time) weighs more than the CTA kernel's
-    // barriers. Measured (B200, us, CTA per row / warp per row, density 0.5): 512x49152 36.6 / 62.8, 1024x16384
-    // 16.9 / 24.1, 1600x8192 12.6 / 14.7, 8192x11000 65.5 / 71.5, 3000x20000 48.9 / 51.3; 4096x11008 in front of a GEMM
-    // 31.8 / 29.3, 2048x32000 66.2 / 61.8, 2960x8192 20.9 / 18.8, 4096x4096 18.9 / 13.2, 11008x4096 44.8 / 31.7,
-    // 32000x512 71.3 / 18.9.
+    // A CTA per row where a warp per row would leave three quarters of the warps idle that the CTAs bring; and for long rows,
+    // of which a warp that starts late holds up the end, wherever that measured faster: a second wave of the warp
+    // kernel (40 rows per SM at a time) that is mostly empty, few rows, or little to decode. Measured (B200, us, CTA per
+    // row / warp per row): few rows 1024x16384 d = 0.5 16.9 / 24.1, 512x49152 36.6 / 62.8; second wave 6600x10000 d = 0.3
+    // 39.6 / 48.4, 8000x12000 56.5 / 61.3, 6600x8192 36.3 / 39.0; little to decode 5200x10000 d = 0.1 24.9 / 27.1, 3600x15000
+    // 25.1 / 28.3. On the other side of the lines: 4400x8192 d = 0.6 33.1 / 27.0, 6600x5000 33.0 / 27.1, 10000x8192
+    // 69.6 / 60.4, 4400x10000 d = 0.3 28.8 / 25.4, 4096x4096 d = 0.5 18.9 / 13.2, 11008x4096 44.8 / 31.7.
+    const long long at_once = 40LL * dev->sm_count;
     const bool few_rows = rows < 2LL * dev->sm_count * per_sm;
-    const bool long_rows = per_sm >= 4 && (cols >= 16384 || (cols >= 10240 && rows > 40LL * dev->sm_count));
+    const bool late_wave = rows > at_once && (rows + at_once - 1) / at_once * at_once * 100 > 135 * rows;
+    const bool sparse = 4 * padded_count < rows * cols;
+    const bool long_rows = per_sm >= 4 && (cols >= 16384 || (cols >= 8192 && late_wave) || (cols >= 9216 && sparse) ||
+                                           (cols >= 9216 && rows < 18LL * dev->sm_count) || (cols >= 10240 && rows < 27LL * dev->sm_count));
     if (per_sm > 0 && (few_rows || long_rows)) {
         // a CTA per row with the row in shared memory; as many CTAs per SM as threads and shared memory allow
         if (row_smem > 48 * 1024) {
