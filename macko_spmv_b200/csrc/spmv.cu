@@ -941,7 +941,9 @@ int launch_l(int L, int D, const void *values, const void *deltas, const int32_t
 //     conflicts, the resource the kernel is bound by) and shorten the cross-lane scan, so the smallest L wins
 //     that still (a) gives at least ~0.55 of the resident warps a block of rows and (b) walks a row in at most
 //     ~64 sub-steps (a row is a serial chain of sub-steps; 16 sub-steps for very wide matrices, where a full
-//     warp per row measured better);
+//     warp per row measured better; 96 for two rows per warp when every warp holds one such block only: 5504x11008
+//     d = 0.9 32.0 us against 38.2 with a warp per row, 6000x10000 31.3 / 36.0, 6784x13312 d = 0.82 40.9 / 44.6,
+//     8000x16384 d = 0.5 38.6 / 39.5; with more blocks than warps 11008x11008 d = 0.9 66.6 / 61.3);
 //   * rows shorter than half a sub-step shrink the group further;
 //   * six units in flight once a row holds more than three sub-steps, four above one, else two.
 struct Shape { int L, D; };
@@ -952,7 +954,9 @@ Shape choose_shape(long long rows, long long cols, long long padded, int residen
     int L = 32;
     for (int cand = 8; cand < 32; cand <<= 1) {
         const bool enough_blocks = rows * cand * 100 >= 55LL * 32 * resident_warps;
-        const bool short_chain = avg_row <= chain * kGroup * cand;
+        // where a warp holds one block of two rows (no warp holds two), half as long a chain again still pays
+        const long long steps = (cand == 16 && chain == 64 && rows * cand <= 32LL * resident_warps) ? 96 : chain;
+        const bool short_chain = avg_row <= steps * kGroup * cand;
         if (enough_blocks && short_chain) { L = cand; break; }
     }
     while (L > 4 && avg_row < (long long)L * kGroup / 2) L >>= 1;
