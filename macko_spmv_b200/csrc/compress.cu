@@ -199,13 +199,14 @@ count_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows,
 // A warp walks its row, 16 columns per lane and step. What a step stores is appended to a ring in shared memory,
 // one 32-bit entry per stored element (value bits, column mod 16 << 16) at ring slot (output slot mod 1024), so that
 // an element costs one store and the ring never moves. The delta of an element is (column - column of the stored
-// element in front of it - 1) mod 16, for pads as well, and is formed for 8 elements at once when they leave. Whenever 512 slots are waiting, each lane takes two groups of
-// 8: the values leave as one vector store, their 8 deltas packed into one 32-bit store. The first and the last
-// group of a row may be shared with the neighbouring rows (rows start at arbitrary slots): their values leave
-// one by one and their nibbles are merged into the word with atomicOr, which is why the caller clears `deltas`
-// before the launch. Pads: only a lane's first non-zero of a step can have pads in front of it (later ones are
-// less than 16 columns apart). The run in front of the first non-zero of the whole step can be as long as the row
-// and is written by the warp together, 512 pads at a time; the others (at most 31 per step) by their lane. The warp of the last row also clears values[n, P).
+// element in front of it - 1) mod 16, for pads as well, and is formed for 8 elements at once when they leave.
+// Whenever 512 slots are waiting, each lane takes two groups of 8: the values leave as one vector store, their 8
+// deltas packed into one 32-bit store. The first and the last group of a row may be shared with the neighbouring rows
+// (rows start at arbitrary slots): their values leave one by one and their nibbles are merged into the word with
+// atomicOr, which is why the caller clears `deltas` before the launch. Pads: only a lane's first non-zero of a step can
+// have pads in front of it (later ones are less than 16 columns apart). The run in front of the first non-zero of the
+// whole step can be as long as the row and is written by the warp together, 512 pads at a time; the others (at most 31
+// per step) by their lane. The warp of the last row also clears values[n, P).
 // Bound by instruction issue (70 % of the slots at 32 warps per SM): 11008x4096 at density 0.5 takes 41.5 us (146 MB)
 // with 31.7 M warp instructions, against 66 us and 58 M with 8 columns per lane, separate 2-byte and 1-byte ring stores
 // and the deltas counted element by element. Five CTAs per SM instead of four cost registers that spill (45.9 us).
