@@ -41,6 +41,8 @@ constexpr int kWin = 1024;       // fp16 slots of a warp's window of the dense r
 // close behind it HBM: 11003x4093 at density 0.2 (113 MB) in 21.5 us = 5.2 TB/s, 4096x11008 at 0.5 (146 MB) in 29.3 us
 // = 5.0 TB/s; a CTA per row takes 32.8 and 31.8 us. With the window flushed and cleared by the same 16-byte loads and
 // stores instead of a bulk copy 22.7 and 32.5 us; with six CTAs per SM instead of five 23.3 and 30.3 us.
+// Element positions are unsigned in both kernels: a walk looks up to 2048 elements ahead of a count that may come close
+// to 2^31, where a signed position turns negative and passes for one inside the row.
 __global__ void __launch_bounds__(kWarps * 32, 5)
 decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
                        const int *__restrict__ ri, int rows, int cols, int stored,
@@ -52,8 +54,8 @@ decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restr
     if (row >= rows) return;
     unsigned short *window = window_s[threadIdx.x >> 5][0], *other = window_s[threadIdx.x >> 5][1];
     // offsets clamped into [0, stored]: a corrupt row_indices cannot send loads outside the buffers
-    const int begin = min(max(__ldg(ri + row), 0), stored);
-    const int end = min(__ldg(ri + row + 1), stored);
+    const unsigned begin = (unsigned)min(max(__ldg(ri + row), 0), stored);
+    const unsigned end = (unsigned)min(max(__ldg(ri + row + 1), 0), stored);
     auto clear = [&]() {
 #pragma unroll
         for (int c = lane; c < kWin / 8; c += 32) reinterpret_cast<uint4 *>(window)[c] = make_uint4(0u, 0u, 0u, 0u);
@@ -65,7 +67,7 @@ decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restr
     const int hi = lo + cols;
     unsigned short *out = dense + (row0 - lo);
     int start = 0;                          // first slot of the window
-    int col2 = 2 * lo - 2 * (begin & 7);    // byte offset in the window of the column in front of the next step
+    int col2 = 2 * lo - 2 * (int)(begin & 7u);    // byte offset in the window of the column in front of the next step
     auto flush = [&]() {
         const int a = max(lo, start), b = min(hi, start + kWin);               // the row's slots in this window
         const int a8 = vec_ok ? (a + 7) & ~7 : b, b8 = vec_ok ? b & ~7 : b;    // the whole 16-byte chunks among them
@@ -92,7 +94,7 @@ decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restr
         __syncwarp();
         clear();
     };
-    auto fetch = [&](int first, uint4 &v, unsigned &w) {
+    auto fetch = [&](unsigned first, uint4 &v, unsigned &w) {
         v = make_uint4(0u, 0u, 0u, 0u);
         w = 0u;
         if (first < end) {
@@ -100,15 +102,15 @@ decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restr
             w = __ldcs(deltas + (first >> 3));
         }
     };
-    int first = (begin & ~7) + lane * 8;   // first element of the lane's unit
+    unsigned first = (begin & ~7u) + (unsigned)(lane * 8);   // first element of the lane's unit
     uint4 v;
     unsigned w;
     fetch(first, v, w);
-    for (int pos = begin & ~7; pos < end && start < hi; pos += 256, first += 256) {
+    for (unsigned pos = begin & ~7u; pos < end && start < hi; pos += 256u, first += 256u) {
         uint4 v_next;
         unsigned w_next;
-        fetch(first + 256, v_next, w_next);
-        if (first < begin || (first < end && first + 8 > end)) keep_elements(v, w, begin - first, end - first);
+        fetch(first + 256u, v_next, w_next);
+        if (first < begin || (first < end && first + 8u > end)) keep_elements(v, w, (int)(begin - first), (int)(end - first));
         const unsigned ev = w & 0x0f0f0f0fu, od = (w >> 4) & 0x0f0f0f0fu;
         const unsigned pe = ev * 0x02020202u + 0x0c080400u, po = od * 0x02020202u;
         const unsigned ce = po * 256u + pe, co = pe + po + 0x02020202u;
@@ -169,16 +171,16 @@ decompress_row_cta_kernel(const uint4 *__restrict__ values, const unsigned *__re
     const unsigned row_bytes = 2u * (unsigned)cols;
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
         // offsets clamped into [0, stored]: a corrupt row_indices cannot send loads outside the buffers
-        const int begin = min(max(__ldg(ri + row), 0), stored);
-        const int end = min(__ldg(ri + row + 1), stored);
+        const unsigned begin = (unsigned)min(max(__ldg(ri + row), 0), stored);
+        const unsigned end = (unsigned)min(max(__ldg(ri + row + 1), 0), stored);
         const long long row0 = row * (long long)cols;
         const int off = vec_ok ? (int)(row0 & 7) : 0;
         unsigned char *base = reinterpret_cast<unsigned char *>(rowbuf + off);
         // twice the column in front of the unit that holds `begin`: its leading elements belong to the row before
-        int col2 = -2 * (begin & 7);
+        int col2 = -2 * (int)(begin & 7u);
         int parity = 0;
-        for (int pos = begin & ~7; pos < end; pos += kRowThreads * 8, parity ^= 1) {
-            const int first = pos + tid * 8;
+        for (unsigned pos = begin & ~7u; pos < end; pos += kRowThreads * 8u, parity ^= 1) {
+            const unsigned first = pos + (unsigned)(tid * 8);
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             unsigned w = 0u;
             const bool active = first < end;
@@ -186,7 +188,7 @@ decompress_row_cta_kernel(const uint4 *__restrict__ values, const unsigned *__re
                 v = __ldg(values + (first >> 3));
                 w = __ldg(deltas + (first >> 3));
                 // a unit that straddles an end of the row: drop what lies outside
-                if (first < begin || first + 8 > end) keep_elements(v, w, begin - first, end - first);
+                if (first < begin || first + 8u > end) keep_elements(v, w, (int)(begin - first), (int)(end - first));
             }
             const unsigned ev = w & 0x0f0f0f0fu, od = (w >> 4) & 0x0f0f0f0fu;
             const unsigned pe = ev * 0x02020202u + 0x0c080400u, po = od * 0x02020202u;
