@@ -210,30 +210,32 @@ count_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows,
 // Bound by instruction issue (70 % of the slots at 32 warps per SM): 11008x4096 at density 0.5 takes 41.5 us (146 MB)
 // with 31.7 M warp instructions, against 66 us and 58 M with 8 columns per lane, separate 2-byte and 1-byte ring stores
 // and the deltas counted element by element. Five CTAs per SM instead of four cost registers that spill (45.9 us).
+// Output slots are unsigned: with a padded count close to 2^31 the slots that a row counts up to (row_indices that do not
+// belong to the matrix) and the last step of the clearing loop lie beyond it, and are refused there, not taken for negative ones.
 constexpr int kEmitCols = 16;   // columns per lane and step: a warp takes 512 columns
 constexpr int kRing = 1024;     // slots; a power of two. At most 511 wait, and a step or a batch of pads adds at most 512.
 constexpr int kFlush = 512;     // slots that leave together: two groups of 8 per lane
 
 struct EmitRing {
-    unsigned *e;    // the ring: value | (column mod 16) << 16
-    int out;        // next output slot (warp-uniform)
-    int flushed;    // output slots below this have left; a multiple of 8 (warp-uniform)
-    int own_lo;     // first output slot that belongs to this row
+    unsigned *e;        // the ring: value | (column mod 16) << 16
+    unsigned out;       // next output slot (warp-uniform)
+    unsigned flushed;   // output slots below this have left; a multiple of 8 (warp-uniform)
+    unsigned own_lo;    // first output slot that belongs to this row
     bool refused;
 };
 
 // Writes out slots [r.flushed, r.flushed + n), n <= 512, a group of 8 per lane at a time; n % 8 != 0 only for the last ones of a row.
 template <bool I8>
 __device__ __forceinline__ void ring_flush(EmitRing &r, typename Raw<I8>::Element *__restrict__ values,
-                                           unsigned *__restrict__ deltas32, int n, int limit, bool vec_v, int lane)
+                                           unsigned *__restrict__ deltas32, unsigned n, unsigned limit, bool vec_v, int lane)
 {
     __syncwarp();
-    for (int at = 8 * lane; at < n; at += 256) {
-        const int slot0 = r.flushed + at;
-        const int lo = max(r.own_lo - slot0, 0), hi = min(n - at, 8);   // the entries of the group that are this row's
+    for (unsigned at = 8u * (unsigned)lane; at < n; at += 256u) {
+        const unsigned slot0 = r.flushed + at;
+        const int lo = max((int)(r.own_lo - slot0), 0), hi = (int)min(n - at, 8u);   // the entries of the group that are this row's
         const uint4 a = *reinterpret_cast<const uint4 *>(r.e + (slot0 & (kRing - 1)));
         const uint4 b = *reinterpret_cast<const uint4 *>(r.e + (slot0 & (kRing - 1)) + 4);
-        const unsigned before = r.e[(slot0 - 1) & (kRing - 1)];
+        const unsigned before = r.e[(slot0 - 1u) & (kRing - 1)];
         const unsigned e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         unsigned col[2];   // 4 nibbles each: (column mod 16) of the entries
 #pragma unroll
@@ -245,7 +247,7 @@ __device__ __forceinline__ void ring_flush(EmitRing &r, typename Raw<I8>::Elemen
         // nibble-wise now - previous - 1 = now + ~previous (ring entries of another row hold anything, and are masked out)
         const unsigned not_prev = ~((now << 4) | ((before >> 16) & 15u));
         const unsigned packed = ((now & 0x77777777u) + (not_prev & 0x77777777u)) ^ ((now ^ not_prev) & 0x88888888u);
-        if (lo <= 0 && hi == 8 && slot0 + 8 <= limit) {
+        if (lo <= 0 && hi == 8 && slot0 + 8u <= limit) {
             if constexpr (I8) {
                 uint2 o;
                 o.x = __byte_perm(__byte_perm(e[0], e[1], 0x0040), __byte_perm(e[2], e[3], 0x0040), 0x5410);
@@ -273,7 +275,7 @@ __device__ __forceinline__ void ring_flush(EmitRing &r, typename Raw<I8>::Elemen
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 if (j >= lo && j < hi) {
-                    if (slot0 + j < limit) {
+                    if (slot0 + (unsigned)j < limit) {
                         values[slot0 + j] = (typename Raw<I8>::Element)e[j];
                     } else {
                         mask &= ~(0xfu << (4 * j));
@@ -295,7 +297,7 @@ template <bool I8>
 __global__ void __launch_bounds__(kThreads, 4)
 emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, int cols, bool vec_ok,
                  const int *__restrict__ row_indices, typename Raw<I8>::Element *__restrict__ values,
-                 unsigned *__restrict__ deltas32, int limit, unsigned nan_add, bool vec_v)
+                 unsigned *__restrict__ deltas32, int slots, unsigned nan_add, bool vec_v)
 {
     __shared__ __align__(16) unsigned ring_s[(kWarpsPerCta + 1) * kRing];
     const int lane = threadIdx.x & 31;
@@ -313,13 +315,14 @@ emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, 
     const unsigned ring_all = (unsigned)__cvta_generic_to_shared(ring_s);
     const unsigned ring_base = ((ring_all + 4u * kRing - 1u) & ~(4u * kRing - 1u)) + (threadIdx.x >> 5) * 4u * kRing;
     ring.e = ring_s + ((ring_base - ring_all) >> 2);
-    const int out0 = min(max(row_indices[row], 0), limit);   // a corrupt offset cannot leave the buffers
+    const unsigned limit = (unsigned)slots;
+    const unsigned out0 = (unsigned)min(max(row_indices[row], 0), slots);   // a corrupt offset cannot leave the buffers
     ring.out = out0;
-    ring.flushed = out0 & ~7;
+    ring.flushed = out0 & ~7u;
     ring.own_lo = out0;
-    ring.refused = row_indices[row] != out0;
+    ring.refused = row_indices[row] != (int)out0;
     // columns mod 16 are counted from the allocation (only differences matter): the one in front of the row
-    if (lane == 0) ring.e[(out0 - 1) & (kRing - 1)] = ((row_lo - 1u - first) & 15u) << 16;
+    if (lane == 0) ring.e[(out0 - 1u) & (kRing - 1)] = ((row_lo - 1u - first) & 15u) << 16;
     __syncwarp();
     int carry = -1;   // column of the last non-zero seen so far in this row
 
@@ -328,9 +331,9 @@ emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, 
         for (int b0 = 0; b0 < n; b0 += kFlush) {
             const int now = min(kFlush, n - b0);
             for (int i = lane; i < now; i += 32)
-                ring.e[(ring.out + i) & (kRing - 1)] = (unsigned)__ldg(dense + row_lo + (unsigned)(after + 16 * (b0 + i + 1))) | (((row_lo - first + (unsigned)after) & 15u) << 16);
-            ring.out += now;
-            if (ring.out - ring.flushed >= kFlush) ring_flush<I8>(ring, values, deltas32, kFlush, limit, vec_v, lane);
+                ring.e[(ring.out + (unsigned)i) & (kRing - 1)] = (unsigned)__ldg(dense + row_lo + (unsigned)(after + 16 * (b0 + i + 1))) | (((row_lo - first + (unsigned)after) & 15u) << 16);
+            ring.out += (unsigned)now;
+            if (ring.out - ring.flushed >= (unsigned)kFlush) ring_flush<I8>(ring, values, deltas32, kFlush, limit, vec_v, lane);
         }
     };
 
@@ -397,12 +400,12 @@ emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, 
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
             asm("{.reg .pred p; .reg .b32 t; shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff; @p add.s32 %0, %0, t;}" : "+r"(incl) : "r"(o));
-        int k = ring.out + incl - mine;
+        unsigned k = ring.out + (unsigned)(incl - mine);
         if (pads) {
             for (int q = 1; q <= npad; ++q, ++k)   // a gap of 16 or more zeros inside the step
                 ring.e[k & (kRing - 1)] = (unsigned)__ldg(dense + row_lo + (unsigned)(prev + 16 * q)) | (((row_lo - first + (unsigned)prev) & 15u) << 16);
         }
-        unsigned at = 4u * (unsigned)k;   // byte offset of the next entry, before the wrap
+        unsigned at = 4u * k;   // byte offset of the next entry, before the wrap
 #pragma unroll
         for (int i = 0; i < kEmitCols; ++i) {
             const unsigned x = w[i >> 3][(i >> 1) & 3];
@@ -412,16 +415,16 @@ emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, 
                          : "r"(x & ((i & 1) ? 0x7fff0000u : 0x7fffu)), "r"(__byte_perm(x, (unsigned)i, (i & 1) ? 0x5432 : 0x5410)), "r"(ring_base),
                            "n"(4 * kRing - 1) : "memory");
         }
-        ring.out += __shfl_sync(0xffffffffu, incl, 31);
-        if (ring.out - ring.flushed >= kFlush) ring_flush<I8>(ring, values, deltas32, kFlush, limit, vec_v, lane);
+        ring.out += (unsigned)__shfl_sync(0xffffffffu, incl, 31);
+        if (ring.out - ring.flushed >= (unsigned)kFlush) ring_flush<I8>(ring, values, deltas32, kFlush, limit, vec_v, lane);
     }
     if constexpr (I8) append_pads(carry, (cols - 1 - carry) >> 4);   // the int8 format keeps the pads inside the zeros at the end of a row
     ring_flush<I8>(ring, values, deltas32, ring.out - ring.flushed, limit, vec_v, lane);
     if (row == rows - 1) {
         // everything from n = row_indices[rows] to the padded count is zero (the deltas already are)
         const int n = row_indices[rows];
-        if (n < 0 || n > limit) ring.refused = true;   // row_indices and P do not belong together
-        for (int i = max(n, 0) + lane; i < limit; i += 32) values[i] = 0;
+        if (n < 0 || n > slots) ring.refused = true;   // row_indices and P do not belong together
+        for (unsigned i = (unsigned)max(n, 0) + (unsigned)lane; i < limit; i += 32u) values[i] = 0;
     }
     if (__any_sync(0xffffffffu, ring.refused) && lane == 0) atomicAdd(&g_compress_overflow, 1u);
 }

@@ -1,6 +1,8 @@
 """Stored counts within a few thousand elements of 2^31, the largest that the entry points take: element positions that run
 ahead of the last stored element must not wrap. A small matrix sits at the very end of buffers of 2^31 - 8 elements (6 GB
 of zeros in front of it, which no row refers to), and has to give what it gives in buffers of its own size."""
+import ctypes
+
 import pytest
 import torch
 
@@ -41,3 +43,41 @@ def test_decompress(buffers, rows, cols):
     dense = torch.full((rows, cols), 7.0, dtype=torch.float16, device=DEV)
     cabi.check(lib, lib.macko_decompress_fp16(v.data_ptr(), d.data_ptr(), ri.data_ptr(), rows, cols, P_MOST, dense.data_ptr(), _stream()))
     assert torch.equal(dense, macko_spmv.decompress(comp))
+
+
+def _emit(lib, M, ri, P, v, d, workspace_bytes):
+    call = lib.macko_compress_emit_int8 if M.dtype == torch.int8 else lib.macko_compress_emit
+    cabi.check(lib, call(M.data_ptr(), *M.shape, ri.data_ptr(), P, v.data_ptr(), d.data_ptr(), v.data_ptr(), workspace_bytes, _stream()))
+    count = ctypes.c_uint32()
+    cabi.check(lib, lib.macko_compress_overflow(ctypes.byref(count), _stream()))
+    return count.value
+
+
+# few columns: the elements end 1..7 slots in front of the padded count, where the clearing loop's next step lies beyond 2^31
+@pytest.mark.parametrize("dtype", [torch.float16, torch.int8])
+@pytest.mark.parametrize("rows,cols", [(7, 4099), (3, 9)])
+def test_emit(buffers, rows, cols, dtype):
+    lib = cabi.load()
+    M = workloads.bernoulli_matrix(rows, cols, 0.6, seed=rows, device=DEV)
+    M = (M * 30).round().clamp(-100, 100).to(dtype)
+    if int(macko_spmv.compress(M)[2][-1]) % 8 == 0:
+        M[0, 2] = 1 - (M[0, 2] != 0).to(dtype)        # one element more or less
+    values, deltas, ri = macko_spmv.compress(M)[:3]
+    P = values.numel()
+    assert int(ri[-1]) < P
+    v, d = buffers["values"].view(dtype)[-P_MOST:], buffers["deltas"]
+    v[-P - 64:] = 3                                   # the slots in front of the matrix keep this
+    assert _emit(lib, M, ri + (P_MOST - P), P_MOST, v, d, P_MOST) == 0
+    assert torch.equal(v[P_MOST - P:], values) and bool((v[-P - 64: -P] == 3).all())
+    assert torch.equal(d[(P_MOST - P) // 2:], deltas) and not d[-P // 2 - 32: -P // 2].any()
+
+
+def test_emit_refuses_what_lies_beyond(buffers):
+    """row_indices of another matrix: a row of 3000 elements that starts 64 slots in front of the end."""
+    lib = cabi.load()
+    M = torch.ones(2, 3000, dtype=torch.float16, device=DEV)
+    v, d = buffers["values"].view(torch.float16), buffers["deltas"]
+    v[-128:] = 3
+    ri = torch.tensor([P_MOST - 64, P_MOST, P_MOST], dtype=torch.int32, device=DEV)
+    assert _emit(lib, M, ri, P_MOST, v, d, P_MOST) == 2
+    assert bool((v[-64:] == 1).all()) and bool((v[-128:-64] == 3).all())
