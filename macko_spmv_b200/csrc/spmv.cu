@@ -386,9 +386,10 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     constexpr int LOG_STEP = (L == 32) ? 8 : (L == 16) ? 7 : (L == 8) ? 6 : 5;
     int my_row = -1;   // plain: row being walked by my group (-1: none); planned: 0 while a virtual row is walked
     unsigned out_word = 0u;   // planned: destination of the virtual row (a row of y, or a partial-sum slot)
-    int begin = 0;     // first stored element of the row
-    int end = 0;       // one past the last stored element
-    int pos = 0;       // first element of the group's next iteration (multiple of 8)
+    // Element positions are unsigned: an iteration runs up to 1536 elements ahead of a count that may come close to 2^31.
+    unsigned begin = 0u;   // first stored element of the row
+    unsigned end = 0u;     // one past the last stored element
+    unsigned pos = 0u;     // first element of the group's next iteration (multiple of 8)
     // Byte address (shared window, or byte offset from x - kXPadFront when x stays in global memory) of
     // "column -1 + index in row" in front of the lane's unit of the next sub-step, less 14 per lane below
     // it in the group: the lane totals that go through the scan carry +14 each (see the decode below).
@@ -491,7 +492,7 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
             const int avail = row_hi - row_next;
             if (avail <= 0) {
                 if (needmask == 0xffffffffu) done = true;
-                if (need) { my_row = -1; pos = 0; end = 0; begin = 0; }
+                if (need) { my_row = -1; pos = 0u; end = 0u; begin = 0u; }
             } else {
                 const unsigned leaders = needmask & kLeaders;
                 const int want = __popc(leaders);
@@ -504,16 +505,16 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
                 const int nr = row_next + rank;
                 // offsets are clamped into [0, stored] so that corrupt row_indices (or a corrupt plan) cannot send
                 // loads outside values/deltas
-                int b, e;
+                unsigned b, e;
                 unsigned colbase2 = 0u;   // planned: twice the column sum in front of the segment (a byte offset into x)
                 if constexpr (PLAN) {
-                    b = min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
+                    b = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
                     const unsigned pk = __shfl_sync(0xffffffffu, pk_reg, (nr - win_base) & 31);
-                    e = min(b + (int)(pk & ((1u << kPlanLenBits) - 1u)), stored);
+                    e = min(b + (pk & ((1u << kPlanLenBits) - 1u)), (unsigned)stored);
                     colbase2 = (pk >> kPlanLenBits) << 1;
                 } else {
-                    b = min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
-                    e = min(__shfl_sync(0xffffffffu, ri_reg, (nr + 1 - win_base) & 31), stored);
+                    b = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
+                    e = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr + 1 - win_base) & 31), (int)b), stored);
                 }
                 if (need) {
                     if (rank < take) {
@@ -523,10 +524,10 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
                         } else {
                             my_row = nr;
                         }
-                        begin = b; end = e; pos = b & ~(kGroup - 1);
-                        run = lane_const + colbase2 - 2u * (unsigned)(b & (kGroup - 1));   // the unit that holds `begin` starts before the row
+                        begin = b; end = e; pos = b & ~(unsigned)(kGroup - 1);
+                        run = lane_const + colbase2 - 2u * (b & (unsigned)(kGroup - 1));   // the unit that holds `begin` starts before the row
                     } else {
-                        my_row = -1; pos = 0; end = 0; begin = 0;
+                        my_row = -1; pos = 0u; end = 0u; begin = 0u;
                     }
                 }
                 row_next += take;
@@ -540,9 +541,9 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
         // ---- issue the loads of the whole iteration ------------------------------------------------------
         uint4 v[D];
         unsigned w[D];
-        const int ord0 = pos + lig * kGroup;
-        const int rem0 = end - ord0;    // elements of the row from the lane's first unit on
-        const int lo0 = begin - ord0;   // > 0: leading elements of sub-step 0 belong to the previous row
+        const int ord0 = (int)(pos + (unsigned)(lig * kGroup));   // not negative where it is used as an index
+        const int rem0 = (int)(end - (unsigned)ord0);    // elements of the row from the lane's first unit on
+        const int lo0 = (int)(begin - (unsigned)ord0);   // > 0: leading elements of sub-step 0 belong to the previous row
         {
             const uint4 *vp = values + (ord0 >> 3);
             const unsigned *dp = deltas + (ord0 >> 3);
@@ -692,7 +693,7 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
         }
         // every sub-step that was skipped lies behind the end of all rows of the warp: `run` is not used again before the next row resets it
         run += (unsigned)(2 * L * D);
-        pos += D * STEP;
+        pos += (unsigned)(D * STEP);
     }
 
     if constexpr (PEER) {

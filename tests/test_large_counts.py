@@ -81,3 +81,37 @@ def test_emit_refuses_what_lies_beyond(buffers):
     ri = torch.tensor([P_MOST - 64, P_MOST, P_MOST], dtype=torch.int32, device=DEV)
     assert _emit(lib, M, ri, P_MOST, v, d, P_MOST) == 2
     assert bool((v[-64:] == 1).all()) and bool((v[-128:-64] == 3).all())
+
+
+@pytest.mark.parametrize("lanes", [4, 8, 16, 32])
+@pytest.mark.parametrize("x_in_shared", [0, 1])
+def test_product(buffers, lanes, x_in_shared):
+    """Rows that end with the buffers, in every launch shape, the same bits as in small buffers."""
+    lib = cabi.load()
+    rows, cols = 37, 4099
+    M = workloads.bernoulli_matrix(rows, cols, 0.6, seed=lanes, device=DEV)
+    M[3] = 0
+    comp = macko_spmv.compress(M)
+    big = _at_the_end(comp, buffers)
+    x = torch.randn(cols, device=DEV).half()
+    for steps in (2, 4, 6):
+        ys = []
+        for v, d, ri, P in ((*comp[:3], comp[0].numel()), (*big, P_MOST)):
+            y = torch.full((rows,), 7.0, dtype=torch.float16, device=DEV)
+            cabi.check(lib, lib.macko_spmv_fp16_tuned(v.data_ptr(), d.data_ptr(), ri.data_ptr(), rows, cols, P, x.data_ptr(), y.data_ptr(),
+                                                      1.0, 0.0, _stream(), lanes, steps, x_in_shared, 0))
+            ys.append(y)
+        assert torch.equal(*ys), steps
+
+
+@pytest.mark.parametrize("frozen", [False, True])
+def test_product_default_and_batched(buffers, frozen):
+    rows, cols = 5, 4099      # rows of about 2500 elements take the same launch shape with either count
+    comp = macko_spmv.compress(workloads.bernoulli_matrix(rows, cols, 0.6, seed=9, device=DEV))
+    big = (*_at_the_end(comp, buffers), rows, cols)
+    V = torch.randn(8, cols, device=DEV).half()
+    if frozen:
+        comp, big = macko_spmv.freeze(comp, plan=False), macko_spmv.freeze(big, plan=False)
+    assert torch.equal(macko_spmv.multiply(big, V[0]), macko_spmv.multiply(comp, V[0]))
+    for n in (2, 4, 8):
+        assert torch.equal(macko_spmv.multiply_batched(big, V[:n]), macko_spmv.multiply_batched(comp, V[:n])), n
