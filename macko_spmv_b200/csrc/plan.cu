@@ -23,7 +23,7 @@ plan_count_kernel(const int *__restrict__ ri, int rows, int stored, int seg, int
     int b, e;
     row_span(ri, row, stored, b, e);
     const int n = e - b;
-    const int nseg = n > 0 ? (e - (b & ~7) + seg - 1) / seg : 1;
+    const int nseg = n > 0 ? (int)(((unsigned)(e - (b & ~7)) + (unsigned)seg - 1u) / (unsigned)seg) : 1;
     seg_first[row + 1] = nseg;
     atomicMax(header + 1, (unsigned)n);
     if (nseg > 1) atomicAdd(header + 2, 1u);
@@ -54,24 +54,25 @@ plan_segments_kernel(const unsigned *__restrict__ deltas32, const int *__restric
         return;
     }
     if (lane == 0) split_list[atomicAdd(header + 3, 1u)] = (unsigned)row;   // the rows the combining pass has to visit
-    const int a0 = b & ~7;
+    // unsigned positions: the last step of a row that ends close to 2^31 looks beyond it
+    const unsigned begin = (unsigned)b, end = (unsigned)e, a0 = begin & ~7u, useg = (unsigned)seg;
     unsigned running = 0;   // sum of (delta + 1) over the row's elements in front of the current step
-    for (int base = a0; base < e; base += 256) {
-        if ((base - a0) % seg == 0 && lane == 0) {
-            const int j = (base - a0) / seg;
-            const int sb = max(b, base), se = min(e, base + seg);
-            tmp_begin[first + j] = sb;
-            tmp_pk[first + j] = (unsigned)(se - sb) | (running << kPlanLenBits);
+    for (unsigned base = a0; base < end; base += 256u) {
+        if ((base - a0) % useg == 0u && lane == 0) {
+            const int j = (int)((base - a0) / useg);
+            const unsigned sb = max(begin, base), se = min(end, base + useg);
+            tmp_begin[first + j] = (int)sb;
+            tmp_pk[first + j] = (se - sb) | (running << kPlanLenBits);
             tmp_out[first + j] = kPlanPartialBit | (unsigned)(first + j);
             vrow[first + j] = (unsigned)row;
         }
-        const int k0 = base + 8 * lane;
+        const unsigned k0 = base + 8u * (unsigned)lane;
         unsigned mine = 0;
-        if (k0 < e) {
+        if (k0 < end) {
             const unsigned w = __ldg(deltas32 + (k0 >> 3));
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (k0 + i >= b && k0 + i < e) mine += ((w >> (4 * i)) & 15u) + 1u;
+            for (unsigned i = 0; i < 8u; ++i)
+                if (k0 + i >= begin && k0 + i < end) mine += ((w >> (4 * i)) & 15u) + 1u;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);

@@ -115,3 +115,14 @@ def test_product_default_and_batched(buffers, frozen):
     assert torch.equal(macko_spmv.multiply(big, V[0]), macko_spmv.multiply(comp, V[0]))
     for n in (2, 4, 8):
         assert torch.equal(macko_spmv.multiply_batched(big, V[:n]), macko_spmv.multiply_batched(comp, V[:n])), n
+
+
+def test_planned(buffers):
+    """A plan of rows that end with the buffers: the same segments, so the same bits."""
+    rows, cols, seg = 3, 60000, 3840
+    comp = macko_spmv.compress(workloads.bernoulli_matrix(rows, cols, 0.6, seed=10, device=DEV))
+    big = (*_at_the_end(comp, buffers), rows, cols)
+    small, large = (macko_spmv.freeze(c, plan=True, segment_elements=seg) for c in (comp, big))
+    assert small.plan_meta[:4] == large.plan_meta[:4] and small.plan_meta[3] == rows
+    x = torch.randn(cols, device=DEV).half()
+    assert torch.equal(macko_spmv.multiply(large, x), macko_spmv.multiply(small, x))
