@@ -18,6 +18,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import sysconfig
 
 import torch
 
@@ -27,6 +28,7 @@ __version__ = "0.1.0"
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _CORE_PATH = os.path.join(_PKG_DIR, "libmacko_b200.so")
 _OPS_PATH = os.path.join(_PKG_DIR, "_torch_ops.so")
+_DIRECT_PATH = os.path.join(_PKG_DIR, "_torch_direct" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 # The reference reads this variable to choose its JIT cache directory
 # (src/macko_spmv/__init__.py:12). Nothing is compiled at import here; it is accepted and ignored.
@@ -42,10 +44,12 @@ def _load_native():
             )
     core = ctypes.CDLL(_CORE_PATH, mode=ctypes.RTLD_GLOBAL)
     torch.ops.load_library(_OPS_PATH)
-    # the same library as a Python module: `multiply` for calls that only want the product
-    spec = importlib.util.spec_from_file_location(__name__ + "._torch_ops", _OPS_PATH)
-    direct = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(direct)
+    # `multiply` for calls that only want the product; built per Python version, where that has its headers
+    direct = None
+    if os.path.exists(_DIRECT_PATH):
+        spec = importlib.util.spec_from_file_location(__name__ + "._torch_direct", _DIRECT_PATH)
+        direct = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(direct)
     return core, direct
 
 
@@ -174,8 +178,9 @@ class FrozenMatrix(tuple):
         return self
 
 
-_direct.set_frozen_type(FrozenMatrix)
-_direct_multiply = _direct.multiply
+if _direct is not None:
+    _direct.set_frozen_type(FrozenMatrix)
+_direct_multiply = _direct.multiply if _direct is not None else lambda compressed_M, V: None
 _is_compiling = torch.compiler.is_compiling
 
 
@@ -205,7 +210,7 @@ def multiply(compressed_M, V, out=None):
     `out` (not in the reference): a contiguous CUDA vector of M_rows elements that receives y, for callers
     that keep their results in one buffer; without it a new tensor is returned, as in the reference."""
     if out is None and not _is_compiling():
-        y = _direct_multiply(compressed_M, V)   # None: not a plain call, or not a valid one
+        y = _direct_multiply(compressed_M, V)   # None: not a plain call
         if y is not None:
             return y
     assert compressed_M[0].is_cuda

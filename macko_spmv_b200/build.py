@@ -1,7 +1,9 @@
 """In-tree build of the two native libraries of this package.
 
 ``libmacko_b200.so``  CUDA kernels + C ABI (nvcc, sm_100a only, no torch dependency)
-``_torch_ops.so``     the `macko_spmv::*` torch operators, linked against the C ABI
+``_torch_ops.so``     the `macko_spmv::*` torch operators, linked against the C ABI and libtorch (no Python)
+``_torch_direct*.so`` `multiply` as a function of this Python version, past the operator dispatcher; left out where
+                      the interpreter comes without its headers: `multiply` then always takes the operator
 ``macko_bench``       command-line benchmark with the reference CLI's arguments (C ABI + cuBLAS)
 
 Run ``python macko_spmv_b200/build.py`` (or call :func:`build`). Nothing is compiled at
@@ -20,6 +22,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_CORE = os.path.join(PKG_DIR, "libmacko_b200.so")
 LIB_TORCH = os.path.join(PKG_DIR, "_torch_ops.so")
+LIB_DIRECT = os.path.join(PKG_DIR, "_torch_direct" + sysconfig.get_config_var("EXT_SUFFIX"))
 BENCH_CLI = os.path.join(PKG_DIR, "macko_bench")
 
 CUDA_SOURCES = ["common.cu", "spmv.cu", "compress.cu", "decompress.cu", "plan.cu", "decode_glue.cu"]
@@ -79,27 +82,44 @@ def build_core(force: bool = False, verbose: bool = False) -> str:
     return LIB_CORE
 
 
-def build_torch_ops(force: bool = False, verbose: bool = False) -> str:
-    src = os.path.join(CSRC, "torch_binding.cpp")
-    if not force and _newer(LIB_TORCH, [src, LIB_CORE, os.path.join(INCLUDE, "macko_b200.h"), __file__]):
-        return LIB_TORCH
+def _build_torch(src: str, out: str, extra: list[str], verbose: bool) -> str:
     import torch
     from torch.utils import cpp_extension as ce
 
-    inc = ["-isystem", sysconfig.get_paths()["include"]]
+    inc = []
     for p in ce.include_paths("cuda"):
         inc += ["-isystem", p]
     lib_dirs = ce.library_paths("cuda")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cmd = [
         "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-        "-DTORCH_API_INCLUDE_EXTENSION_H", "-I", INCLUDE, *inc, src, "-o", LIB_TORCH,
+        "-DTORCH_API_INCLUDE_EXTENSION_H", "-I", INCLUDE, *inc, src, "-o", out,
         *[f"-L{d}" for d in lib_dirs], "-L", PKG_DIR,
-        "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-l:libmacko_b200.so",
+        "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", *extra, "-l:libmacko_b200.so",
         "-Wl,-rpath,$ORIGIN", *[f"-Wl,-rpath,{d}" for d in lib_dirs],
     ]
     _run(cmd, verbose)
-    return LIB_TORCH
+    return out
+
+
+def build_torch_ops(force: bool = False, verbose: bool = False) -> str:
+    src = os.path.join(CSRC, "torch_binding.cpp")
+    headers = [os.path.join(CSRC, "torch_products.h"), os.path.join(INCLUDE, "macko_b200.h")]
+    if not force and _newer(LIB_TORCH, [src, LIB_CORE, *headers, __file__]):
+        return LIB_TORCH
+    return _build_torch(src, LIB_TORCH, [], verbose)
+
+
+def build_torch_direct(force: bool = False, verbose: bool = False) -> str | None:
+    src = os.path.join(CSRC, "torch_direct.cpp")
+    headers = [os.path.join(CSRC, "torch_products.h"), os.path.join(INCLUDE, "macko_b200.h")]
+    python_inc = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(python_inc, "Python.h")):
+        print(f"no Python.h in {python_inc}: multiply will go through the operator dispatcher", file=sys.stderr)
+        return None
+    if not force and _newer(LIB_DIRECT, [src, LIB_TORCH, *headers, __file__]):
+        return LIB_DIRECT
+    return _build_torch(src, LIB_DIRECT, ["-isystem", python_inc, "-ltorch_python", "-l:_torch_ops.so"], verbose)
 
 
 def build_cli(force: bool = False, verbose: bool = False) -> str:
@@ -114,6 +134,7 @@ def build_cli(force: bool = False, verbose: bool = False) -> str:
 def build(force: bool = False, verbose: bool = False) -> None:
     build_core(force, verbose)
     build_torch_ops(force, verbose)
+    build_torch_direct(force, verbose)
     build_cli(force, verbose)
 
 
