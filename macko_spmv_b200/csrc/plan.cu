@@ -174,7 +174,7 @@ int check_plan_args(int64_t rows, int64_t cols, int64_t padded_count, int32_t se
     if (rows >= (1LL << 30) || padded_count >= (1LL << 31) || cols >= (1LL << (32 - kPlanLenBits)))
         return fail(MACKO_ERR_SIZE_OVERFLOW, "rows=%lld cols=%lld P=%lld are beyond what a plan can index",
                     (long long)rows, (long long)cols, (long long)padded_count);
-    const int seg = segment_elements == 0 ? plan_default_segment(padded_count) : segment_elements;
+    const int seg = segment_elements == 0 ? plan_default_segment(padded_count, cols) : segment_elements;
     if (seg < 256 || seg > kPlanMaxSegment || seg % 256 != 0)
         return fail(MACKO_ERR_INVALID_ARGUMENT, "segment_elements must be 0 or a multiple of 256 in [256, %d] (got %d)",
                     kPlanMaxSegment, segment_elements);
@@ -255,7 +255,7 @@ int macko_spmv_plan(const void *deltas, const int32_t *row_indices, int64_t rows
     // not the same number of elements), in a matrix that is large enough for the second kernel to pay.
     const long long mean = rows > 0 ? padded_count / rows : 0;
     info->recommended = (info->longest_row > 2 * seg && (long long)info->longest_row >= 3 * mean &&
-                         padded_count >= kPlanMinShare * kPlanGroups) ? 1 : 0;
+                         padded_count >= kPlanMinShare * plan_groups(cols)) ? 1 : 0;
     return MACKO_OK;
 }
 }

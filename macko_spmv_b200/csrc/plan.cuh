@@ -15,9 +15,12 @@
 
 namespace macko {
 
+// x in shared memory is framed by zeros
+constexpr int kXPadFront = 32;       // fp16 slots in front of x[0] (64 bytes: keeps x 16B-aligned)
+constexpr int kXPadBack = 160;       // fp16 slots after x[cols-1]  (> 8 * 16 + 8)
+
 constexpr int kPlanLenBits = 12;                         // a virtual row holds fewer than 4096 stored elements
 constexpr int kPlanMaxSegment = 3840;                    // largest segment length (a multiple of 256)
-constexpr long long kPlanGroups = 148LL * 32 * 4;        // rows that a planned launch walks at once on a B200: 4 per resident warp
 constexpr int kPlanBuckets = 64;                         // length classes: 64-element sub-steps spanned, 0..60
 constexpr unsigned kPlanPartialBit = 0x80000000u;        // destination word: a partial-sum slot, not a row of y
 
@@ -64,16 +67,23 @@ inline PlanLayout plan_layout(long long rows, long long padded, int seg)
     return l;
 }
 
-// Segment length where the caller names none. A group of lanes gets a share of padded / kPlanGroups elements: a
+// Virtual rows that a planned launch walks at once: four per resident warp, with 32 warps on an SM while two CTAs hold x
+// in its shared memory, else 16. The number of SMs is that of a B200 and not asked for: macko_spmv_plan_bytes has to
+// agree with the builder and may be called where no device is.
+constexpr long long kPlanTwoCtaCols = (227 * 1024 / 2 - 1024) / 2 - kXPadFront - kXPadBack;   // 57408: what launch_variant works out
+inline long long plan_groups(long long cols) { return 148LL * 4 * (cols <= kPlanTwoCtaCols ? 32 : 16); }
+
+// Segment length where the caller names none. A group of lanes gets a share of padded / plan_groups elements: a
 // segment a little longer than the share leaves one long segment per group and the short rows to even the ends out,
 // a much longer one leaves groups without work while others walk it, a much shorter one costs a hand-over and a
 // partial sum each time. Above about 1088 elements per group a fixed 1536 is as good as any choice. Skewed matrices of
 // mean density 0.2 (B200, graph of products, us, this rule / always 1536): 4879x7688 (share 474) 13.8 / 19.5,
 // 12000x4096 (617) 14.5 / 19.9, 16000x4096 (822) 16.8 / 20.7, 4096x16384 (858) 20.9 / 23.7, 9000x9000 (1032)
-// 20.6 / 22.5.
-inline int plan_default_segment(long long padded)
+// 20.6 / 22.5. With one CTA per SM (shares of twice the size; this rule / the segment for 32 warps / always 1536):
+// 300x100000 (794) 23.7 / 32.0 / 25.8, 400x65536 (684) 14.8 / 18.7 / 18.0.
+inline int plan_default_segment(long long padded, long long cols)
 {
-    const long long share = padded / kPlanGroups;
+    const long long share = padded / plan_groups(cols);
     if (share > 1088) return 1536;
     const long long seg = (share + 16 + 255) / 256 * 256;
     return (int)(seg < 512 ? 512 : seg);

@@ -44,8 +44,6 @@ namespace {
 constexpr int kThreads = 512;        // threads per CTA
 constexpr int kWarpsPerCta = kThreads / 32;
 constexpr int kGroup = 8;            // stored elements per lane per sub-step (one 128-bit value load)
-constexpr int kXPadFront = 32;       // zero fp16 slots in front of x[0] (64 bytes: keeps x 16B-aligned)
-constexpr int kXPadBack = 160;       // zero fp16 slots after x[cols-1]  (> 8 * 16 + 8)
 
 // acc += fp16(low or high half of vword) * fp16(low half of xbits): the sm_100 mixed-precision FMA
 // (exact fp16 product accumulated in fp32, round to nearest); the halves are split inside the asm so

@@ -10,11 +10,13 @@ DEV = "cuda:0"
 GROUPS = 148 * 32 * 4
 
 
-def test_plan_bytes_follow_the_default_segment():
+# 57408 columns are the most that two CTAs of an SM can hold; with one the groups are half as many
+@pytest.mark.parametrize("cols,groups", [(8192, GROUPS), (57408, GROUPS), (57409, GROUPS // 2), (100000, GROUPS // 2)])
+def test_plan_bytes_follow_the_default_segment(cols, groups):
     lib = cabi.load()
     for share, seg in ((0, 512), (496, 512), (497, 768), (752, 768), (1008, 1024), (1009, 1280), (1088, 1280), (1089, 1536), (9000, 1536)):
-        padded = share * GROUPS
-        assert lib.macko_spmv_plan_bytes(5000, 8192, padded, 0) == lib.macko_spmv_plan_bytes(5000, 8192, padded, seg), share
+        padded = share * groups
+        assert lib.macko_spmv_plan_bytes(5000, cols, padded, 0) == lib.macko_spmv_plan_bytes(5000, cols, padded, seg), share
 
 
 @pytest.mark.gpu
