@@ -40,3 +40,17 @@ def test_default_plans(rows, dense_rows, cols, planned, seg):
         ref, l1 = M.double() @ x.double(), M.double().abs() @ x.double().abs()
         # half a unit in the last place of y, and 2^-23 of the absolute sum per addition of the fp32 sums
         assert bool(((y - ref).abs() <= 2.0 ** -11 * ref.abs() + cols * 2.0 ** -23 * l1 + 2.0 ** -24).all())
+
+
+@pytest.mark.gpu
+def test_no_plan_where_x_does_not_fit():
+    """120 000 columns: the planned launch would refuse the matrix that `freeze` made."""
+    rows, cols = 300, 120_000
+    M = torch.zeros(rows, cols, dtype=torch.float16, device=DEV)
+    M[::4, ::7] = 0.01
+    M[:70] = torch.randn(70, cols, device=DEV).half()
+    comp = macko_spmv.compress(M)
+    frozen = macko_spmv.freeze(comp)
+    assert frozen.plan is None
+    x = torch.randn(cols, device=DEV).half()
+    assert torch.equal(macko_spmv.multiply(frozen, x), macko_spmv.multiply(comp, x))
