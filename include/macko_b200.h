@@ -148,8 +148,8 @@ int macko_spmv_shape(int64_t rows, int64_t cols, int64_t padded_count, int sm_co
  *                          cols must fit shared memory (about 116 000). Calls that use one plan must not
  *                          overlap on the GPU (they share the partial sums inside it).
  * info->recommended is 1 when the row statistics say that the planned launch should beat macko_spmv_fp16
- * (rows cut into several segments and much longer than the average row, in a matrix of some size and no wider than
- * the planned launch can take).
+ * (rows cut into several segments and much longer than the average row, in a matrix of some size or with a row that
+ * outlasts the rest of the launch, and no wider than the planned launch can take).
  * No counterpart in the reference: its kernel gives every row one warp (kernels_torch_launchers.cuh:15-16),
  * which is what makes uneven rows slow there.
  */

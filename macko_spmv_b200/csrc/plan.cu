@@ -252,15 +252,19 @@ int macko_spmv_plan(const void *deltas, const int32_t *row_indices, int64_t rows
     info->split_rows = (int32_t)host_header[2];
     // Worth it when some rows are long enough to be cut several times (a row is a serial chain of sub-steps for the
     // lanes that walk it) and far longer than the average (the plain launch gives every warp the same number of rows,
-    // not the same number of elements), in a matrix that is large enough for the second kernel to pay; and only where the
-    // planned launch can run at all, which takes x in shared memory.
+    // not the same number of elements), in a matrix that is large enough for the second kernel to pay or has a row that
+    // outlasts it (plan.cuh); and only where the planned launch can run at all, which takes x in shared memory.
     const long long mean = rows > 0 ? padded_count / rows : 0;
     const DeviceInfo *dev = nullptr;
     st = current_device_info(&dev);
     if (st != MACKO_OK) return st;
     const bool x_fits = (kXPadFront + cols + kXPadBack) * 2 <= dev->max_smem_optin;
-    info->recommended = (x_fits && info->longest_row > 2 * seg && (long long)info->longest_row >= 3 * mean &&
-                         padded_count >= kPlanMinShare * plan_groups(cols)) ? 1 : 0;
+    int lanes = 0, steps = 0;   // of the default launch
+    st = macko_spmv_shape(rows, cols, padded_count, dev->sm_count, &lanes, &steps);
+    if (st != MACKO_OK) return st;
+    const bool large = padded_count >= kPlanMinShare * plan_groups(cols);
+    const bool long_row = (long long)info->longest_row >= kPlanMinChain * 8 * lanes;
+    info->recommended = (x_fits && info->longest_row > 2 * seg && (long long)info->longest_row >= 3 * mean && (large || long_row)) ? 1 : 0;
     return MACKO_OK;
 }
 }

@@ -89,10 +89,19 @@ inline int plan_default_segment(long long padded, long long cols)
     return (int)(seg < 512 ? 512 : seg);
 }
 
-// Fewest elements per group for which a plan is recommended: below, the launch is over before the balance pays for the
-// hand-overs and the second kernel. Default launch / plan (us): 5504x3200 (share 221) 8.4 / 10.5, 2500x9000 (287)
-// 11.7 / 13.2, 3000x9000 (346) 10.7 / 12.8; 7436x4034 (382) 11.4 / 11.0, 6000x6000 (458) 14.3 / 13.0.
+// When a plan of cut rows is recommended: either a group's share is kPlanMinShare elements or more, or the lanes that walk
+// the longest row in the default launch take kPlanMinChain sub-steps or more over it (0.2 us each, whatever the rest of
+// the chip does). Smaller matrices without such a row are done before the balance pays for the hand-overs and the second
+// kernel. Default launch / plan (us) by share and sub-steps, B200, graph of products of rotating matrices:
+//   neither     skewed, mean density 0.2: 5504x3200 (221, 25) 9.7 / 10.9, 2000x8192 (210, 32) 10.8 / 12.3, 3000x8192 (314, 32)
+//               11.9 / 13.4, 3000x9000 (345, 35) 12.5 / 13.7; 4096x8192, 20 dense rows among d = 0.1 (224, 32) 11.4 / 10.9
+//   long row    skewed: 1200x11008 (168, 43) 13.5 / 12.4, 2400x11008 (335, 43) 14.6 / 14.1, 2048x13184 (344, 51) 15.8 / 14.6, 1400x16384
+//               (298, 64) 18.1 / 15.1, 400x65536 (684, 256) 58.9 / 14.8; dense rows among empty or sparse ones: 20 of 512x65536
+//               (138, 256) 58.7 / 11.6, 200 of 900x30000 (316, 117) 30.3 / 17.1, 20 of 20000x4096 (313, 64) 18.1 / 10.7
+//   large       skewed: 20000x1500 (373, 23) 14.0 / 11.6, 5000x6000 (381, 23) 14.4 / 13.2, 6000x5000 (380, 39) 14.4 / 12.6, but
+//               3500x8500 (377, 33) 12.9 / 13.8 and 3072x18304 20.7 / 22.3: the share alone does not tell these apart
 constexpr long long kPlanMinShare = 365;
+constexpr long long kPlanMinChain = 40;
 
 // Length class of a virtual row: 64-element sub-steps between the unit its first element sits in and its end.
 __host__ __device__ inline int plan_length_class(int begin, int len)

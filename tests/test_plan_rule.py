@@ -21,8 +21,13 @@ def test_plan_bytes_follow_the_default_segment(cols, groups):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,dense_rows,cols,planned,seg", [
-    (900, 200, 30000, False, 512),     # 317 elements per group: too small for a plan
+    (3000, 300, 10232, False, 512),    # 162 elements per group, 39.97 sub-steps of a warp over the longest row: no plan
+    (3000, 300, 10240, True, 512),     # 40 sub-steps
+    (512, 20, 65536, True, 512),       # 138 elements per group (of one CTA per SM), 256 sub-steps
+    (900, 200, 30000, True, 512),      # 317, 117 sub-steps
     (900, 240, 30000, True, 512),      # 380
+    (8192, 1700, 4000, False, 512),    # 358 elements per group, 31 sub-steps of 16 lanes
+    (8192, 1740, 4000, True, 512),     # 367
     (2000, 400, 30000, True, 768),     # 634
     (900, 800, 30000, False, 1536),    # 1267, but no row is far longer than the mean
     (4000, 640, 30000, True, 1280),    # 1014
