@@ -247,10 +247,13 @@ DENSE_BATCH_THRESHOLD = 16
 
 
 def _dense_copy_pays(compressed_M, batch: int) -> bool:
-    """9..DENSE_BATCH_THRESHOLD vectors of an fp16 matrix: passes of the multi-vector kernel (8 vectors each, measured
-    at 1.3 TB/s of compressed bytes) against one decompression (3.0 TB/s of compressed + dense bytes) plus about
-    19 us for the GEMM and the dense buffer. At 50 % density the dense copy wins from 9 vectors on (68 against
-    85 us for 16 vectors on 11008x4096), at 30 % and below the two passes do."""
+    """9..DENSE_BATCH_THRESHOLD vectors of an fp16 matrix: passes of the multi-vector kernel against one dense copy and a GEMM.
+
+    The line: ceil(batch / 8) passes at 1.3 TB/s of compressed bytes against the copy at 3.0 TB/s of compressed + dense bytes
+    plus 19 us. The rates are those of an earlier decompressor; today's takes about 5 TB/s, so the line keeps to the passes where
+    the copy is already ahead. Measured (B200, us, passes / copy, * = chosen): 11008x4096 16 vectors d = 0.2 *47.5 / 39.4,
+    0.3 *59.7 / 42.5, 0.4 71.6 / *45.5, 0.5 85.4 / *47.6; 9 vectors 0.2 *32.8 / 39.4, 0.4 49.5 / *45.4; 4096x4096 16 vectors
+    0.5 *45.9 / 22.6, 0.7 52.3 / *24.9; 8192x8192 9 vectors 0.3 *54.1 / 73.1, 0.5 78.6 / *84.6, 16 vectors 0.3 *78.1 / 73.2."""
     if batch <= 8 or compressed_M[0].dtype != torch.float16:
         return False
     stored_bytes = 2.5 * compressed_M[0].numel()

@@ -942,7 +942,8 @@ int launch_l(int L, int D, const void *values, const void *deltas, const int32_t
 //     ~64 sub-steps (a row is a serial chain of sub-steps; 16 sub-steps for very wide matrices, where a full
 //     warp per row measured better; 96 for two rows per warp when every warp holds one such block only: 5504x11008
 //     d = 0.9 32.0 us against 38.2 with a warp per row, 6000x10000 31.3 / 36.0, 6784x13312 d = 0.82 40.9 / 44.6,
-//     8000x16384 d = 0.5 38.6 / 39.5; with more blocks than warps 11008x11008 d = 0.9 66.6 / 61.3);
+//     8000x16384 d = 0.5 38.6 / 39.5; with more blocks than warps 11008x11008 d = 0.9 66.6 / 61.3; plain launches in
+//     a graph, matrices declared immutable take 30.1 / 35.6 on the first);
 //   * rows shorter than half a sub-step shrink the group further;
 //   * six units in flight once a row holds more than three sub-steps, four above one, else two.
 struct Shape { int L, D; };
