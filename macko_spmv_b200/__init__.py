@@ -190,7 +190,8 @@ def freeze(compressed_M, plan="auto", segment_elements=0):
     Waits once for the device work that produced the buffers (they must be complete before a kernel may read
     them ahead of stream order). `plan`: "auto" builds the plan and keeps it only if the row statistics
     recommend it (rows far longer than the average, e.g. skewed matrices), True keeps it always, False builds
-    none. The reference has no counterpart (src/macko_spmv/__init__.py has only compress / multiply)."""
+    none. The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
+    (from several streams, order them or freeze once per stream). The reference has no counterpart (src/macko_spmv/__init__.py has only compress / multiply)."""
     assert compressed_M[0].is_cuda and compressed_M[1].is_cuda and compressed_M[2].is_cuda
     torch.cuda.synchronize(compressed_M[0].device)
     if plan is False or compressed_M[0].dtype != torch.float16:
