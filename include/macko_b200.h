@@ -191,6 +191,31 @@ int macko_spmm_fp16(const void *values, const void *deltas, const int32_t *row_i
                     const void *x, void *y, int64_t batch, float alpha, float beta, void *stream);
 
 /*
+ * The same product over column windows, for a matrix that is multiplied with several vectors again and again. Windows are
+ * side metadata built once per matrix on the GPU (8 bytes per row and window of up to 1408 columns; the three MACKO buffers stay as they
+ * are): where the stored elements of every row enter each window of columns. With them a CTA holds its window of x eight
+ * times over in shared memory, so that the lanes of a gather never meet in a bank, the resource that macko_spmm_fp16 is bound
+ * by. The sums of a row over the windows are added in window order by a second, small kernel: y is reproducible and
+ * matches macko_spmm_fp16 up to the order of the fp32 additions. No counterpart in the reference (BATCH = 1,
+ * c_benchmarking/utils.cuh:299).
+ *
+ *   macko_spmm_windows_bytes  size of the windows buffer (-1 for sizes that windows cannot index)
+ *   macko_spmm_windows        builds it into `windows` (device memory, 8-byte aligned) on `stream`
+ *   macko_spmm_windowed_workspace_bytes  scratch that a product with `batch` vectors needs (partial sums; 0 for narrow
+ *                             matrices). It belongs to one call: products that overlap on the GPU need one each.
+ *   macko_spmm_fp16_windowed  the product, 8 vectors per pass over the matrix (4 for up to 4 vectors). `windows` must have been
+ *                             built from the same deltas and row_indices. flags: MACKO_SPMV_MATRIX_IMMUTABLE, which here
+ *                             covers `windows` too.
+ */
+int64_t macko_spmm_windows_bytes(int64_t rows, int64_t cols, int64_t padded_count);
+int macko_spmm_windows(const void *deltas, const int32_t *row_indices, int64_t rows, int64_t cols, int64_t padded_count,
+                       void *windows, int64_t windows_bytes, void *stream);
+int64_t macko_spmm_windowed_workspace_bytes(int64_t rows, int64_t cols, int64_t padded_count, int64_t batch);
+int macko_spmm_fp16_windowed(const void *values, const void *deltas, const int32_t *row_indices, int64_t rows, int64_t cols,
+                             int64_t padded_count, const void *windows, int64_t windows_bytes, const void *x, void *y, int64_t batch,
+                             float alpha, float beta, void *workspace, int64_t workspace_bytes, uint32_t flags, void *stream);
+
+/*
  * Dense row-major fp16 [rows][cols] from a compressed matrix: element k of a row goes to column
  * (sum of the deltas of elements 0..k) + k, as the reference kernel decodes it
  * (src/macko_spmv/cuda/kernels.cuh:86-108); stored non-zeros keep their bits, everything else

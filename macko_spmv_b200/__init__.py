@@ -58,6 +58,8 @@ _core.macko_version.restype = ctypes.c_int
 _core.macko_last_error.restype = ctypes.c_char_p
 _core.macko_status_string.restype = ctypes.c_char_p
 _core.macko_status_string.argtypes = [ctypes.c_int]
+_core.macko_spmm_windows_bytes.restype = ctypes.c_int64
+_core.macko_spmm_windows_bytes.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int64]
 
 
 def native_library_paths() -> tuple[str, str]:
@@ -87,6 +89,17 @@ def _compress_fake(M):
 
 @torch.library.register_fake("macko_spmv::multiply_batched")
 def _multiply_batched_fake(M_values, M_deltas, M_row_indices, M_rows, M_cols, V):
+    return torch.empty((V.shape[0], M_rows), device=M_values.device, dtype=M_values.dtype)
+
+
+@torch.library.register_fake("macko_spmv::windows_build")
+def _windows_build_fake(M_deltas, M_row_indices, M_rows, M_cols):
+    n = torch.library.get_ctx().new_dynamic_size()
+    return M_deltas.new_empty((n,))
+
+
+@torch.library.register_fake("macko_spmv::multiply_windowed")
+def _multiply_windowed_fake(M_values, M_deltas, M_row_indices, M_rows, M_cols, windows, V, frozen):
     return torch.empty((V.shape[0], M_rows), device=M_values.device, dtype=M_values.dtype)
 
 
@@ -170,11 +183,15 @@ class FrozenMatrix(tuple):
 
     plan = None        # device buffer of the plan, or None
     plan_meta = None   # (virtual_rows, segment_elements, longest_row, split_rows, recommended)
+    windows = None     # device buffer of the column windows that `multiply_batched` walks, or None
+    windows_of = None  # write counts of deltas and row_indices when the windows were built
 
-    def __new__(cls, compressed, plan=None, plan_meta=None):
+    def __new__(cls, compressed, plan=None, plan_meta=None, windows=None, windows_of=None):
         self = super().__new__(cls, tuple(compressed[:5]))
         self.plan = plan
         self.plan_meta = plan_meta
+        self.windows = windows
+        self.windows_of = windows_of
         return self
 
 
@@ -190,19 +207,40 @@ def freeze(compressed_M, plan="auto", segment_elements=0):
     Waits once for the device work that produced the buffers (they must be complete before a kernel may read
     them ahead of stream order). `plan`: "auto" builds the plan and keeps it only if the row statistics
     recommend it (rows far longer than the average, e.g. skewed matrices), True keeps it always, False builds
-    none. The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
+    none. Unless it is False, an fp16 matrix also gets its column windows, which `multiply_batched` walks (8 bytes per row and
+    window of up to 1408 columns, at most 5 % of the matrix). The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
     (from several streams, order them or freeze once per stream). The reference has no counterpart (src/macko_spmv/__init__.py has only compress / multiply)."""
     assert compressed_M[0].is_cuda and compressed_M[1].is_cuda and compressed_M[2].is_cuda
     torch.cuda.synchronize(compressed_M[0].device)
     if plan is False or compressed_M[0].dtype != torch.float16:
         return FrozenMatrix(compressed_M)
+    windows, windows_of = _build_windows(compressed_M)   # before the plan, which waits for the device
     buf, meta = torch.ops.macko_spmv.plan_build.default(
         compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], compressed_M[0].numel(), int(segment_elements))
     meta = [int(v) for v in meta.tolist()]
     info = (meta[3], meta[4], meta[5], meta[6], meta[7])
     if plan is True or info[4]:
-        return FrozenMatrix(compressed_M, buf, info)
-    return FrozenMatrix(compressed_M, None, info)
+        return FrozenMatrix(compressed_M, buf, info, windows, windows_of)
+    return FrozenMatrix(compressed_M, None, info, windows, windows_of)
+
+
+def _write_counts(deltas, row_indices):
+    """How often the two tensors have been written in place, or None where that is not counted (inference tensors)."""
+    if deltas.is_inference() or row_indices.is_inference():
+        return None
+    return deltas._version, row_indices._version
+
+
+def _build_windows(compressed_M):
+    """Column windows of an fp16 matrix (`macko_spmm_windows`) and what they were built from, or (None, None) where the rows are so
+    short that their 8 bytes per row and window would weigh more than 5 % of the matrix."""
+    _, deltas, row_indices, rows, cols = compressed_M[:5]
+    stored = 2 * deltas.numel()
+    if rows == 0 or rows >= 1 << 30 or cols >= 1 << 24:
+        return None, None
+    if 20 * _core.macko_spmm_windows_bytes(rows, cols, stored) > 2.5 * stored:
+        return None, None
+    return torch.ops.macko_spmv.windows_build.default(deltas, row_indices, rows, cols), _write_counts(deltas, row_indices)
 
 
 def multiply(compressed_M, V, out=None):
@@ -270,19 +308,58 @@ def decompress(compressed_M):
     return torch.ops.macko_spmv.decompress.default(*compressed_M[:5])
 
 
+# Beyond this many right-hand sides the windowed product has never been ahead of the dense copy.
+WINDOWED_BATCH_LIMIT = 64
+
+
+def _windows_pay(frozen, V) -> bool:
+    """Whether a batch goes over the column windows of a frozen matrix (`macko_spmm_fp16_windowed`).
+
+    3..8 vectors always do, where the other choice is one pass of the one-kernel product: 11008x4096 d = 0.5 8 vectors 25.0
+    against 42.4 us, 4 vectors 20.7 / 27.0; 8192x8192 d = 0.3 24.2 / 38.8; 512x512 d = 0.5 5.5 / 6.5 and, the only loss, 3 vectors
+    4.4 / 4.2. Two vectors are level or behind (11008x4096 20.7 / 19.3, 4096x4096 d = 0.7 12.8 / 11.1).
+    Larger batches take every 8 vectors through the matrix, against one dense copy and a GEMM: the two models below, in us, fit 18
+    shapes x 9..48 vectors with a standard deviation of 7 % and 21 %. 16 vectors, windows / copy: 4096x11008 d = 0.5 39.3 / 48.6,
+    d = 0.2 24.8 / 42.6, 4096x4096 d = 0.7 23.4 / 21.3, 16384x4096 d = 0.9 92.6 / 77.3; 24 vectors: 4096x11008 d = 0.2 35.9 / 42.9,
+    11008x4096 d = 0.5 57.4 / 44.0, 1024x16384 d = 0.3 18.9 / 26.9. The GEMM is slower where rows of the copy do not start on
+    16 bytes: 1500x5001 d = 0.15 16 vectors 8.5 / 21.5."""
+    batch = V.shape[0]
+    if frozen.windows is None or batch < 3 or batch > WINDOWED_BATCH_LIMIT or _is_compiling():
+        return False
+    if frozen.windows_of != _write_counts(frozen[1], frozen[2]):
+        return False   # written since: the windows may be those of another matrix
+    if batch <= 8:
+        return True
+    # the dense copy goes through operators that can be differentiated and transformed
+    if (V.requires_grad and torch.is_grad_enabled()) or type(V) is not torch.Tensor or torch._C._functorch.peek_interpreter_stack() is not None \
+            or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    rows, cols, stored = frozen[3], frozen[4], 2 * frozen[1].numel()
+    windows, groups, blocks = frozen.windows.numel() // (8 * rows), (batch + 7) // 8, (rows + 3) // 4
+    ctas = windows * groups
+    warps = 32 * max(1, 148 // ctas)
+    rounds = 0.5 * (blocks / warps - blocks // -warps) * -(ctas // -148)
+    windows_us = 4.6 + 0.74 * rounds * (stored / (64.0 * rows * windows) + 1.5) + 3.7e-6 * windows * rows * batch
+    copy_us = (6.9 + 0.63e-6 * rows * cols + 0.52e-6 * stored) * (1.0 if cols % 8 == 0 else 1.7)
+    return windows_us < copy_us
+
+
 def multiply_batched(compressed_M, V):
     """Y[batch, rows] = V[batch, cols] @ M^T for a compressed matrix and fp16 CUDA vectors.
 
     The reference runs batched inputs as a loop of `multiply` calls (torch.vmap fallback,
     python_scripts/util_run_pruned_llm.py:112-115). Here up to 8 vectors share one pass over the compressed
     matrix; 9..DENSE_BATCH_THRESHOLD take two passes or, where the matrix is dense enough for that to be cheaper,
-    the route of the larger batches: decompress once and run a dense GEMM.
+    the route of the larger batches: decompress once and run a dense GEMM. A frozen matrix (`freeze`) has column windows, over
+    which a pass is up to twice as fast, so more batches stay with the compressed matrix.
     """
     assert compressed_M[0].is_cuda
     assert V.is_cuda
     assert V.is_contiguous()
     if V.dim() != 2:
         raise RuntimeError("V must have shape [batch, cols]")
+    if type(compressed_M) is FrozenMatrix and _windows_pay(compressed_M, V):
+        return torch.ops.macko_spmv.multiply_windowed.default(*compressed_M[:5], compressed_M.windows, V, True)
     if V.shape[0] > DENSE_BATCH_THRESHOLD or _dense_copy_pays(compressed_M, V.shape[0]):
         return V @ decompress(compressed_M).t()
     return torch.ops.macko_spmv.multiply_batched.default(*compressed_M[:5], V)

@@ -25,7 +25,7 @@ LIB_TORCH = os.path.join(PKG_DIR, "_torch_ops.so")
 LIB_DIRECT = os.path.join(PKG_DIR, "_torch_direct" + sysconfig.get_config_var("EXT_SUFFIX"))
 BENCH_CLI = os.path.join(PKG_DIR, "macko_bench")
 
-CUDA_SOURCES = ["common.cu", "spmv.cu", "compress.cu", "decompress.cu", "plan.cu", "decode_glue.cu"]
+CUDA_SOURCES = ["common.cu", "spmv.cu", "windows.cu", "compress.cu", "decompress.cu", "plan.cu", "decode_glue.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",
@@ -56,7 +56,7 @@ def _nvcc() -> str:
 
 
 def build_core(force: bool = False, verbose: bool = False) -> str:
-    headers = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "plan.cuh"), os.path.join(INCLUDE, "macko_b200.h")]
+    headers = [os.path.join(CSRC, h) for h in ("common.cuh", "plan.cuh", "unit.cuh", "windows.cuh")] + [os.path.join(INCLUDE, "macko_b200.h")]
     sources = [os.path.join(CSRC, s) for s in CUDA_SOURCES]
     if not force and _newer(LIB_CORE, sources + headers + [__file__]):
         return LIB_CORE

@@ -55,6 +55,10 @@ SIGNATURES = {
     "macko_spmv_fp16_tuned": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _f, _f, _vp, _int, _int, _int, _int]),
     "macko_spmv_shape": (_int, [_i64, _i64, _i64, _int, _vp, _vp]),
     "macko_spmm_fp16": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _i64, _f, _f, _vp]),
+    "macko_spmm_windows_bytes": (_i64, [_i64, _i64, _i64]),
+    "macko_spmm_windows": (_int, [_vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp]),
+    "macko_spmm_windowed_workspace_bytes": (_i64, [_i64, _i64, _i64, _i64]),
+    "macko_spmm_fp16_windowed": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp, _i64, _f, _f, _vp, _i64, _u32, _vp]),
     "macko_decompress_fp16": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
     "macko_compress_count": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "macko_compress_workspace_bytes": (_i64, [_i64]),

@@ -1,5 +1,6 @@
 #include "common.cuh"
 
+#include <cstdlib>
 #include <mutex>
 
 namespace macko {
@@ -37,6 +38,37 @@ int current_device_info(const DeviceInfo **out)
     }
     *out = &d;
     return MACKO_OK;
+}
+
+int check_product_args(const void *values, const void *deltas, const int32_t *ri, int64_t rows, int64_t cols,
+                       int64_t padded_count, const void *x, const void *y)
+{
+    if (rows < 0 || cols < 0 || padded_count < 0)
+        return fail(MACKO_ERR_INVALID_ARGUMENT, "negative size (rows=%lld cols=%lld P=%lld)",
+                    (long long)rows, (long long)cols, (long long)padded_count);
+    if (rows >= (1LL << 31) - 64 || cols >= (1LL << 30) || padded_count >= (1LL << 31))
+        return fail(MACKO_ERR_SIZE_OVERFLOW, "rows=%lld cols=%lld P=%lld exceed 31-bit indexing",
+                    (long long)rows, (long long)cols, (long long)padded_count);
+    if (padded_count % 8 != 0)
+        return fail(MACKO_ERR_INVALID_ARGUMENT, "padded_count %lld is not a multiple of 8", (long long)padded_count);
+    if (rows == 0) return MACKO_OK;
+    if (!ri || !y) return fail(MACKO_ERR_INVALID_ARGUMENT, "null row_indices or y");
+    if (cols > 0 && !x) return fail(MACKO_ERR_INVALID_ARGUMENT, "null x");
+    if (padded_count > 0 && (!values || !deltas)) return fail(MACKO_ERR_INVALID_ARGUMENT, "null values or deltas");
+    if (!aligned(values, 16)) return fail(MACKO_ERR_MISALIGNED, "values must be 16-byte aligned");
+    if (!aligned(deltas, 4)) return fail(MACKO_ERR_MISALIGNED, "deltas must be 4-byte aligned");
+    if (!aligned(ri, 4)) return fail(MACKO_ERR_MISALIGNED, "row_indices must be 4-byte aligned");
+    if (!aligned(x, 2) || !aligned(y, 2)) return fail(MACKO_ERR_MISALIGNED, "x and y must be 2-byte aligned");
+    return MACKO_OK;
+}
+
+bool use_pdl()
+{
+    static const bool on = [] {
+        const char *v = getenv("MACKO_SPMV_PDL");
+        return !(v && v[0] == '0');
+    }();
+    return on;
 }
 
 }  // namespace macko

@@ -29,6 +29,14 @@ int current_device_info(const DeviceInfo **out);
 // shared by the compressor and the plan builder).
 int launch_row_scan(int *counts, int rows, cudaStream_t stream);
 
+// Sizes, null pointers and alignment of the arguments that every product takes.
+int check_product_args(const void *values, const void *deltas, const int32_t *ri, int64_t rows, int64_t cols,
+                       int64_t padded_count, const void *x, const void *y);
+
+// Overlap of consecutive launches (programmatic dependent launch) can be switched off with
+// MACKO_SPMV_PDL=0 in the environment, read once.
+bool use_pdl();
+
 inline bool aligned(const void *p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
 }  // namespace macko

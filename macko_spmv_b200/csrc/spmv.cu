@@ -31,11 +31,11 @@
 //     which balances matrices with very uneven rows; the compressed buffers stay untouched.
 #include "common.cuh"
 #include "plan.cuh"
+#include "unit.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include <cstdlib>
 #include <type_traits>
 
 namespace macko {
@@ -43,7 +43,6 @@ namespace {
 
 constexpr int kThreads = 512;        // threads per CTA
 constexpr int kWarpsPerCta = kThreads / 32;
-constexpr int kGroup = 8;            // stored elements per lane per sub-step (one 128-bit value load)
 
 // acc += fp16(low or high half of vword) * fp16(low half of xbits): the sm_100 mixed-precision FMA
 // (exact fp16 product accumulated in fp32, round to nearest); the halves are split inside the asm so
@@ -122,48 +121,6 @@ __device__ __forceinline__ void mask_unit_bytes(uint4 &v, unsigned &w, int lo, i
     v.y &= keep[1];
 }
 
-// acc += fp16(half VH of vword) * fp16(half XH of xword)
-template <int VH, int XH>
-__device__ __forceinline__ float fma_hh(float acc, unsigned vword, unsigned xword)
-{
-    if (VH == 0 && XH == 0)
-        asm("{.reg .b16 vl,vh,xl,xh; mov.b32 {vl,vh}, %1; mov.b32 {xl,xh}, %2; fma.rn.f32.f16 %0, vl, xl, %0;}" : "+f"(acc) : "r"(vword), "r"(xword));
-    else if (VH == 0 && XH == 1)
-        asm("{.reg .b16 vl,vh,xl,xh; mov.b32 {vl,vh}, %1; mov.b32 {xl,xh}, %2; fma.rn.f32.f16 %0, vl, xh, %0;}" : "+f"(acc) : "r"(vword), "r"(xword));
-    else if (VH == 1 && XH == 0)
-        asm("{.reg .b16 vl,vh,xl,xh; mov.b32 {vl,vh}, %1; mov.b32 {xl,xh}, %2; fma.rn.f32.f16 %0, vh, xl, %0;}" : "+f"(acc) : "r"(vword), "r"(xword));
-    else
-        asm("{.reg .b16 vl,vh,xl,xh; mov.b32 {vl,vh}, %1; mov.b32 {xl,xh}, %2; fma.rn.f32.f16 %0, vh, xh, %0;}" : "+f"(acc) : "r"(vword), "r"(xword));
-    return acc;
-}
-
-// BV consecutive fp16 values (BV = 2, 4 or 8) from shared memory into BV/2 words
-template <int BV>
-__device__ __forceinline__ void lds_vec(unsigned addr, unsigned (&r)[BV / 2])
-{
-    if constexpr (BV == 2)
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r[0]) : "r"(addr));
-    else if constexpr (BV == 4)
-        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-    else
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-
-__device__ __forceinline__ uint4 ldg_stream_v4(const uint4 *p)
-{
-    uint4 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-    return r;
-}
-
-__device__ __forceinline__ unsigned ldg_stream_u32(const unsigned *p)
-{
-    unsigned r;
-    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(r) : "l"(p));
-    return r;
-}
-
 __device__ __forceinline__ unsigned lds_u16(unsigned addr)
 {
     unsigned r;
@@ -171,35 +128,8 @@ __device__ __forceinline__ unsigned lds_u16(unsigned addr)
     return r;
 }
 
-// c + byte `J` of a: one integer dot-product instruction extracts the byte and adds the base, and it
-// does not run on the (half-rate) integer ALU pipe the rest of the index arithmetic competes for.
-template <int J, int M = 1>
-__device__ __forceinline__ int add_byte(unsigned a, int c)
-{
-    return __dp4a(a, (unsigned)M << (8 * J), (unsigned)c);   // c + M * byte J of a
-}
-
-// Zero the deltas and the fp16 values of one 8-element unit outside element range [lo, hi).
-__device__ __forceinline__ void mask_unit(uint4 &v, unsigned &w, int lo, int hi)
-{
-    lo = min(max(lo, 0), kGroup);
-    hi = min(max(hi, 0), kGroup);
-    unsigned m = lo >= kGroup ? 0u : (0xffffffffu << (4 * lo));
-    if (hi < kGroup) m &= ~(0xffffffffu << (4 * hi));
-    w &= m;
-    unsigned *vw = reinterpret_cast<unsigned *>(&v);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const unsigned lo16 = ((m >> (8 * j)) & 1u) * 0xffffu;
-        const unsigned hi16 = ((m >> (8 * j + 4)) & 1u) * 0xffff0000u;
-        vw[j] &= (lo16 | hi16);
-    }
-}
-
 // Where a row-sharded launch delivers its slice of y: the full-y buffer of every rank (peer-mapped
 // device pointers) and every rank's flag words. world == 0 for an ordinary launch.
-template <int V> struct Int { static constexpr int value = V; };
-
 // A virtual row of a planned launch is done (called by the leader lane of its group): a whole row goes to
 // y; a segment of a cut row leaves its fp32 sum in the plan, where plan_combine_kernel adds the segments of
 // every cut row in segment order once the product kernel has finished.
@@ -825,17 +755,6 @@ __global__ void peer_wait_kernel(unsigned *flags, int world, unsigned spin_limit
     flags[world + 2] = 1u + (unsigned)p;   // gave up: the host can read which rank never arrived
 }
 
-// Overlap of consecutive launches (programmatic dependent launch) can be switched off with
-// MACKO_SPMV_PDL=0 in the environment, read once.
-bool use_pdl()
-{
-    static const bool on = [] {
-        const char *v = getenv("MACKO_SPMV_PDL");
-        return !(v && v[0] == '0');
-    }();
-    return on;
-}
-
 template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
@@ -985,34 +904,6 @@ int launch_batched(const void *values, const void *deltas, const int32_t *ri, in
                 : launch<8, 1, true, false, BV>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta, stream, dev, 0, Peers{}, batch);
 }
 
-int check_args(const void *values, const void *deltas, const int32_t *ri, int64_t rows, int64_t cols,
-               int64_t padded_count, const void *x, const void *y)
-{
-    if (rows < 0 || cols < 0 || padded_count < 0)
-        return fail(MACKO_ERR_INVALID_ARGUMENT, "negative size (rows=%lld cols=%lld P=%lld)",
-                    (long long)rows, (long long)cols, (long long)padded_count);
-    if (rows >= (1LL << 31) - 64 || cols >= (1LL << 30) || padded_count >= (1LL << 31))
-        return fail(MACKO_ERR_SIZE_OVERFLOW, "rows=%lld cols=%lld P=%lld exceed 31-bit indexing",
-                    (long long)rows, (long long)cols, (long long)padded_count);
-    if (padded_count % 8 != 0)
-        return fail(MACKO_ERR_INVALID_ARGUMENT, "padded_count %lld is not a multiple of 8", (long long)padded_count);
-    if (rows == 0) return MACKO_OK;
-    if (!ri || !y) return fail(MACKO_ERR_INVALID_ARGUMENT, "null row_indices or y");
-    if (cols > 0 && !x) return fail(MACKO_ERR_INVALID_ARGUMENT, "null x");
-    if (padded_count > 0 && (!values || !deltas)) return fail(MACKO_ERR_INVALID_ARGUMENT, "null values or deltas");
-    if (!aligned(values, 16)) return fail(MACKO_ERR_MISALIGNED, "values must be 16-byte aligned");
-    if (!aligned(deltas, 4)) return fail(MACKO_ERR_MISALIGNED, "deltas must be 4-byte aligned");
-    if (!aligned(ri, 4)) return fail(MACKO_ERR_MISALIGNED, "row_indices must be 4-byte aligned");
-    if (!aligned(x, 2) || !aligned(y, 2)) return fail(MACKO_ERR_MISALIGNED, "x and y must be 2-byte aligned");
-    return MACKO_OK;
-}
-
-}  // namespace
-}  // namespace macko
-
-namespace macko {
-namespace {
-
 int check_flags(uint32_t flags)
 {
     if (flags & ~(uint32_t)MACKO_SPMV_MATRIX_IMMUTABLE)
@@ -1026,7 +917,7 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
                  int64_t rows, int64_t cols, int64_t padded_count,
                  const void *x, void *y, float alpha, float beta, uint32_t flags, void *stream)
 {
-    int st = check_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
+    int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
     if (st == MACKO_OK) st = check_flags(flags);
     if (st != MACKO_OK) return st;
     if (rows == 0) return MACKO_OK;
@@ -1058,7 +949,7 @@ int macko_spmv_fp16_tuned(const void *values, const void *deltas, const int32_t 
                           int lanes_per_row, int steps_in_flight, int x_in_shared, int ctas_per_sm)
 {
     using namespace macko;
-    int st = check_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
+    int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
     if (st != MACKO_OK) return st;
     if (rows == 0) return MACKO_OK;
     if (ctas_per_sm < 0) return fail(MACKO_ERR_INVALID_ARGUMENT, "ctas_per_sm must be >= 0");
@@ -1111,7 +1002,7 @@ int macko_spmv_fp16_planned(const void *values, const void *deltas, const int32_
                             const void *x, void *y, float alpha, float beta, uint32_t flags, void *stream)
 {
     using namespace macko;
-    int st = check_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
+    int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
     if (st == MACKO_OK) st = check_flags(flags);
     if (st != MACKO_OK) return st;
     if (!plan || !info) return fail(MACKO_ERR_INVALID_ARGUMENT, "null plan or plan info");
@@ -1185,7 +1076,7 @@ int macko_spmm_fp16(const void *values, const void *deltas, const int32_t *row_i
     using namespace macko;
     if (batch < 0) return fail(MACKO_ERR_INVALID_ARGUMENT, "negative batch %lld", (long long)batch);
     if (batch == 0) return MACKO_OK;   // nothing to read or write: x and y may be null
-    int st = check_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
+    int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
     if (st != MACKO_OK) return st;
     if (rows == 0) return MACKO_OK;
     const DeviceInfo *dev = nullptr;
@@ -1243,7 +1134,7 @@ int macko_spmv_fp16_scatter_ex(const void *values, const void *deltas, const int
     peers.rank = rank;
     peers.spin_limit = spin_limit == 0 ? kDefaultSpinLimit : spin_limit;
     peers.deferred = (flags & MACKO_SCATTER_DEFERRED_WAIT) ? 1 : 0;
-    int st = check_args(values, deltas, row_indices, rows, cols, padded_count, x, peer_y[rank]);
+    int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, peer_y[rank]);
     if (st != MACKO_OK) return st;
     const DeviceInfo *dev = nullptr;
     st = current_device_info(&dev);

@@ -231,6 +231,46 @@ at::Tensor multiply_batched_cuda(const at::Tensor &values, const at::Tensor &del
     return y;
 }
 
+// Column windows of a compressed matrix for multiply_windowed, as a byte buffer on its device.
+at::Tensor windows_build_cuda(const at::Tensor &deltas, const at::Tensor &ri, int64_t rows, int64_t cols)
+{
+    TORCH_CHECK(deltas.is_cuda() && ri.is_cuda() && deltas.device() == ri.device(), "compressed buffers must be CUDA tensors");
+    TORCH_CHECK(deltas.dtype() == at::kByte && ri.dtype() == at::kInt, "M_deltas must be uint8 and M_row_indices int32");
+    TORCH_CHECK(deltas.is_contiguous() && ri.is_contiguous(), "compressed buffers must be contiguous");
+    TORCH_CHECK(rows >= 0 && cols >= 0 && ri.numel() == rows + 1 && deltas.numel() % 4 == 0, "sizes are not those of a MACKO matrix");
+    const int64_t bytes = macko_spmm_windows_bytes(rows, cols, deltas.numel() * 2);
+    TORCH_CHECK(bytes >= 0, "macko_spmm_windows_bytes: ", macko_last_error());
+    const c10::cuda::CUDAGuard guard(deltas.device());
+    at::Tensor windows = at::empty({bytes}, deltas.options());
+    check_status(macko_spmm_windows(deltas.data_ptr(), ri.data_ptr<int32_t>(), rows, cols, deltas.numel() * 2, windows.data_ptr(),
+                                    bytes, c10::cuda::getCurrentCUDAStream()),
+                 "macko_spmm_windows");
+    return windows;
+}
+
+// Y[batch, rows] for V[batch, cols] over the matrix's column windows. The partial sums are scratch of this call alone.
+at::Tensor multiply_windowed_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
+                                  int64_t rows, int64_t cols, const at::Tensor &windows, const at::Tensor &V, bool frozen)
+{
+    check_compressed(values, deltas, ri, rows, cols);
+    TORCH_CHECK(values.dtype() == at::kHalf && V.dtype() == at::kHalf, "M and V must be torch.half");
+    TORCH_CHECK(V.is_cuda() && V.device() == values.device() && windows.is_cuda() && windows.device() == values.device(),
+                "V and the windows must be on the device of M");
+    TORCH_CHECK(V.is_contiguous() && windows.is_contiguous(), "V and the windows must be contiguous");
+    TORCH_CHECK(V.dim() == 2 && V.size(1) == cols, "V must have shape [batch, M_cols]");
+    const int64_t bytes = macko_spmm_windowed_workspace_bytes(rows, cols, values.numel(), V.size(0));
+    TORCH_CHECK(bytes >= 0, "macko_spmm_windowed_workspace_bytes: sizes out of range");
+    const c10::cuda::CUDAGuard guard(values.device());
+    at::Tensor y = at::empty({V.size(0), rows}, values.options());
+    const at::Tensor partial = at::empty({bytes}, deltas.options());
+    check_status(macko_spmm_fp16_windowed(values.data_ptr(), deltas.data_ptr(), ri.data_ptr<int32_t>(), rows, cols, values.numel(),
+                                          windows.data_ptr(), windows.numel() * windows.element_size(), V.data_ptr(), y.data_ptr(), V.size(0), 1.0f, 0.0f,
+                                          partial.data_ptr(), bytes, frozen ? MACKO_SPMV_MATRIX_IMMUTABLE : 0u,
+                                          c10::cuda::getCurrentCUDAStream()),
+                 "macko_spmm_fp16_windowed");
+    return y;
+}
+
 at::Tensor decompress_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
                            int64_t rows, int64_t cols)
 {
@@ -391,6 +431,9 @@ TORCH_LIBRARY(macko_spmv, m)
           "Tensor(a!) y, float alpha, float beta) -> ()");
     m.def("compress_dense(Tensor M) -> (Tensor, Tensor, Tensor)");
     m.def("multiply_batched(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor V) -> Tensor");
+    m.def("windows_build(Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols) -> Tensor");
+    m.def("multiply_windowed(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor windows, "
+          "Tensor V, bool frozen) -> Tensor");
     m.def("decompress(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols) -> Tensor");
     m.def("multiply_ex(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor V, "
           "Tensor(a!) y, float alpha, float beta, int flags) -> ()");
@@ -413,6 +456,8 @@ TORCH_LIBRARY_IMPL(macko_spmv, CUDA, m)
     m.impl("multiply_out", &multiply_out_cuda);
     m.impl("compress_dense", &compress_cuda);
     m.impl("multiply_batched", &multiply_batched_cuda);
+    m.impl("windows_build", &windows_build_cuda);
+    m.impl("multiply_windowed", &multiply_windowed_cuda);
     m.impl("decompress", &decompress_cuda);
     m.impl("multiply_ex", &multiply_ex_cuda);
     m.impl("multiply_frozen", &multiply_frozen_cuda);
