@@ -188,7 +188,7 @@ def test_route_of_a_frozen_matrix(monkeypatch):
     x = V(17, grad=True)
     macko_spmv.multiply_batched(frozen, x).sum().backward()
     assert float((x.grad.float() - M.float().sum(0)).abs().max()) < 0.1
-    for batch in (3, 8, 9, 30):
+    for batch in (3, 8, 9):
         _check(macko_spmv.multiply_batched(frozen, V(batch)), M, V(batch), f"frozen, batch {batch}")
     # a matrix written after freeze(): another one in the same buffers
     turned = M.roll(1, 0).contiguous()
