@@ -43,6 +43,7 @@ namespace {
 
 constexpr int kThreads = 512;        // threads per CTA
 constexpr int kWarpsPerCta = kThreads / 32;
+constexpr int kThreadsPerSm = 1024;  // at 64 registers each
 
 // acc += fp16(low or high half of vword) * fp16(low half of xbits): the sm_100 mixed-precision FMA
 // (exact fp16 product accumulated in fp32, round to nearest); the halves are split inside the asm so
@@ -224,8 +225,9 @@ struct Extra {
 // EARLY the caller has declared the matrix immutable: the first matrix loads are issued before the wait for the
 //       previous kernel of the stream and before x is staged (a separate instantiation, so that the default
 //       launch keeps the simpler code: wait, stage x, then walk the rows)
-template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false>
-__global__ void __launch_bounds__(kThreads, 2)
+// T     threads of a CTA: 512, two CTAs on an SM, or 1024, one CTA and one copy of x (see kWideSmem)
+template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads>
+__global__ void __launch_bounds__(T, kThreadsPerSm / T)
 spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
             const int *__restrict__ ri, const __half *__restrict__ x, __half *__restrict__ y,
             int rows, int cols, int stored, float alpha, float beta, int batch, unsigned flags,
@@ -255,8 +257,8 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     // ---- this warp's work: a contiguous row range dealt in blocks of K rows (so that the groups of a warp
     //      run out of rows together), or, planned, every n_warps-th block of K virtual rows of the sorted
     //      list, the direction alternating from round to round (longest first: the ends even out) ------------
-    const long long n_warps = (long long)gridDim.x * kWarpsPerCta;
-    const long long warp_id = (long long)blockIdx.x * kWarpsPerCta + (tid >> 5);
+    const long long n_warps = (long long)gridDim.x * (T / 32);
+    const long long warp_id = (long long)blockIdx.x * (T / 32) + (tid >> 5);
     int row_next, row_hi;   // plain: rows [row_next, row_hi); planned: positions in the warp's sequence
     if constexpr (PLAN) {
         const int V = plan.n_virtual;
@@ -287,9 +289,9 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     // PEER: rows of the whole CTA (its warps own consecutive ranges) and the staging area for their y
     int cta_row_lo = 0, cta_row_hi = 0;
     if constexpr (PEER) {
-        const unsigned cta_w0 = blockIdx.x * kWarpsPerCta;
+        const unsigned cta_w0 = blockIdx.x * (T / 32);
         cta_row_lo = block_boundary<K>(rows, cta_w0, (unsigned)n_warps);
-        cta_row_hi = block_boundary<K>(rows, cta_w0 + kWarpsPerCta, (unsigned)n_warps);
+        cta_row_hi = block_boundary<K>(rows, cta_w0 + (T / 32), (unsigned)n_warps);
     }
     __half *ystage = reinterpret_cast<__half *>(smem + (((size_t)(kXPadFront + cols + kXPadBack) * sizeof(__half) + 15) & ~(size_t)15));
 
@@ -337,13 +339,13 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     if (BV > 1) {
         __half *xs = reinterpret_cast<__half *>(smem);
         const int n_total = (kXPadFront + cols + kXPadBack) * BV;
-        for (int i = tid; i < kXPadFront * BV; i += kThreads) xs[i] = __ushort_as_half(0);
-        for (int i = (kXPadFront + cols) * BV + tid; i < n_total; i += kThreads) xs[i] = __ushort_as_half(0);
+        for (int i = tid; i < kXPadFront * BV; i += T) xs[i] = __ushort_as_half(0);
+        for (int i = (kXPadFront + cols) * BV + tid; i < n_total; i += T) xs[i] = __ushort_as_half(0);
 #pragma unroll
         for (int b = 0; b < BV; ++b) {
             const __half *xb = x + (size_t)b * cols;
 #pragma unroll 4
-            for (int c = tid; c < cols; c += kThreads)
+            for (int c = tid; c < cols; c += T)
                 xs[(size_t)(kXPadFront + c) * BV + b] = b < batch ? xb[c] : __ushort_as_half(0);
         }
         __syncthreads();
@@ -351,9 +353,9 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
         __half *xs = reinterpret_cast<__half *>(smem);
         const int n_total = kXPadFront + cols + kXPadBack;
 #pragma unroll 1
-        for (int i = tid; i < kXPadFront; i += kThreads) xs[i] = __ushort_as_half(0);
+        for (int i = tid; i < kXPadFront; i += T) xs[i] = __ushort_as_half(0);
 #pragma unroll 1
-        for (int i = kXPadFront + cols + tid; i < n_total; i += kThreads) xs[i] = __ushort_as_half(0);
+        for (int i = kXPadFront + cols + tid; i < n_total; i += T) xs[i] = __ushort_as_half(0);
         if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
             // 16-byte asynchronous copies global -> shared: no registers, all of a thread's copies in flight
             // together, and the matrix loads issued above stay in flight beside them
@@ -361,15 +363,15 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
             const unsigned dst0 = (unsigned)x_base + 2u * kXPadFront;
             const char *src0 = reinterpret_cast<const char *>(x);
 #pragma unroll 1
-            for (int i = tid; i < n_vec; i += kThreads)
+            for (int i = tid; i < n_vec; i += T)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + 16u * (unsigned)i), "l"(src0 + 16 * (size_t)i) : "memory");
 #pragma unroll 1
-            for (int i = (n_vec << 3) + tid; i < cols; i += kThreads) xs[kXPadFront + i] = x[i];
+            for (int i = (n_vec << 3) + tid; i < cols; i += T) xs[kXPadFront + i] = x[i];
             asm volatile("cp.async.commit_group;" ::: "memory");
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else {
 #pragma unroll 1
-            for (int i = tid; i < cols; i += kThreads) xs[kXPadFront + i] = x[i];
+            for (int i = tid; i < cols; i += T) xs[kXPadFront + i] = x[i];
         }
         __syncthreads();
     }
@@ -633,7 +635,7 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
         const int n_mine = cta_row_hi - cta_row_lo;
         {
             __half *dst = peers.y[peers.rank] + peers.row_offset + cta_row_lo;
-            for (int i = tid; i < n_mine; i += kThreads) dst[i] = ystage[i];
+            for (int i = tid; i < n_mine; i += T) dst[i] = ystage[i];
         }
         __shared__ unsigned last_cta_seq;
         __shared__ unsigned is_last_cta;
@@ -648,25 +650,25 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
         __syncthreads();
         if (is_last_cta) {
             // Forward this rank's slice (read around L1: other SMs wrote it) to every other rank; chunk c of the
-            // slice goes to all peers before chunk c + kThreads, so the stores to different peers are in flight together.
+            // slice goes to all peers before chunk c + T, so the stores to different peers are in flight together.
             const unsigned short *src = reinterpret_cast<const unsigned short *>(peers.y[peers.rank] + peers.row_offset);
             bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
             for (int p = 0; p < peers.world; ++p)
                 vec = vec && ((reinterpret_cast<uintptr_t>(peers.y[p] + peers.row_offset) & 15) == 0);
             if (vec) {
                 const int chunks = rows >> 3;
-                for (int c = tid; c < chunks; c += kThreads) {
+                for (int c = tid; c < chunks; c += T) {
                     const uint4 val = __ldcg(reinterpret_cast<const uint4 *>(src) + c);
                     for (int p = 0; p < peers.world; ++p)
                         if (p != peers.rank) reinterpret_cast<uint4 *>(peers.y[p] + peers.row_offset)[c] = val;
                 }
-                for (int i = (chunks << 3) + tid; i < rows; i += kThreads) {
+                for (int i = (chunks << 3) + tid; i < rows; i += T) {
                     const unsigned short val = __ldcg(src + i);
                     for (int p = 0; p < peers.world; ++p)
                         if (p != peers.rank) reinterpret_cast<unsigned short *>(peers.y[p] + peers.row_offset)[i] = val;
                 }
             } else {
-                for (int i = tid; i < rows; i += kThreads) {
+                for (int i = tid; i < rows; i += T) {
                     const unsigned short val = __ldcg(src + i);
                     for (int p = 0; p < peers.world; ++p)
                         if (p != peers.rank) reinterpret_cast<unsigned short *>(peers.y[p] + peers.row_offset)[i] = val;
@@ -755,27 +757,27 @@ __global__ void peer_wait_kernel(unsigned *flags, int world, unsigned spin_limit
     flags[world + 2] = 1u + (unsigned)p;   // gave up: the host can read which rank never arrived
 }
 
-template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY>
+template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra);
 
 // The instantiation with or without early matrix loads, by the immutable-matrix flag of the call.
-template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16>
+template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads>
 int launch(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
            const void *x, void *y, float alpha, float beta, cudaStream_t stream,
            const DeviceInfo &dev, int ctas_per_sm, const Peers &peers = Peers{}, int batch = 1, const Extra &extra = Extra{})
 {
     if constexpr (BV == 1) {
         if (extra.flags & MACKO_SPMV_MATRIX_IMMUTABLE)
-            return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, true>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
+            return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, true, T>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
                                                                          stream, dev, ctas_per_sm, peers, batch, extra);
     }
-    return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, false>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
+    return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, false, T>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
                                                                   stream, dev, ctas_per_sm, peers, batch, extra);
 }
 
-template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY>
+template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra)
@@ -786,13 +788,13 @@ int launch_variant(const void *values, const void *deltas, const int32_t *ri, in
     if (smem > (size_t)dev.max_smem_optin)
         return fail(MACKO_ERR_INVALID_ARGUMENT, "the launch needs %lld bytes of shared memory, the device offers %d (cols=%d)",
                     (long long)smem, dev.max_smem_optin, cols);
-    auto kernel = spmv_kernel<L, NPAIR, XS, PEER, BV, PLAN, VT, EARLY>;
+    auto kernel = spmv_kernel<L, NPAIR, XS, PEER, BV, PLAN, VT, EARLY, T>;
     if (smem > 48 * 1024) {
         // Idempotent and cheap; set on every call so that every device is covered.
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     }
-    int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 2;
+    int per_sm = ctas_per_sm > 0 ? ctas_per_sm : kThreadsPerSm / T;
     if (smem > 0) per_sm = max(1, min(per_sm, (int)((size_t)dev.max_smem_optin / (smem + 1024))));
     // Always a whole number of CTAs per SM: with fewer CTAs than that, some SMs would hold twice the rows
     // of others. Only matrices with fewer row groups than CTAs get a smaller grid (one group per CTA).
@@ -802,7 +804,7 @@ int launch_variant(const void *values, const void *deltas, const int32_t *ri, in
     if (groups < ctas) ctas = groups < 1 ? 1 : groups;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(T);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -866,6 +868,15 @@ int launch_l(int L, int D, const void *values, const void *deltas, const int32_t
 //   * rows shorter than half a sub-step shrink the group further;
 //   * six units in flight once a row holds more than three sub-steps, four above one, else two.
 struct Shape { int L, D; };
+
+// Above this size of x a warp-per-row launch takes CTAs of 1024 threads that share one copy of x instead of two CTAs of 512
+// with a copy each. Two copies of more than 65 KB leave the SM's first-level cache 92 KB or less (28 KB from 41 000 columns on),
+// and the matrix data that its 1024 threads keep in flight, 120 KB with six units a lane, passes through that cache; from
+// 57408 columns on only one CTA of 512 threads fits at all. 1024 / 512 threads (B200, graph of products, matrices declared
+// immutable, us): 12288x49152 d = 0.5 158.6 / 166.1, d = 0.1 46.2 / 49.5, 3000x40000 d = 0.5 37.8 / 40.1; below the line the
+// shared barrier costs as much as it gives: 4096x32768 39.8 / 39.8, 8192x24576 58.1 / 59.0, 4096x11008 d = 0.5 16.1 / 15.2.
+// Groups of fewer lanes are left with two CTAs (not measured).
+constexpr size_t kWideSmem = 65 * 1024;
 Shape choose_shape(long long rows, long long cols, long long padded, int resident_warps)
 {
     const long long avg_row = rows > 0 ? padded / rows : 0;
@@ -933,6 +944,9 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Extra extra = {};
     extra.flags = flags;
+    if (xs && L == 32 && D == 6 && smem > kWideSmem)
+        return launch<32, 3, true, false, 1, false, VT, 2 * kThreads>(values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y,
+                                                                      alpha, beta, s, *dev, 0, Peers{}, 1, extra);
     if (xs)
         return launch_l<true, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);
     return launch_l<false, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);
