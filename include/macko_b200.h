@@ -242,6 +242,14 @@ int macko_decompress_fp16(const void *values, const void *deltas, const int32_t 
 int macko_compress_count(const void *dense, int64_t rows, int64_t cols,
                          int32_t *row_indices, void *stream);
 
+/*
+ * The same (int8 matrices: value_bytes 1, 16-bit ones: 2), and the unpadded stored count also goes to *total, pinned host memory
+ * (cudaHostAlloc or registered): a host that has set it to -1 before the call can wait for the count by watching that word,
+ * which takes no copy and no synchronisation of the stream. *total is written once, before the stream passes this call.
+ */
+int macko_compress_count_total(const void *dense, int64_t rows, int64_t cols, int32_t value_bytes, int32_t *row_indices,
+                               int32_t *total, void *stream);
+
 /* Bytes of scratch macko_compress_emit needs for a padded stored count P. */
 int64_t macko_compress_workspace_bytes(int64_t padded_count);
 

@@ -61,6 +61,7 @@ SIGNATURES = {
     "macko_spmm_fp16_windowed": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp, _i64, _f, _f, _vp, _i64, _u32, _vp]),
     "macko_decompress_fp16": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
     "macko_compress_count": (_int, [_vp, _i64, _i64, _vp, _vp]),
+    "macko_compress_count_total": (_int, [_vp, _i64, _i64, _i32, _vp, _vp, _vp]),
     "macko_compress_workspace_bytes": (_i64, [_i64]),
     "macko_compress_emit": (_int, [_vp, _i64, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp]),
     "macko_compress_emit_bf16": (_int, [_vp, _i64, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp]),

@@ -26,8 +26,8 @@ struct DeviceInfo {
 int current_device_info(const DeviceInfo **out);
 
 // In-place inclusive prefix sum over counts[1..rows] with counts[0] = 0 (one CTA; defined in compress.cu,
-// shared by the compressor and the plan builder).
-int launch_row_scan(int *counts, int rows, cudaStream_t stream);
+// shared by the compressor and the plan builder). `total`: where the sum goes as well, or null.
+int launch_row_scan(int *counts, int rows, cudaStream_t stream, int *total = nullptr);
 
 // Sizes, null pointers and alignment of the arguments that every product takes.
 int check_product_args(const void *values, const void *deltas, const int32_t *ri, int64_t rows, int64_t cols,

@@ -131,6 +131,7 @@ template <bool I8>
 __global__ void __launch_bounds__(kThreads)
 count_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, int cols, bool vec_ok, int *__restrict__ counts)
 {
+    asm volatile("griddepcontrol.launch_dependents;");
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -434,8 +435,11 @@ emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, 
 // In-place inclusive prefix sum over counts[1..rows]; counts[0] = 0. One CTA; a warp takes 512 consecutive entries per
 // iteration (four 16-byte loads per lane, all in flight together), the CTA 16384: the iterations are a serial chain of
 // loads, shuffles and barriers, and most matrices need only one.
-__global__ void __launch_bounds__(1024) scan_rows_kernel(int *__restrict__ ri, int rows)
+// Launched as a programmatic dependent: its CTA is in place when the last counts are written. With `total` (host memory that
+// the device can write) the sum goes there as well, for a host that waits for it without a copy.
+__global__ void __launch_bounds__(1024) scan_rows_kernel(int *__restrict__ ri, int rows, int *total)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ int warp_sums[32];
     __shared__ int carry_s;
     constexpr int kVecs = 4, kPerWarp = 128 * kVecs;
@@ -498,6 +502,7 @@ __global__ void __launch_bounds__(1024) scan_rows_kernel(int *__restrict__ ri, i
         if (tid == 31) carry_s += sum;
         __syncthreads();
     }
+    if (total != nullptr && tid == 0) *reinterpret_cast<volatile int *>(total) = carry_s;
 }
 
 // Largest padded count of macko_compress_emit_static (part of its contract).
@@ -524,16 +529,26 @@ int launch_error(const char *what)
 
 }  // namespace
 
-int launch_row_scan(int *counts, int rows, cudaStream_t stream)
+int launch_row_scan(int *counts, int rows, cudaStream_t stream, int *total)
 {
-    scan_rows_kernel<<<1, 1024, 0, stream>>>(counts, rows);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = use_pdl() ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, scan_rows_kernel, counts, rows, total);
+    if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "row scan launch: %s", cudaGetErrorString(e));
     return launch_error("row scan launch");
 }
 
 }  // namespace macko
 
 template <bool I8>
-static int compress_count_typed(const void *dense, int64_t rows, int64_t cols, int32_t *row_indices, void *stream)
+static int compress_count_typed(const void *dense, int64_t rows, int64_t cols, int32_t *row_indices, int32_t *total, void *stream)
 {
     using namespace macko;
     using Element = typename Raw<I8>::Element;
@@ -549,7 +564,7 @@ static int compress_count_typed(const void *dense, int64_t rows, int64_t cols, i
         st = launch_error("compress count launch");
         if (st != MACKO_OK) return st;
     }
-    return launch_row_scan(row_indices, (int)rows, s);
+    return launch_row_scan(row_indices, (int)rows, s, total);
 }
 
 // Checks and launch shared by the emit entry points.
@@ -601,7 +616,24 @@ extern "C" {
 
 int macko_compress_count(const void *dense, int64_t rows, int64_t cols, int32_t *row_indices, void *stream)
 {
-    return compress_count_typed<false>(dense, rows, cols, row_indices, stream);
+    return compress_count_typed<false>(dense, rows, cols, row_indices, nullptr, stream);
+}
+
+int macko_compress_count_total(const void *dense, int64_t rows, int64_t cols, int32_t value_bytes, int32_t *row_indices,
+                               int32_t *total, void *stream)
+{
+    using namespace macko;
+    if (value_bytes != 1 && value_bytes != 2) return fail(MACKO_ERR_INVALID_ARGUMENT, "value_bytes must be 1 or 2 (got %d)", value_bytes);
+    if (!total) return fail(MACKO_ERR_INVALID_ARGUMENT, "null total");
+    if (!aligned(total, 4)) return fail(MACKO_ERR_MISALIGNED, "total must be 4-byte aligned");
+    void *device_total = nullptr;
+    const cudaError_t e = cudaHostGetDevicePointer(&device_total, total, 0);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return fail(MACKO_ERR_INVALID_ARGUMENT, "total is not host memory that the device can write: %s", cudaGetErrorString(e));
+    }
+    return value_bytes == 1 ? compress_count_typed<true>(dense, rows, cols, row_indices, static_cast<int32_t *>(device_total), stream)
+                            : compress_count_typed<false>(dense, rows, cols, row_indices, static_cast<int32_t *>(device_total), stream);
 }
 
 int64_t macko_compress_workspace_bytes(int64_t padded_count) { return padded_count < 0 ? 0 : padded_count; }
@@ -624,7 +656,7 @@ int macko_compress_emit_bf16(const void *dense, int64_t rows, int64_t cols, cons
 
 int macko_compress_count_int8(const void *dense, int64_t rows, int64_t cols, int32_t *row_indices, void *stream)
 {
-    return compress_count_typed<true>(dense, rows, cols, row_indices, stream);
+    return compress_count_typed<true>(dense, rows, cols, row_indices, nullptr, stream);
 }
 
 int macko_compress_emit_int8(const void *dense, int64_t rows, int64_t cols, const int32_t *row_indices,

@@ -1,0 +1,60 @@
+"""The stored count that the compressor leaves in pinned host memory (`macko_compress_count_total`), against the last row offset: row
+counts around the 512 that a warp and the 16384 that the CTA of the prefix sum takes at a time, empty matrices, both value
+widths, several threads at once."""
+import threading
+
+import pytest
+import torch
+
+import macko_spmv_b200 as macko_spmv
+from macko_spmv_b200 import cabi, workloads
+
+
+def test_refuses_before_touching_the_device():
+    lib = cabi.load()
+    a = 0x1000   # never dereferenced
+    assert lib.macko_compress_count_total(a, 4, 4, 4, a, a, None) == cabi.ERR_INVALID_ARGUMENT
+    assert lib.macko_compress_count_total(a, 4, 4, 2, a, None, None) == cabi.ERR_INVALID_ARGUMENT
+    assert lib.macko_compress_count_total(a, 4, 4, 2, a, a + 2, None) == cabi.ERR_MISALIGNED
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(0, 64), (5, 0), (1, 1), (511, 40), (512, 40), (16382, 24), (16383, 24), (16384, 24), (40001, 17)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.int8])
+def test_total_is_the_last_row_offset(rows, cols, dtype):
+    lib = cabi.load()
+    M = (workloads.bernoulli_matrix(rows, cols, 0.4, seed=rows + cols, device="cuda") * 20).to(dtype) if rows and cols else torch.empty(rows, cols, dtype=dtype, device="cuda")
+    ri = torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+    total = torch.full((1,), -1, dtype=torch.int32).pin_memory()
+    cabi.check(lib, lib.macko_compress_count_total(M.data_ptr(), rows, cols, M.element_size(), ri.data_ptr(), total.data_ptr(),
+                                                   torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    counts = torch.empty_like(ri)
+    count = lib.macko_compress_count_int8 if dtype is torch.int8 else lib.macko_compress_count
+    cabi.check(lib, count(M.data_ptr(), rows, cols, counts.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(ri, counts) and int(total[0]) == int(counts[rows])
+    values, deltas, row_indices = macko_spmv.compress(M)[:3]
+    assert values.numel() == (int(total[0]) + 7) // 8 * 8 == 2 * deltas.numel() and torch.equal(row_indices, ri)
+
+
+@pytest.mark.gpu
+def test_threads_and_streams_at_once():
+    mats = [workloads.bernoulli_matrix(700 + 13 * i, 900 + 7 * i, 0.1 + 0.1 * i, seed=i, device="cuda") for i in range(6)]
+    want = [macko_spmv.compress(M) for M in mats]
+    torch.cuda.synchronize()
+    got = [[None] * 8 for _ in mats]
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for k in range(8):
+                got[i][k] = macko_spmv.compress(mats[i])
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(mats))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for w, g in zip(want, got):
+        for c in g:
+            assert all(torch.equal(a, b) for a, b in zip(w[:3], c[:3]))
