@@ -205,6 +205,7 @@ __device__ __forceinline__ int block_boundary(int rows, unsigned w, unsigned n_w
 // What a launch carries besides the reference's arguments.
 struct Extra {
     unsigned flags;               // MACKO_SPMV_MATRIX_IMMUTABLE
+    int tail_rows;                // TAIL kernels only
     PlanView plan;                // planned launch: virtual rows instead of row_indices (PLAN kernels only)
 };
 
@@ -225,12 +226,13 @@ struct Extra {
 // EARLY the caller has declared the matrix immutable: the first matrix loads are issued before the wait for the
 //       previous kernel of the stream and before x is staged (a separate instantiation, so that the default
 //       launch keeps the simpler code: wait, stage x, then walk the rows)
+// TAIL  the last `tail_rows` rows are walked with a warp per row (see choose_tail)
 // T     threads of a CTA: 512, two CTAs on an SM, or 1024, one CTA and one copy of x (see kWideSmem)
-template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads>
+template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads, bool TAIL = false>
 __global__ void __launch_bounds__(T, kThreadsPerSm / T)
 spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
             const int *__restrict__ ri, const __half *__restrict__ x, __half *__restrict__ y,
-            int rows, int cols, int stored, float alpha, float beta, int batch, unsigned flags,
+            int rows, int cols, int stored, float alpha, float beta, int batch, unsigned flags, int tail_rows,
             const PeersArg<PEER> peers, const PlanArg<PLAN> plan)
 {
     static_assert(BV == 1 || (XS && !PEER), "batched products gather from shared memory and have no scatter epilogue");
@@ -238,14 +240,10 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     static_assert(VT == kF16 || (!PEER && BV == 1 && !PLAN), "bfloat16 and int8 values are built for the plain single-vector product");
     static_assert(!EARLY || BV == 1, "early matrix loads are built for the single-vector product");
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int STEP = kGroup * L;   // elements per group per sub-step
     constexpr int D = 2 * NPAIR;       // sub-steps per iteration
     constexpr int K = 32 / L;          // rows a warp walks at once
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int lig = lane & (L - 1);          // lane in group
-    const int group_lane0 = lane & ~(L - 1); // first lane of my group
-    constexpr unsigned kLeaders = (L == 32) ? 0x1u : (L == 16) ? 0x00010001u : (L == 8) ? 0x01010101u : 0x11111111u;
     unsigned short *y16 = reinterpret_cast<unsigned short *>(y);
 
     // Programmatic dependent launch: let the next kernel of the stream start occupying SMs as ours
@@ -276,8 +274,9 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
             if (last_blk == nb - 1) row_hi -= nb * K - V;   // the very last block may hold fewer than K
         }
     } else {
-        row_next = block_boundary<K>(rows, (unsigned)warp_id, (unsigned)n_warps);
-        row_hi = block_boundary<K>(rows, (unsigned)warp_id + 1u, (unsigned)n_warps);
+        const int rounds_rows = TAIL ? rows - tail_rows : rows;
+        row_next = block_boundary<K>(rounds_rows, (unsigned)warp_id, (unsigned)n_warps);
+        row_hi = block_boundary<K>(rounds_rows, (unsigned)warp_id + 1u, (unsigned)n_warps);
     }
     // sorted index of position p of this warp's sequence (planned)
     auto sorted_index = [&](int p) -> int {
@@ -295,44 +294,10 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     }
     __half *ystage = reinterpret_cast<__half *>(smem + (((size_t)(kXPadFront + cols + kXPadBack) * sizeof(__half) + 15) & ~(size_t)15));
 
-    // Window of 32 row offsets (planned: 32 virtual-row descriptors) held one per lane and read by shuffle.
-    int win_base = row_next;
-    int ri_reg = 0;      // plain: ri[win_base + lane]; planned: first stored element of the virtual row
-    unsigned pk_reg = 0; // planned: length | starting column << kPlanLenBits
-    auto load_window = [&]() {
-        if constexpr (PLAN) {
-            const int p = win_base + lane;
-            uint2 d = make_uint2(0u, 0u);
-            if (p < row_hi) d = __ldg(plan.desc + sorted_index(p));
-            ri_reg = (int)d.x;
-            pk_reg = d.y;
-        } else {
-            ri_reg = __ldg(ri + min(win_base + lane, rows));
-        }
-    };
-    if (row_next < row_hi) load_window();
-
-    // ---- per-group state ------------------------------------------------------------------------------
-    constexpr int LOG_STEP = (L == 32) ? 8 : (L == 16) ? 7 : (L == 8) ? 6 : 5;
-    int my_row = -1;   // plain: row being walked by my group (-1: none); planned: 0 while a virtual row is walked
-    unsigned out_word = 0u;   // planned: destination of the virtual row (a row of y, or a partial-sum slot)
-    // Element positions are unsigned: an iteration runs up to 1536 elements ahead of a count that may come close to 2^31.
-    unsigned begin = 0u;   // first stored element of the row
-    unsigned end = 0u;     // one past the last stored element
-    unsigned pos = 0u;     // first element of the group's next iteration (multiple of 8)
-    // Byte address (shared window, or byte offset from x - kXPadFront when x stays in global memory) of
-    // "column -1 + index in row" in front of the lane's unit of the next sub-step, less 14 per lane below
-    // it in the group: the lane totals that go through the scan carry +14 each (see the decode below).
     // x_base (the shared-window address of the front padding) is known before x is staged.
     const int x_base = (XS || BV > 1) ? (int)__cvta_generic_to_shared(smem) : 0;
     const int x_fold = (BV == 1) ? x_base : 0;   // batched: offsets stay per-vector and are scaled by BV at the gather
-    const unsigned lane_const = (unsigned)(x_fold + 2 * kXPadFront + 2 * lig);
     const unsigned a_max = (unsigned)(x_fold + 2 * (kXPadFront + cols));
-    unsigned run = 0u;
-    float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
-    float accb[BV][2];   // batched: per vector, even and odd elements
-#pragma unroll
-    for (int b = 0; b < BV; ++b) accb[b][0] = accb[b][1] = 0.f;
 
     // Stages x into shared memory, framed by zeros (one CTA-wide barrier at its end).
     auto stage_x = [&]() {
@@ -376,254 +341,306 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
         __syncthreads();
     }
     };
-    if constexpr (!EARLY) stage_x();
-    bool first_pass = EARLY;
-    for (;;) {
-        bool done = false;
-        // ---- groups that ran out of work finish their row and take the next one ---------------------
-        const bool need = pos >= end;
-        const unsigned needmask = __ballot_sync(0xffffffffu, need);
-        if (needmask) {
-            if constexpr (BV == 1) {
-                float total = (acc0 + acc1) + (acc2 + acc3);
-#pragma unroll
-                for (int o = L / 2; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-                if (need) {
-                    if (my_row >= 0 && lig == 0) {
-                        if constexpr (PLAN) {
-                            plan_row_done(plan, out_word, total, alpha, beta, y16, rows);
-                        } else if constexpr (PEER) {
-                            ystage[my_row - cta_row_lo] = __float2half_rn(alpha * total);   // delivered in bulk at the end
-                        } else {
-                            float r = alpha * total;
-                            if (beta != 0.f) r += beta * from_bits16<VT>(y16[my_row]);
-                            y16[my_row] = to_bits16<VT>(r);
-                        }
-                    }
-                    acc0 = acc1 = acc2 = acc3 = 0.f;
-                }
+    // Walks rows [row_next, row_hi) (planned: positions) with LN lanes per row. FIRST: the walk in front of which x is staged.
+    auto walk = [&](auto lanes_tag, auto first_tag, int row_next, int row_hi) {
+        constexpr int LN = decltype(lanes_tag)::value;
+        constexpr bool FIRST = decltype(first_tag)::value != 0;
+        constexpr int STEP = kGroup * LN;   // elements per group per sub-step
+        const int lig = lane & (LN - 1);          // lane in group
+        const int group_lane0 = lane & ~(LN - 1); // first lane of my group
+        constexpr unsigned leader_lanes = (LN == 32) ? 0x1u : (LN == 16) ? 0x00010001u : (LN == 8) ? 0x01010101u : 0x11111111u;
+        // Window of 32 row offsets (planned: 32 virtual-row descriptors) held one per lane and read by shuffle.
+        int win_base = row_next;
+        int ri_reg = 0;      // plain: ri[win_base + lane]; planned: first stored element of the virtual row
+        unsigned pk_reg = 0; // planned: length | starting column << kPlanLenBits
+        auto load_window = [&]() {
+            if constexpr (PLAN) {
+                const int p = win_base + lane;
+                uint2 d = make_uint2(0u, 0u);
+                if (p < row_hi) d = __ldg(plan.desc + sorted_index(p));
+                ri_reg = (int)d.x;
+                pk_reg = d.y;
             } else {
+                ri_reg = __ldg(ri + min(win_base + lane, rows));
+            }
+        };
+        if (row_next < row_hi) load_window();
+
+        // ---- per-group state ------------------------------------------------------------------------------
+        constexpr int LOG_STEP = (LN == 32) ? 8 : (LN == 16) ? 7 : (LN == 8) ? 6 : 5;
+        int my_row = -1;   // plain: row being walked by my group (-1: none); planned: 0 while a virtual row is walked
+        unsigned out_word = 0u;   // planned: destination of the virtual row (a row of y, or a partial-sum slot)
+        // Element positions are unsigned: an iteration runs up to 1536 elements ahead of a count that may come close to 2^31.
+        unsigned begin = 0u;   // first stored element of the row
+        unsigned end = 0u;     // one past the last stored element
+        unsigned pos = 0u;     // first element of the group's next iteration (multiple of 8)
+        // Byte address (shared window, or byte offset from x - kXPadFront when x stays in global memory) of
+        // "column -1 + index in row" in front of the lane's unit of the next sub-step, less 14 per lane below
+        // it in the group: the lane totals that go through the scan carry +14 each (see the decode below).
+        const unsigned lane_const = (unsigned)(x_fold + 2 * kXPadFront + 2 * lig);
+        unsigned run = 0u;
+        float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
+        float accb[BV][2];   // batched: per vector, even and odd elements
 #pragma unroll
-                for (int b = 0; b < BV; ++b) {
-                    float total = accb[b][0] + accb[b][1];
+        for (int b = 0; b < BV; ++b) accb[b][0] = accb[b][1] = 0.f;
+
+        if constexpr (FIRST && !EARLY) stage_x();
+        bool first_pass = EARLY && FIRST;
+        for (;;) {
+            bool done = false;
+            // ---- groups that ran out of work finish their row and take the next one ---------------------
+            const bool need = pos >= end;
+            const unsigned needmask = __ballot_sync(0xffffffffu, need);
+            if (needmask) {
+                if constexpr (BV == 1) {
+                    float total = (acc0 + acc1) + (acc2 + acc3);
 #pragma unroll
-                    for (int o = L / 2; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+                    for (int o = LN / 2; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
                     if (need) {
-                        if (my_row >= 0 && lig == 0 && b < batch) {
-                            __half *yb = y + (size_t)b * rows;
-                            float r = alpha * total;
-                            if (beta != 0.f) r += beta * __half2float(yb[my_row]);
-                            yb[my_row] = __float2half_rn(r);
+                        if (my_row >= 0 && lig == 0) {
+                            if constexpr (PLAN) {
+                                plan_row_done(plan, out_word, total, alpha, beta, y16, rows);
+                            } else if constexpr (PEER) {
+                                ystage[my_row - cta_row_lo] = __float2half_rn(alpha * total);   // delivered in bulk at the end
+                            } else {
+                                float r = alpha * total;
+                                if (beta != 0.f) r += beta * from_bits16<VT>(y16[my_row]);
+                                y16[my_row] = to_bits16<VT>(r);
+                            }
                         }
-                        accb[b][0] = accb[b][1] = 0.f;
+                        acc0 = acc1 = acc2 = acc3 = 0.f;
+                    }
+                } else {
+#pragma unroll
+                    for (int b = 0; b < BV; ++b) {
+                        float total = accb[b][0] + accb[b][1];
+#pragma unroll
+                        for (int o = LN / 2; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+                        if (need) {
+                            if (my_row >= 0 && lig == 0 && b < batch) {
+                                __half *yb = y + (size_t)b * rows;
+                                float r = alpha * total;
+                                if (beta != 0.f) r += beta * __half2float(yb[my_row]);
+                                yb[my_row] = __float2half_rn(r);
+                            }
+                            accb[b][0] = accb[b][1] = 0.f;
+                        }
                     }
                 }
-            }
-            const int avail = row_hi - row_next;
-            if (avail <= 0) {
-                if (needmask == 0xffffffffu) done = true;
-                if (need) { my_row = -1; pos = 0u; end = 0u; begin = 0u; }
-            } else {
-                const unsigned leaders = needmask & kLeaders;
-                const int want = __popc(leaders);
-                const int take = min(want, avail);
-                if (row_next + take > win_base + (PLAN ? 32 : 31)) {  // warp-uniform
-                    win_base = row_next;
-                    load_window();
-                }
-                const int rank = __popc(leaders & ((1u << group_lane0) - 1u));
-                const int nr = row_next + rank;
-                // offsets are clamped into [0, stored] so that corrupt row_indices (or a corrupt plan) cannot send
-                // loads outside values/deltas
-                unsigned b, e;
-                unsigned colbase2 = 0u;   // planned: twice the column sum in front of the segment (a byte offset into x)
-                if constexpr (PLAN) {
-                    b = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
-                    const unsigned pk = __shfl_sync(0xffffffffu, pk_reg, (nr - win_base) & 31);
-                    e = min(b + (pk & ((1u << kPlanLenBits) - 1u)), (unsigned)stored);
-                    colbase2 = (pk >> kPlanLenBits) << 1;
+                const int avail = row_hi - row_next;
+                if (avail <= 0) {
+                    if (needmask == 0xffffffffu) done = true;
+                    if (need) { my_row = -1; pos = 0u; end = 0u; begin = 0u; }
                 } else {
-                    b = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
-                    e = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr + 1 - win_base) & 31), (int)b), stored);
-                }
-                if (need) {
-                    if (rank < take) {
-                        if constexpr (PLAN) {
-                            my_row = 0;
-                            out_word = __ldg(plan.out + sorted_index(nr));   // needed only when the virtual row ends
+                    const unsigned leaders = needmask & leader_lanes;
+                    const int want = __popc(leaders);
+                    const int take = min(want, avail);
+                    if (row_next + take > win_base + (PLAN ? 32 : 31)) {  // warp-uniform
+                        win_base = row_next;
+                        load_window();
+                    }
+                    const int rank = __popc(leaders & ((1u << group_lane0) - 1u));
+                    const int nr = row_next + rank;
+                    // offsets are clamped into [0, stored] so that corrupt row_indices (or a corrupt plan) cannot send
+                    // loads outside values/deltas
+                    unsigned b, e;
+                    unsigned colbase2 = 0u;   // planned: twice the column sum in front of the segment (a byte offset into x)
+                    if constexpr (PLAN) {
+                        b = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
+                        const unsigned pk = __shfl_sync(0xffffffffu, pk_reg, (nr - win_base) & 31);
+                        e = min(b + (pk & ((1u << kPlanLenBits) - 1u)), (unsigned)stored);
+                        colbase2 = (pk >> kPlanLenBits) << 1;
+                    } else {
+                        b = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr - win_base) & 31), 0), stored);
+                        e = (unsigned)min(max(__shfl_sync(0xffffffffu, ri_reg, (nr + 1 - win_base) & 31), (int)b), stored);
+                    }
+                    if (need) {
+                        if (rank < take) {
+                            if constexpr (PLAN) {
+                                my_row = 0;
+                                out_word = __ldg(plan.out + sorted_index(nr));   // needed only when the virtual row ends
+                            } else {
+                                my_row = nr;
+                            }
+                            begin = b; end = e; pos = b & ~(unsigned)(kGroup - 1);
+                            run = lane_const + colbase2 - 2u * (b & (unsigned)(kGroup - 1));   // the unit that holds `begin` starts before the row
                         } else {
-                            my_row = nr;
+                            my_row = -1; pos = 0u; end = 0u; begin = 0u;
                         }
-                        begin = b; end = e; pos = b & ~(unsigned)(kGroup - 1);
-                        run = lane_const + colbase2 - 2u * (b & (unsigned)(kGroup - 1));   // the unit that holds `begin` starts before the row
-                    } else {
-                        my_row = -1; pos = 0u; end = 0u; begin = 0u;
+                    }
+                    row_next += take;
+                }
+            }
+
+            if constexpr (!(EARLY && FIRST)) {
+                if (done) break;
+            }
+
+            // ---- issue the loads of the whole iteration ------------------------------------------------------
+            uint4 v[D];
+            unsigned w[D];
+            const int ord0 = (int)(pos + (unsigned)(lig * kGroup));   // not negative where it is used as an index
+            const int rem0 = (int)(end - (unsigned)ord0);    // elements of the row from the lane's first unit on
+            const int lo0 = (int)(begin - (unsigned)ord0);   // > 0: leading elements of sub-step 0 belong to the previous row
+            {
+                const uint4 *vp = values + (ord0 >> 3);
+                const unsigned *dp = deltas + (ord0 >> 3);
+#pragma unroll
+                for (int s = 0; s < D; ++s) {
+                    v[s] = make_uint4(0u, 0u, 0u, 0u);
+                    w[s] = 0u;
+                    if (s * STEP < rem0) {
+                        if constexpr (VT == kI8) {
+                            const uint2 t = ldg_stream_v2(reinterpret_cast<const uint2 *>(values) + (ord0 >> 3) + s * LN);
+                            v[s].x = t.x;
+                            v[s].y = t.y;
+                        } else {
+                            v[s] = ldg_stream_v4(vp + s * LN);
+                        }
+                        w[s] = ldg_stream_u32(dp + s * LN);
                     }
                 }
-                row_next += take;
             }
-        }
 
-        if constexpr (!EARLY) {
+            // ---- first pass only: with the first matrix loads in flight, wait for the previous kernel of the
+            //      stream (if that has not happened yet) and stage x into shared memory, framed by zeros. Every
+            //      warp comes through here, also one without rows. ---------------------------------------------
+            if constexpr (EARLY && FIRST) {
+                if (first_pass) {
+                    first_pass = false;
+                    asm volatile("griddepcontrol.wait;" ::: "memory");
+                    stage_x();
+                }
+            }
             if (done) break;
-        }
 
-        // ---- issue the loads of the whole iteration ------------------------------------------------------
-        uint4 v[D];
-        unsigned w[D];
-        const int ord0 = (int)(pos + (unsigned)(lig * kGroup));   // not negative where it is used as an index
-        const int rem0 = (int)(end - (unsigned)ord0);    // elements of the row from the lane's first unit on
-        const int lo0 = (int)(begin - (unsigned)ord0);   // > 0: leading elements of sub-step 0 belong to the previous row
-        {
-            const uint4 *vp = values + (ord0 >> 3);
-            const unsigned *dp = deltas + (ord0 >> 3);
+            // Which sub-steps hold a unit that straddles the first or the last element of a row, and how far the
+            // longest row of the warp still reaches: two warp-wide reductions per iteration replace a vote per unit.
+            unsigned mybits = 0u;
+            if (rem0 > 0) {
+                if (lo0 > 0) mybits = 1u;
+                const int tail = rem0 & (STEP - 1);
+                const unsigned s_end = (unsigned)rem0 >> LOG_STEP;
+                if (tail > 0 && tail < kGroup && s_end < (unsigned)D) mybits |= 1u << s_end;
+            }
+            const unsigned straddle = __reduce_or_sync(0xffffffffu, mybits);
+            const int max_rem = __reduce_max_sync(0xffffffffu, rem0);
+
 #pragma unroll
-            for (int s = 0; s < D; ++s) {
-                v[s] = make_uint4(0u, 0u, 0u, 0u);
-                w[s] = 0u;
-                if (s * STEP < rem0) {
+            for (int p = 0; p < NPAIR; ++p) {
+                // a pair in which no lane of the warp has an element left ends the iteration
+                if (p > 0 && max_rem <= 2 * p * STEP) break;
+                // Byte-SIMD prefix sums of the 8 deltas of a unit, scaled by 2 (byte offsets into fp16 x):
+                //   ce byte j = 2*(inclusive prefix of element 2j)   + 2*(2j)
+                //   co byte j = 2*(inclusive prefix of element 2j+1) + 2*(2j+1)
+                // so the top byte of co is 2*(sum of the 8 deltas) + 14.
+                unsigned ce[2], co[2];
+#pragma unroll
+                for (int hs = 0; hs < 2; ++hs) {
+                    const int s = 2 * p + hs;
+                    if (straddle & (1u << s)) {
+                        if constexpr (VT == kI8) mask_unit_bytes(v[s], w[s], (s == 0) ? lo0 : 0, rem0 - s * STEP);
+                        else mask_unit(v[s], w[s], (s == 0) ? lo0 : 0, rem0 - s * STEP);
+                    }
+                    const unsigned ev = w[s] & 0x0f0f0f0fu;
+                    const unsigned od = (w[s] >> 4) & 0x0f0f0f0fu;
+                    const unsigned pe = ev * 0x02020202u + 0x0c080400u;
+                    const unsigned po = od * 0x02020202u;
+                    ce[hs] = po * 256u + pe;
+                    co[hs] = pe + po + 0x02020202u;
+                }
+                // one scan for both sub-steps: lane totals packed as two 16-bit fields (each < 2^13)
+                const unsigned t = (co[0] >> 24) | ((co[1] >> 8) & 0x00ff0000u);
+                unsigned inc = t;
+#pragma unroll
+                for (int o = 1; o < LN; o <<= 1) {
+                    const unsigned u = __shfl_up_sync(0xffffffffu, inc, o, LN);
+                    if (lig >= o) inc += u;
+                }
+                const unsigned g = __shfl_sync(0xffffffffu, inc, LN - 1, LN);
+                const unsigned ex = inc - t;
+#pragma unroll
+                for (int hs = 0; hs < 2; ++hs) {
+                    const int s = 2 * p + hs;
+                    // lane base = run + (low or high field of ex); the group advances by its field of g, which
+                    // holds 14 per lane where 16 (2 bytes x 8 elements) are due: 2*LN more per sub-step
+                    const unsigned sel = hs ? 0x0100u : 0x0001u;
+                    const unsigned a0 = min(__dp2a_lo(ex, sel, run) + (unsigned)(2 * LN * s), a_max);   // keeps malformed input inside the padded x
+                    run = __dp2a_lo(g, sel, run);
+                    unsigned vconv[4];   // int8: the unit's 8 values as four f16x2 words
                     if constexpr (VT == kI8) {
-                        const uint2 t = ldg_stream_v2(reinterpret_cast<const uint2 *>(values) + (ord0 >> 3) + s * L);
-                        v[s].x = t.x;
-                        v[s].y = t.y;
-                    } else {
-                        v[s] = ldg_stream_v4(vp + s * L);
+                        bytes_to_f16x2(v[s].x, vconv[0], vconv[1]);
+                        bytes_to_f16x2(v[s].y, vconv[2], vconv[3]);
                     }
-                    w[s] = ldg_stream_u32(dp + s * L);
-                }
-            }
-        }
-
-        // ---- first pass only: with the first matrix loads in flight, wait for the previous kernel of the
-        //      stream (if that has not happened yet) and stage x into shared memory, framed by zeros. Every
-        //      warp comes through here, also one without rows. ---------------------------------------------
-        if constexpr (EARLY) {
-            if (first_pass) {
-                first_pass = false;
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                stage_x();
-            }
-        }
-        if (done) break;
-
-        // Which sub-steps hold a unit that straddles the first or the last element of a row, and how far the
-        // longest row of the warp still reaches: two warp-wide reductions per iteration replace a vote per unit.
-        unsigned mybits = 0u;
-        if (rem0 > 0) {
-            if (lo0 > 0) mybits = 1u;
-            const int tail = rem0 & (STEP - 1);
-            const unsigned s_end = (unsigned)rem0 >> LOG_STEP;
-            if (tail > 0 && tail < kGroup && s_end < (unsigned)D) mybits |= 1u << s_end;
-        }
-        const unsigned straddle = __reduce_or_sync(0xffffffffu, mybits);
-        const int max_rem = __reduce_max_sync(0xffffffffu, rem0);
-
+                    const unsigned *vw = (VT == kI8) ? vconv : reinterpret_cast<const unsigned *>(&v[s]);
+                    if constexpr (BV > 1) {
+                        const int ab = x_base + (int)a0 * BV;
+                        auto element_pair = [&](auto jt) {
+                            constexpr int J = decltype(jt)::value;
+                            unsigned xe[BV / 2], xo[BV / 2];
+                            lds_vec<BV>((unsigned)add_byte<J, BV>(ce[hs], ab), xe);
+                            lds_vec<BV>((unsigned)add_byte<J, BV>(co[hs], ab), xo);
 #pragma unroll
-        for (int p = 0; p < NPAIR; ++p) {
-            // a pair in which no lane of the warp has an element left ends the iteration
-            if (p > 0 && max_rem <= 2 * p * STEP) break;
-            // Byte-SIMD prefix sums of the 8 deltas of a unit, scaled by 2 (byte offsets into fp16 x):
-            //   ce byte j = 2*(inclusive prefix of element 2j)   + 2*(2j)
-            //   co byte j = 2*(inclusive prefix of element 2j+1) + 2*(2j+1)
-            // so the top byte of co is 2*(sum of the 8 deltas) + 14.
-            unsigned ce[2], co[2];
-#pragma unroll
-            for (int hs = 0; hs < 2; ++hs) {
-                const int s = 2 * p + hs;
-                if (straddle & (1u << s)) {
-                    if constexpr (VT == kI8) mask_unit_bytes(v[s], w[s], (s == 0) ? lo0 : 0, rem0 - s * STEP);
-                    else mask_unit(v[s], w[s], (s == 0) ? lo0 : 0, rem0 - s * STEP);
-                }
-                const unsigned ev = w[s] & 0x0f0f0f0fu;
-                const unsigned od = (w[s] >> 4) & 0x0f0f0f0fu;
-                const unsigned pe = ev * 0x02020202u + 0x0c080400u;
-                const unsigned po = od * 0x02020202u;
-                ce[hs] = po * 256u + pe;
-                co[hs] = pe + po + 0x02020202u;
-            }
-            // one scan for both sub-steps: lane totals packed as two 16-bit fields (each < 2^13)
-            const unsigned t = (co[0] >> 24) | ((co[1] >> 8) & 0x00ff0000u);
-            unsigned inc = t;
-#pragma unroll
-            for (int o = 1; o < L; o <<= 1) {
-                const unsigned u = __shfl_up_sync(0xffffffffu, inc, o, L);
-                if (lig >= o) inc += u;
-            }
-            const unsigned g = __shfl_sync(0xffffffffu, inc, L - 1, L);
-            const unsigned ex = inc - t;
-#pragma unroll
-            for (int hs = 0; hs < 2; ++hs) {
-                const int s = 2 * p + hs;
-                // lane base = run + (low or high field of ex); the group advances by its field of g, which
-                // holds 14 per lane where 16 (2 bytes x 8 elements) are due: 2*L more per sub-step
-                const unsigned sel = hs ? 0x0100u : 0x0001u;
-                const unsigned a0 = min(__dp2a_lo(ex, sel, run) + (unsigned)(2 * L * s), a_max);   // keeps malformed input inside the padded x
-                run = __dp2a_lo(g, sel, run);
-                unsigned vconv[4];   // int8: the unit's 8 values as four f16x2 words
-                if constexpr (VT == kI8) {
-                    bytes_to_f16x2(v[s].x, vconv[0], vconv[1]);
-                    bytes_to_f16x2(v[s].y, vconv[2], vconv[3]);
-                }
-                const unsigned *vw = (VT == kI8) ? vconv : reinterpret_cast<const unsigned *>(&v[s]);
-                if constexpr (BV > 1) {
-                    const int ab = x_base + (int)a0 * BV;
-                    auto element_pair = [&](auto jt) {
-                        constexpr int J = decltype(jt)::value;
-                        unsigned xe[BV / 2], xo[BV / 2];
-                        lds_vec<BV>((unsigned)add_byte<J, BV>(ce[hs], ab), xe);
-                        lds_vec<BV>((unsigned)add_byte<J, BV>(co[hs], ab), xo);
-#pragma unroll
-                        for (int b = 0; b < BV; b += 2) {
-                            accb[b][0] = fma_hh<0, 0>(accb[b][0], vw[J], xe[b / 2]);
-                            accb[b + 1][0] = fma_hh<0, 1>(accb[b + 1][0], vw[J], xe[b / 2]);
-                            accb[b][1] = fma_hh<1, 0>(accb[b][1], vw[J], xo[b / 2]);
-                            accb[b + 1][1] = fma_hh<1, 1>(accb[b + 1][1], vw[J], xo[b / 2]);
-                        }
-                    };
-                    element_pair(Int<0>{});
-                    element_pair(Int<1>{});
-                    element_pair(Int<2>{});
-                    element_pair(Int<3>{});
-                } else {
-                    unsigned xe[4], xo[4];
-                    if (XS) {
-                        xe[0] = lds_u16((unsigned)add_byte<0>(ce[hs], (int)a0));
-                        xo[0] = lds_u16((unsigned)add_byte<0>(co[hs], (int)a0));
-                        xe[1] = lds_u16((unsigned)add_byte<1>(ce[hs], (int)a0));
-                        xo[1] = lds_u16((unsigned)add_byte<1>(co[hs], (int)a0));
-                        xe[2] = lds_u16((unsigned)add_byte<2>(ce[hs], (int)a0));
-                        xo[2] = lds_u16((unsigned)add_byte<2>(co[hs], (int)a0));
-                        xe[3] = lds_u16((unsigned)add_byte<3>(ce[hs], (int)a0));
-                        xo[3] = lds_u16((unsigned)add_byte<3>(co[hs], (int)a0));
-                    } else {
-                        const unsigned short *xg = reinterpret_cast<const unsigned short *>(x);
-                        const int cmax = cols - 1;
-                        auto gather = [&](int off2) -> unsigned {
-                            return (unsigned)__ldg(xg + min(max((off2 >> 1) - kXPadFront, 0), cmax));
+                            for (int b = 0; b < BV; b += 2) {
+                                accb[b][0] = fma_hh<0, 0>(accb[b][0], vw[J], xe[b / 2]);
+                                accb[b + 1][0] = fma_hh<0, 1>(accb[b + 1][0], vw[J], xe[b / 2]);
+                                accb[b][1] = fma_hh<1, 0>(accb[b][1], vw[J], xo[b / 2]);
+                                accb[b + 1][1] = fma_hh<1, 1>(accb[b + 1][1], vw[J], xo[b / 2]);
+                            }
                         };
-                        xe[0] = gather(add_byte<0>(ce[hs], (int)a0));
-                        xo[0] = gather(add_byte<0>(co[hs], (int)a0));
-                        xe[1] = gather(add_byte<1>(ce[hs], (int)a0));
-                        xo[1] = gather(add_byte<1>(co[hs], (int)a0));
-                        xe[2] = gather(add_byte<2>(ce[hs], (int)a0));
-                        xo[2] = gather(add_byte<2>(co[hs], (int)a0));
-                        xe[3] = gather(add_byte<3>(ce[hs], (int)a0));
-                        xo[3] = gather(add_byte<3>(co[hs], (int)a0));
+                        element_pair(Int<0>{});
+                        element_pair(Int<1>{});
+                        element_pair(Int<2>{});
+                        element_pair(Int<3>{});
+                    } else {
+                        unsigned xe[4], xo[4];
+                        if (XS) {
+                            xe[0] = lds_u16((unsigned)add_byte<0>(ce[hs], (int)a0));
+                            xo[0] = lds_u16((unsigned)add_byte<0>(co[hs], (int)a0));
+                            xe[1] = lds_u16((unsigned)add_byte<1>(ce[hs], (int)a0));
+                            xo[1] = lds_u16((unsigned)add_byte<1>(co[hs], (int)a0));
+                            xe[2] = lds_u16((unsigned)add_byte<2>(ce[hs], (int)a0));
+                            xo[2] = lds_u16((unsigned)add_byte<2>(co[hs], (int)a0));
+                            xe[3] = lds_u16((unsigned)add_byte<3>(ce[hs], (int)a0));
+                            xo[3] = lds_u16((unsigned)add_byte<3>(co[hs], (int)a0));
+                        } else {
+                            const unsigned short *xg = reinterpret_cast<const unsigned short *>(x);
+                            const int cmax = cols - 1;
+                            auto gather = [&](int off2) -> unsigned {
+                                return (unsigned)__ldg(xg + min(max((off2 >> 1) - kXPadFront, 0), cmax));
+                            };
+                            xe[0] = gather(add_byte<0>(ce[hs], (int)a0));
+                            xo[0] = gather(add_byte<0>(co[hs], (int)a0));
+                            xe[1] = gather(add_byte<1>(ce[hs], (int)a0));
+                            xo[1] = gather(add_byte<1>(co[hs], (int)a0));
+                            xe[2] = gather(add_byte<2>(ce[hs], (int)a0));
+                            xo[2] = gather(add_byte<2>(co[hs], (int)a0));
+                            xe[3] = gather(add_byte<3>(ce[hs], (int)a0));
+                            xo[3] = gather(add_byte<3>(co[hs], (int)a0));
+                        }
+                        acc0 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc0, vw[0], xe[0]);
+                        acc1 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc1, vw[0], xo[0]);
+                        acc2 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc2, vw[1], xe[1]);
+                        acc3 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc3, vw[1], xo[1]);
+                        acc0 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc0, vw[2], xe[2]);
+                        acc1 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc1, vw[2], xo[2]);
+                        acc2 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc2, vw[3], xe[3]);
+                        acc3 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc3, vw[3], xo[3]);
                     }
-                    acc0 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc0, vw[0], xe[0]);
-                    acc1 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc1, vw[0], xo[0]);
-                    acc2 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc2, vw[1], xe[1]);
-                    acc3 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc3, vw[1], xo[1]);
-                    acc0 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc0, vw[2], xe[2]);
-                    acc1 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc1, vw[2], xo[2]);
-                    acc2 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc2, vw[3], xe[3]);
-                    acc3 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc3, vw[3], xo[3]);
                 }
             }
+            // every sub-step that was skipped lies behind the end of all rows of the warp: `run` is not used again before the next row resets it
+            run += (unsigned)(2 * LN * D);
+            pos += (unsigned)(D * STEP);
         }
-        // every sub-step that was skipped lies behind the end of all rows of the warp: `run` is not used again before the next row resets it
-        run += (unsigned)(2 * L * D);
-        pos += (unsigned)(D * STEP);
+    };
+    walk(Int<L>{}, Int<1>{}, row_next, row_hi);
+    if constexpr (TAIL) {
+        if (tail_rows > 0) {   // the rows beyond the last full round, a warp each (see choose_tail)
+            const int first = rows - tail_rows;
+            walk(Int<32>{}, Int<0>{}, first + block_boundary<1>(tail_rows, (unsigned)warp_id, (unsigned)n_warps),
+                 first + block_boundary<1>(tail_rows, (unsigned)warp_id + 1u, (unsigned)n_warps));
+        }
     }
 
     if constexpr (PEER) {
@@ -757,27 +774,27 @@ __global__ void peer_wait_kernel(unsigned *flags, int world, unsigned spin_limit
     flags[world + 2] = 1u + (unsigned)p;   // gave up: the host can read which rank never arrived
 }
 
-template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T>
+template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T, bool TAIL>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra);
 
 // The instantiation with or without early matrix loads, by the immutable-matrix flag of the call.
-template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads>
+template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads, bool TAIL = false>
 int launch(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
            const void *x, void *y, float alpha, float beta, cudaStream_t stream,
            const DeviceInfo &dev, int ctas_per_sm, const Peers &peers = Peers{}, int batch = 1, const Extra &extra = Extra{})
 {
     if constexpr (BV == 1) {
         if (extra.flags & MACKO_SPMV_MATRIX_IMMUTABLE)
-            return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, true, T>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
+            return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, true, T, TAIL>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
                                                                          stream, dev, ctas_per_sm, peers, batch, extra);
     }
-    return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, false, T>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
+    return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, false, T, TAIL>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
                                                                   stream, dev, ctas_per_sm, peers, batch, extra);
 }
 
-template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T>
+template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T, bool TAIL>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra)
@@ -788,7 +805,7 @@ int launch_variant(const void *values, const void *deltas, const int32_t *ri, in
     if (smem > (size_t)dev.max_smem_optin)
         return fail(MACKO_ERR_INVALID_ARGUMENT, "the launch needs %lld bytes of shared memory, the device offers %d (cols=%d)",
                     (long long)smem, dev.max_smem_optin, cols);
-    auto kernel = spmv_kernel<L, NPAIR, XS, PEER, BV, PLAN, VT, EARLY, T>;
+    auto kernel = spmv_kernel<L, NPAIR, XS, PEER, BV, PLAN, VT, EARLY, T, TAIL>;
     if (smem > 48 * 1024) {
         // Idempotent and cheap; set on every call so that every device is covered.
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -815,13 +832,14 @@ int launch_variant(const void *values, const void *deltas, const int32_t *ri, in
     // next kernel move in early only takes SM slots away from it (measured: slower). With a deferred wait the
     // kernel publishes and returns, and overlaps like any other.
     cfg.numAttrs = (use_pdl() && (!PEER || peers.deferred)) ? 1 : 0;
+    const int tail_rows = TAIL ? extra.tail_rows : 0;
     PeersArg<PEER> peers_arg{};
     PlanArg<PLAN> plan_arg{};
     if constexpr (PEER) peers_arg = peers;
     if constexpr (PLAN) plan_arg = extra.plan;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel,
         static_cast<const uint4 *>(values), static_cast<const unsigned *>(deltas), ri,
-        static_cast<const __half *>(x), static_cast<__half *>(y), rows, cols, (int)padded, alpha, beta, batch, extra.flags,
+        static_cast<const __half *>(x), static_cast<__half *>(y), rows, cols, (int)padded, alpha, beta, batch, extra.flags, tail_rows,
         peers_arg, plan_arg);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "spmv launch: %s", cudaGetErrorString(e));
@@ -894,6 +912,21 @@ Shape choose_shape(long long rows, long long cols, long long padded, int residen
     return {L, D};
 }
 
+// Rows at the end of a matrix that are walked with a warp per row. With 8 or 16 lanes per row the blocks of four or two rows fill the
+// warps in rounds, and where the last round has a block for less than half of them, the others idle while those few walk theirs
+// (32 to 64 sub-steps); a warp per row, over all warps, takes a quarter (half) as long. Above half, the last round loads the
+// pipe of the SM well enough that nothing is gained (28000x3000 d = 0.5, 1.48 rounds: 24.2 / 24.0), and a matrix of less than one round
+// would only lose the compact groups' fewer bank conflicts. With / without (B200, graph of products, immutable, us):
+// 22016x4096 (1.16 rounds) d = 0.5 26.3 / 29.3, d = 0.9 38.6 / 44.4, d = 0.1 11.5 / 11.5, 21000x9000 d = 0.4 (1.11) 44.1 / 50.0, 42000x4096
+// d = 0.3 (2.22) 31.6 / 33.2; 16 lanes: 10000x8192 d = 0.5 (1.06) 28.2 / 30.6, 12288x11008 (1.30) 38.0 / 40.6. A kernel of its own: with the
+// second walk in the code, launches that do not need it took up to 3 % longer.
+int choose_tail(int64_t rows, int block, int64_t warps)
+{
+    const int64_t blocks = (rows + block - 1) / block, rounds = blocks / warps, left = blocks - rounds * warps;
+    if (rounds == 0 || left == 0 || 2 * left > warps) return 0;
+    return (int)(rows - rounds * warps * block);
+}
+
 // One launch for up to BV vectors. Lanes per row as in the single-vector product; fewer units in flight with
 // more vectors, whose accumulators and gathered values take the registers.
 template <int BV>
@@ -944,6 +977,14 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Extra extra = {};
     extra.flags = flags;
+    if (xs && (L == 8 || L == 16) && D == 6) {
+        extra.tail_rows = choose_tail(rows, 32 / L, (int64_t)dev->sm_count * ctas * kWarpsPerCta);
+        if (extra.tail_rows > 0) {
+            const int r = (int)rows, c = (int)cols;
+            return L == 8 ? launch<8, 3, true, false, 1, false, VT, kThreads, true>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, ctas, Peers{}, 1, extra)
+                          : launch<16, 3, true, false, 1, false, VT, kThreads, true>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, ctas, Peers{}, 1, extra);
+        }
+    }
     if (xs && L == 32 && D == 6 && smem > kWideSmem)
         return launch<32, 3, true, false, 1, false, VT, 2 * kThreads>(values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y,
                                                                       alpha, beta, s, *dev, 0, Peers{}, 1, extra);
