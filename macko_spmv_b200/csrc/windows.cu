@@ -29,6 +29,7 @@ constexpr int D = 2;                 // sub-steps in flight: more cost registers
 // ---- windows of a matrix -----------------------------------------------------------------------------------------------
 // One warp per row walks its deltas once, 256 elements per step; the lane whose unit is the first of a window writes the
 // section. Corrupt input is clamped: every section is written, none reaches beyond the row.
+constexpr int kSteps = 4;
 __global__ void __launch_bounds__(256)
 window_sections_kernel(const unsigned *__restrict__ deltas32, const int *__restrict__ ri, int rows, int stored, int windows, int width,
                        uint2 *__restrict__ sections)
@@ -42,30 +43,39 @@ window_sections_kernel(const unsigned *__restrict__ deltas32, const int *__restr
     if (lane == 0) mine[0] = make_uint2(begin, (unsigned)kWindowFront);
     int col = 0;        // columns used up by the row's elements in front of the step
     int last = 0;       // window of the last unit in front of it
-    for (unsigned base = begin & ~7u; base < end; base += 256u) {
-        const unsigned k0 = base + 8u * (unsigned)lane;
-        const bool live = k0 < end;
-        const unsigned w = live ? __ldg(deltas32 + (k0 >> 3)) : 0u;
-        int sum = 0;
+    for (unsigned group = begin & ~7u; group < end; group += 256u * kSteps) {
+        unsigned w[kSteps];   // the loads of several steps are in flight together
 #pragma unroll
-        for (unsigned i = 0; i < 8u; ++i)
-            if (k0 + i >= begin && k0 + i < end) sum += (int)((w >> (4 * i)) & 15u) + 1;
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
+        for (int u = 0; u < kSteps; ++u) {
+            const unsigned k0 = group + 256u * (unsigned)u + 8u * (unsigned)lane;
+            w[u] = k0 < end ? __ldg(deltas32 + (k0 >> 3)) : 0u;
         }
-        const int front = col + incl - sum;   // columns used up in front of the unit
-        // window of the unit; the row's first unit is in the first one whatever its elements say
-        const int win = k0 <= begin ? 0 : min((front + (int)(w & 15u)) / width, windows - 1);
-        int before = __shfl_up_sync(0xffffffffu, win, 1);
-        if (lane == 0) before = last;
-        if (live)
-            for (int q = before + 1; q <= win; ++q)
-                mine[(size_t)q * rows] = make_uint2(k0, (unsigned)min(max(front - q * width + kWindowFront, 0), (1 << kWindowColBits) - 1));
-        last = __shfl_sync(0xffffffffu, win, 31 - __clz(__ballot_sync(0xffffffffu, live)));
-        col += __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+        for (int u = 0; u < kSteps; ++u) {
+            const unsigned base = group + 256u * (unsigned)u, k0 = base + 8u * (unsigned)lane;
+            if (base >= end) break;   // warp-uniform
+            const bool live = k0 < end;
+            // columns of the unit: its deltas and one per element, without those of the neighbouring rows
+            const unsigned lo = k0 < begin ? min(begin - k0, 8u) : 0u, hi = live ? min(end - k0, 8u) : 0u;
+            const unsigned mine_w = lo < hi ? w[u] & (0xffffffffu << (4u * lo)) & (0xffffffffu >> (4u * (8u - hi))) : 0u;
+            const int sum = (int)__dp4a((mine_w & 0x0f0f0f0fu) + ((mine_w >> 4) & 0x0f0f0f0fu), 0x01010101u, lo < hi ? hi - lo : 0u);
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const int front = col + incl - sum;   // columns used up in front of the unit
+            // window of the unit; the row's first unit is in the first one whatever its elements say
+            const int win = k0 <= begin ? 0 : min((front + (int)(w[u] & 15u)) / width, windows - 1);
+            int before = __shfl_up_sync(0xffffffffu, win, 1);
+            if (lane == 0) before = last;
+            if (live)
+                for (int q = before + 1; q <= win; ++q)
+                    mine[(size_t)q * rows] = make_uint2(k0, (unsigned)min(max(front - q * width + kWindowFront, 0), (1 << kWindowColBits) - 1));
+            last = __shfl_sync(0xffffffffu, win, 31 - __clz(__ballot_sync(0xffffffffu, live)));
+            col += __shfl_sync(0xffffffffu, incl, 31);
+        }
     }
     for (int q = last + 1 + lane; q < windows; q += 32) mine[(size_t)q * rows] = make_uint2(end, (unsigned)kWindowFront);
     __threadfence_block();
