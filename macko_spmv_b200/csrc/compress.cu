@@ -129,71 +129,73 @@ __device__ __forceinline__ int prev_nonzero_before_lane(unsigned any, int lane, 
 constexpr int kCarryInLast = -0x7fffffff;
 template <bool I8>
 __global__ void __launch_bounds__(kThreads)
-count_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, int cols, bool vec_ok, int *__restrict__ counts)
+count_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, int cols, bool vec_ok, int rows_per_warp, int *__restrict__ counts)
 {
     asm volatile("griddepcontrol.launch_dependents;");
     const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    // element indices fit 32 bits: the entry points refuse matrices of 2^31 elements or more, and a walk ends
-    // less than 2048 elements behind its row
-    const unsigned total = (unsigned)rows * (unsigned)cols;
-    const unsigned row_lo = (unsigned)row * (unsigned)cols;
-    const unsigned row_hi = row_lo + (unsigned)cols;
-    // The first step starts at the 8-element boundary at or below the row start.
-    const unsigned first = vec_ok ? (row_lo & ~7u) : row_lo;
-    int count = 0;          // stored elements seen by this lane
-    int carry = -1;         // column of the last non-zero seen so far in this row, unless the last step was a short one:
-    unsigned last = 0u;     // then it is the last of lane 31's `last` fields, whose first column is `last_c0`
-    int last_c0 = 0;
-    bool ends_dense = true; // at most 7 zeros lie between the last non-zero (the row's start) and the next step
-    for (unsigned group0 = first; group0 < row_hi; group0 += (unsigned)(kUnroll * kColsPerStep)) {
-        // all loads of kUnroll steps are issued before the first one is consumed
-        typename Raw<I8>::Vec v[kUnroll];
-        const bool inner = vec_ok && group0 >= row_lo && group0 + (unsigned)(kUnroll * kColsPerStep) <= row_hi;   // warp-uniform
-        if (inner) {
+    const unsigned first_row = (blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5)) * (unsigned)rows_per_warp;
+#pragma unroll 1
+    for (unsigned row = first_row; row < min(first_row + (unsigned)rows_per_warp, (unsigned)rows); ++row) {
+        // element indices fit 32 bits: the entry points refuse matrices of 2^31 elements or more, and a walk ends
+        // less than 2048 elements behind its row
+        const unsigned total = (unsigned)rows * (unsigned)cols;
+        const unsigned row_lo = row * (unsigned)cols;
+        const unsigned row_hi = row_lo + (unsigned)cols;
+        // The first step starts at the 8-element boundary at or below the row start.
+        const unsigned first = vec_ok ? (row_lo & ~7u) : row_lo;
+        int count = 0;          // stored elements seen by this lane
+        int carry = -1;         // column of the last non-zero seen so far in this row, unless the last step was a short one:
+        unsigned last = 0u;     // then it is the last of lane 31's `last` fields, whose first column is `last_c0`
+        int last_c0 = 0;
+        bool ends_dense = true; // at most 7 zeros lie between the last non-zero (the row's start) and the next step
+        for (unsigned group0 = first; group0 < row_hi; group0 += (unsigned)(kUnroll * kColsPerStep)) {
+            // all loads of kUnroll steps are issued before the first one is consumed
+            typename Raw<I8>::Vec v[kUnroll];
+            const bool inner = vec_ok && group0 >= row_lo && group0 + (unsigned)(kUnroll * kColsPerStep) <= row_hi;   // warp-uniform
+            if (inner) {
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) v[u] = load8_inside<I8>(dense, group0 + (unsigned)(u * kColsPerStep + lane * kColsPerLane));
-        } else {
+                for (int u = 0; u < kUnroll; ++u) v[u] = load8_inside<I8>(dense, group0 + (unsigned)(u * kColsPerStep + lane * kColsPerLane));
+            } else {
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u)
-                v[u] = load8<I8>(dense, group0 + (unsigned)(u * kColsPerStep + lane * kColsPerLane), row_lo, row_hi, total, vec_ok);
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const unsigned step0 = group0 + (unsigned)(u * kColsPerStep), g0 = step0 + (unsigned)(lane * kColsPerLane);
-            if (!inner && step0 >= row_hi) break;   // warp-uniform
-            unsigned w[4];
-            words_of<I8>(v[u], w);
-            if (!inner) clear_outside(w, g0, row_lo, row_hi);
-            const unsigned fields = nonzero_fields(w);
-            count += __popc(fields);
-            const unsigned any = __ballot_sync(0xffffffffu, fields != 0u);
-            const int step_c0 = (int)(step0 - row_lo);   // may be negative on the first step
-            if (any == 0xffffffffu && ends_dense) {
-                last = fields;
-                last_c0 = step_c0 + 31 * kColsPerLane;
-                carry = kCarryInLast;
-                continue;
+                for (int u = 0; u < kUnroll; ++u)
+                    v[u] = load8<I8>(dense, group0 + (unsigned)(u * kColsPerStep + lane * kColsPerLane), row_lo, row_hi, total, vec_ok);
             }
-            if (carry == kCarryInLast) carry = last_c0 + 31 - __clz(ordered_bits(__shfl_sync(0xffffffffu, last, 31)));
-            ends_dense = (int)any < 0;   // lane 31
-            if (any == 0u) continue;
-            const int c0 = step_c0 + lane * kColsPerLane;
-            const unsigned nz = ordered_bits(fields);
-            const int my_last = c0 + (31 - __clz(nz | 1u));
-            const int prev = prev_nonzero_before_lane(any, lane, my_last, carry);
-            if (nz) count += (c0 + (__ffs(nz) - 1) - prev - 1) >> 4;
-            carry = __shfl_sync(0xffffffffu, my_last, 31 - __clz(any));
-        }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-    if constexpr (I8) {
-        if (carry == kCarryInLast) carry = last_c0 + 31 - __clz(ordered_bits(__shfl_sync(0xffffffffu, last, 31)));
-        count += (cols - 1 - carry) >> 4;
+            for (int u = 0; u < kUnroll; ++u) {
+                const unsigned step0 = group0 + (unsigned)(u * kColsPerStep), g0 = step0 + (unsigned)(lane * kColsPerLane);
+                if (!inner && step0 >= row_hi) break;   // warp-uniform
+                unsigned w[4];
+                words_of<I8>(v[u], w);
+                if (!inner) clear_outside(w, g0, row_lo, row_hi);
+                const unsigned fields = nonzero_fields(w);
+                count += __popc(fields);
+                const unsigned any = __ballot_sync(0xffffffffu, fields != 0u);
+                const int step_c0 = (int)(step0 - row_lo);   // may be negative on the first step
+                if (any == 0xffffffffu && ends_dense) {
+                    last = fields;
+                    last_c0 = step_c0 + 31 * kColsPerLane;
+                    carry = kCarryInLast;
+                    continue;
+                }
+                if (carry == kCarryInLast) carry = last_c0 + 31 - __clz(ordered_bits(__shfl_sync(0xffffffffu, last, 31)));
+                ends_dense = (int)any < 0;   // lane 31
+                if (any == 0u) continue;
+                const int c0 = step_c0 + lane * kColsPerLane;
+                const unsigned nz = ordered_bits(fields);
+                const int my_last = c0 + (31 - __clz(nz | 1u));
+                const int prev = prev_nonzero_before_lane(any, lane, my_last, carry);
+                if (nz) count += (c0 + (__ffs(nz) - 1) - prev - 1) >> 4;
+                carry = __shfl_sync(0xffffffffu, my_last, 31 - __clz(any));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
+        if constexpr (I8) {
+            if (carry == kCarryInLast) carry = last_c0 + 31 - __clz(ordered_bits(__shfl_sync(0xffffffffu, last, 31)));
+            count += (cols - 1 - carry) >> 4;
+        }
+        if (lane == 0) counts[row + 1] = count;
     }
-    if (lane == 0) counts[row + 1] = count;
 }
 
 // ---- emit: values and packed deltas in one pass ----------------------------------------------------------
@@ -293,6 +295,17 @@ __device__ __forceinline__ void ring_flush(EmitRing &r, typename Raw<I8>::Elemen
     __syncwarp();
 }
 
+// Clears the deltas. The emit kernel is its programmatic dependent: its CTAs move in, read their row offsets and fetch their first
+// columns while this runs, and wait for it before they write.
+__global__ void __launch_bounds__(256) clear_deltas_kernel(unsigned *__restrict__ deltas32, unsigned words)
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    const unsigned stride = gridDim.x * 256u, i0 = blockIdx.x * 256u + threadIdx.x;
+    const unsigned vecs = (reinterpret_cast<uintptr_t>(deltas32) & 15) == 0 ? words >> 2 : 0u;
+    for (unsigned i = i0; i < vecs; i += stride) reinterpret_cast<uint4 *>(deltas32)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (unsigned i = (vecs << 2) + i0; i < words; i += stride) deltas32[i] = 0u;
+}
+
 // `nan_add`: what lifts the bits (without sign) of every NaN of the value type to 0x8000 and above, in both halves
 // of a word: 0x7fff minus the bits of +infinity. Every NaN is stored as 0x7fff (what the reference's float round
 // trip makes of it, cpu_compressor.cuh:26,36). Not used with int8 values.
@@ -352,6 +365,7 @@ emit_rows_kernel(const typename Raw<I8>::Element *__restrict__ dense, int rows, 
         }
     };
     fetch(first, v_next);
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the deltas are cleared
 #pragma unroll 1
     for (unsigned step0 = first; step0 < row_hi; step0 += 32u * kEmitCols) {
         const unsigned g0 = step0 + (unsigned)(lane * kEmitCols);
@@ -547,6 +561,14 @@ int launch_row_scan(int *counts, int rows, cudaStream_t stream, int *total)
 
 }  // namespace macko
 
+// Rows that a warp of the counting kernel takes one after the other: as many as make one round of the warps that the GPU holds
+// at a time (48 on each of 148 SMs), so that no second round runs mostly empty.
+static int count_rows_per_warp(int64_t rows)
+{
+    const int64_t n = (rows + 148 * 48 - 1) / (148 * 48);
+    return (int)(n < 1 ? 1 : n > 8 ? 8 : n);
+}
+
 template <bool I8>
 static int compress_count_typed(const void *dense, int64_t rows, int64_t cols, int32_t *row_indices, int32_t *total, void *stream)
 {
@@ -558,9 +580,10 @@ static int compress_count_typed(const void *dense, int64_t rows, int64_t cols, i
     if (!aligned(row_indices, 4)) return fail(MACKO_ERR_MISALIGNED, "row_indices must be 4-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (rows > 0) {
-        const unsigned grid = (unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta);
+        const int per_warp = count_rows_per_warp(rows);
+        const unsigned grid = (unsigned)((rows + kWarpsPerCta * per_warp - 1) / (kWarpsPerCta * per_warp));
         count_rows_kernel<I8><<<grid, kThreads, 0, s>>>(static_cast<const Element *>(dense), (int)rows, (int)cols,
-                                                        aligned(dense, 8 * sizeof(Element)), row_indices);
+                                                        aligned(dense, 8 * sizeof(Element)), per_warp, row_indices);
         st = launch_error("compress count launch");
         if (st != MACKO_OK) return st;
     }
@@ -576,18 +599,31 @@ static int compress_emit_typed(const void *dense, int64_t rows, int64_t cols, co
     using Element = typename Raw<I8>::Element;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // Boundary groups of neighbouring rows merge their nibbles into one word: the deltas start at zero.
-    cudaError_t e = cudaMemsetAsync(deltas, 0, (size_t)padded_count / 2, s);
-    if (e == cudaSuccess && rows == 0) e = cudaMemsetAsync(values, 0, (size_t)padded_count * sizeof(Element), s);
-    if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "clearing the outputs: %s", cudaGetErrorString(e));
-    if (rows > 0) {
-        const unsigned grid = (unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta);
-        emit_rows_kernel<I8><<<grid, kThreads, 0, s>>>(
-            static_cast<const Element *>(dense), (int)rows, (int)cols, aligned(dense, 8 * sizeof(Element)), row_indices,
-            static_cast<Element *>(values), static_cast<unsigned *>(deltas), (int)padded_count,
-            (0x7fffu - infinity_bits) * 0x10001u, aligned(values, 8 * sizeof(Element)));
-        return launch_error("compress emit launch");
+    if (rows == 0) {
+        cudaError_t e = cudaMemsetAsync(deltas, 0, (size_t)padded_count / 2, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(values, 0, (size_t)padded_count * sizeof(Element), s);
+        if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "clearing the outputs: %s", cudaGetErrorString(e));
+        return MACKO_OK;
     }
-    return MACKO_OK;
+    const unsigned words = (unsigned)(padded_count >> 3);   // a multiple of 8 stored elements: whole words
+    clear_deltas_kernel<<<(unsigned)((words + 4095u) / 4096u < 592u ? (words + 4095u) / 4096u : 592u), 256, 0, s>>>(static_cast<unsigned *>(deltas), words);
+    const int st = launch_error("clearing the deltas");
+    if (st != MACKO_OK) return st;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta));
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = use_pdl() ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, emit_rows_kernel<I8>,
+        static_cast<const Element *>(dense), (int)rows, (int)cols, aligned(dense, 8 * sizeof(Element)), row_indices,
+        static_cast<Element *>(values), static_cast<unsigned *>(deltas), (int)padded_count,
+        (0x7fffu - infinity_bits) * 0x10001u, aligned(values, 8 * sizeof(Element)));
+    if (e != cudaSuccess) return fail(MACKO_ERR_CUDA, "compress emit launch: %s", cudaGetErrorString(e));
+    return launch_error("compress emit launch");
 }
 
 template <bool I8>
