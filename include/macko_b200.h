@@ -122,8 +122,9 @@ int macko_spmv_fp16_tuned(const void *values, const void *deltas, const int32_t 
                           int lanes_per_row, int steps_in_flight, int x_in_shared, int ctas_per_sm);
 
 /*
- * The launch shape macko_spmv_fp16 picks for a matrix on a GPU with `sm_count` SMs: lanes per row (4, 8, 16
- * or 32) and 8-element units in flight per lane (2, 4 or 6), the two arguments macko_spmv_fp16_tuned takes.
+ * The best launch shape among those that macko_spmv_fp16_tuned can take, for a matrix on a GPU with `sm_count` SMs: lanes per
+ * row (4, 8, 16 or 32) and 8-element units in flight per lane (2, 4 or 6), its two arguments. macko_spmv_fp16 uses it for short
+ * rows; for longer ones it also has CTAs of 1024 threads and a tail of rows that are walked with a warp each.
  * Pure host arithmetic (no CUDA call), for logging and for tests of the heuristic. No counterpart in the
  * reference, whose launch shape is fixed (32 x 32 threads, one warp per row, kernels_torch_launchers.cuh:15-16).
  */

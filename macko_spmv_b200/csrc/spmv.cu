@@ -227,7 +227,7 @@ struct Extra {
 //       previous kernel of the stream and before x is staged (a separate instantiation, so that the default
 //       launch keeps the simpler code: wait, stage x, then walk the rows)
 // TAIL  the last `tail_rows` rows are walked with a warp per row (see choose_tail)
-// T     threads of a CTA: 512, two CTAs on an SM, or 1024, one CTA and one copy of x (see kWideSmem)
+// T     threads of a CTA: 512, two CTAs on an SM, or 1024, one CTA and one copy of x (see choose_launch)
 template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads, bool TAIL = false>
 __global__ void __launch_bounds__(T, kThreadsPerSm / T)
 spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
@@ -873,7 +873,8 @@ int launch_l(int L, int D, const void *values, const void *deltas, const int32_t
     }
 }
 
-// Lanes per row (L) and units in flight per lane (D) for a matrix, calibrated on B200 over row counts
+// Lanes per row (L) and units in flight per lane (D) for two CTAs of 512 threads without a tail: what macko_spmv_fp16_tuned can
+// launch and macko_spmv_shape answers, and the default launch of short rows (choose_launch has the others). Calibrated on B200 over row counts
 // 4096..49152, row lengths 500..25000 stored elements and densities 0.1..0.9:
 //   * fewer lanes per row keep the x gathers of one load instruction close together (fewer shared-memory bank
 //     conflicts, the resource the kernel is bound by) and shorten the cross-lane scan, so the smallest L wins
@@ -886,15 +887,6 @@ int launch_l(int L, int D, const void *values, const void *deltas, const int32_t
 //   * rows shorter than half a sub-step shrink the group further;
 //   * six units in flight once a row holds more than three sub-steps, four above one, else two.
 struct Shape { int L, D; };
-
-// Above this size of x a warp-per-row launch takes CTAs of 1024 threads that share one copy of x instead of two CTAs of 512
-// with a copy each. Two copies of more than 65 KB leave the SM's first-level cache 92 KB or less (28 KB from 41 000 columns on),
-// and the matrix data that its 1024 threads keep in flight, 120 KB with six units a lane, passes through that cache; from
-// 57408 columns on only one CTA of 512 threads fits at all. 1024 / 512 threads (B200, graph of products, matrices declared
-// immutable, us): 12288x49152 d = 0.5 158.6 / 166.1, d = 0.1 46.2 / 49.5, 3000x40000 d = 0.5 37.8 / 40.1; below the line the
-// shared barrier costs as much as it gives: 4096x32768 39.8 / 39.8, 8192x24576 58.1 / 59.0, 4096x11008 d = 0.5 16.1 / 15.2.
-// Groups of fewer lanes are left with two CTAs (not measured).
-constexpr size_t kWideSmem = 65 * 1024;
 Shape choose_shape(long long rows, long long cols, long long padded, int resident_warps)
 {
     const long long avg_row = rows > 0 ? padded / rows : 0;
@@ -925,6 +917,38 @@ int choose_tail(int64_t rows, int block, int64_t warps)
     const int64_t blocks = (rows + block - 1) / block, rounds = blocks / warps, left = blocks - rounds * warps;
     if (rounds == 0 || left == 0 || 2 * left > warps) return 0;
     return (int)(rows - rounds * warps * block);
+}
+
+// The default launch of one vector with x in shared memory and rows long enough for six units in flight. Against choose_shape, the
+// best shape of two CTAs of 512 threads whose last round may be mostly empty, it has the tail and CTAs of 1024 threads, and the rule is
+// simpler. 143 shapes (1024..49152 rows, 2048..49152 columns, d = 0.1..0.9, six launches each): within 0.3 % of the fastest on
+// average and at most 4 %, 2.1 % ahead of choose_shape on average (B200, graph of products, immutable, us, this / before):
+//   lanes   the fewest with which every warp still gets a block of rows: fewer bank conflicts, a shorter scan. 5139x12557 d = 0.15 10.2 / 12.4,
+//           5120x13824 d = 0.5 23.8 / 27.4, 10176x7155 d = 0.24 14.3 / 16.5, 14437x25305 d = 0.75 133.9 / 153.6, but 4693x9710 (not quite a row per
+//           warp) 7.2 with 32 lanes and 7.6 with 16. From 38000 columns on 16 at least: 12288x49152 d = 0.5 155.2, with eight lanes 162.4.
+//           Rows of very uneven length want more lanes; a matrix declared immutable has usually been looked at (such rows get a
+//           plan), any other takes the lower number only from 1.1 times as many rows on: skewed 9600x5000 21.9 with 16 lanes, 28.7
+//           with 8, 5000x6000 16.9 / 18.3.
+//   threads one CTA of 1024 threads and one copy of x, or two of 512. Two large copies leave the SM's first-level cache little room
+//           (28 KB from 41000 columns on), and the matrix data that 1024 threads keep in flight, 120 KB with six units a lane, passes
+//           through it; from 57408 columns on only one CTA of 512 threads fits at all. Fewer lanes per row touch more lines at a time
+//           and need the room earlier: 8 lanes, 1024 / 512 threads: 11623x14035 63.1 / 67.0, 12623x8247 38.0 / 37.5; 16 lanes: 8192x24576 55.4 /
+//           55.7, 6681x46940 53.9 / 58.5, 8234x14855 39.6 / 39.4; a warp per row: 3000x40000 37.8 / 40.1, 4096x28672 35.5 / 35.5, 4096x11008 16.1 /
+//           15.2. Few long rows, less than half a row per warp, take it as well: 1143x29165 18.9 / 21.4, 1286x5290 7.9 / 9.0.
+struct Launch {
+    int L;          // 0: none, the rows are too short
+    int threads;
+    int tail_rows;
+};
+Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, bool immutable)
+{
+    const int64_t warps = (int64_t)sm_count * (kThreadsPerSm / 32), avg_row = padded / rows;
+    // rows from which on there are blocks enough for 16 lanes; for 8 lanes twice as many
+    const int64_t from = immutable ? warps + 1 : (55 * 2 * warps + 99) / 100;
+    const int L = rows < from ? 32 : rows < 2 * from || cols >= 38000 ? 16 : 8;
+    if (avg_row <= 3LL * L * kGroup) return {0, kThreads, 0};
+    const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384 : cols > 33088 || (2 * rows <= warps && avg_row >= 4600);
+    return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps)};
 }
 
 // One launch for up to BV vectors. Lanes per row as in the single-vector product; fewer units in flight with
@@ -977,17 +1001,25 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Extra extra = {};
     extra.flags = flags;
-    if (xs && (L == 8 || L == 16) && D == 6) {
-        extra.tail_rows = choose_tail(rows, 32 / L, (int64_t)dev->sm_count * ctas * kWarpsPerCta);
-        if (extra.tail_rows > 0) {
-            const int r = (int)rows, c = (int)cols;
-            return L == 8 ? launch<8, 3, true, false, 1, false, VT, kThreads, true>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, ctas, Peers{}, 1, extra)
-                          : launch<16, 3, true, false, 1, false, VT, kThreads, true>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, ctas, Peers{}, 1, extra);
+    if (xs) {
+        const Launch best = choose_launch(rows, cols, padded_count, dev->sm_count, (flags & MACKO_SPMV_MATRIX_IMMUTABLE) != 0);
+        extra.tail_rows = best.tail_rows;
+        const int r = (int)rows, c = (int)cols;
+#define MACKO_LAUNCH(LL, T, TAIL) \
+    launch<LL, 3, true, false, 1, false, VT, T, TAIL>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, 0, Peers{}, 1, extra)
+#define MACKO_LAUNCH_T(LL, T) (best.tail_rows > 0 ? MACKO_LAUNCH(LL, T, true) : MACKO_LAUNCH(LL, T, false))
+        switch (best.L * 10 + (best.threads == kThreads ? 0 : 1)) {
+            case 80: return MACKO_LAUNCH_T(8, kThreads);
+            case 81: return MACKO_LAUNCH_T(8, 2 * kThreads);
+            case 160: return MACKO_LAUNCH(16, kThreads, false);   // up to two rows per warp: one round at most
+            case 161: return MACKO_LAUNCH_T(16, 2 * kThreads);
+            case 320: return MACKO_LAUNCH(32, kThreads, false);
+            case 321: return MACKO_LAUNCH(32, 2 * kThreads, false);
+            default: break;   // rows too short for six units in flight
         }
+#undef MACKO_LAUNCH_T
+#undef MACKO_LAUNCH
     }
-    if (xs && L == 32 && D == 6 && smem > kWideSmem)
-        return launch<32, 3, true, false, 1, false, VT, 2 * kThreads>(values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y,
-                                                                      alpha, beta, s, *dev, 0, Peers{}, 1, extra);
     if (xs)
         return launch_l<true, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);
     return launch_l<false, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);

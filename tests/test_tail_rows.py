@@ -16,12 +16,12 @@ DEV = "cuda:0"
 OPS = torch.ops.macko_spmv
 
 
-# 8 lanes: blocks of four rows, 4736 of them a round; 16 lanes: of two, for rows of more than 4096 stored elements
+# 8 lanes: blocks of four rows, 4736 of them a round; 16 lanes: of two, from 38000 columns on
 @pytest.mark.parametrize("rows,cols,d", [(18944, 500, 0.5), (18945, 500, 0.5), (18951, 500, 0.5), (28416, 500, 0.5), (28417, 500, 0.5), (37889, 407, 0.6),
-                                         (9473, 8300, 0.5), (14208, 8300, 0.5), (14211, 8300, 0.5)])
+                                         (18947, 10000, 0.03), (9473, 38000, 0.02), (14208, 38000, 0.02)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.int8])
 def test_product_against_float64(rows, cols, d, dtype):
-    if rows * cols > 40 << 20 and dtype is not torch.float16 and rows != 9473:
+    if rows * cols > 100 << 20 and dtype is not torch.float16:
         pytest.skip("one type for the large ones")
     M = workloads.bernoulli_matrix(rows, cols, d, seed=rows + cols, device=DEV)
     M[-1] = 0
