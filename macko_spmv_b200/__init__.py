@@ -183,21 +183,24 @@ class FrozenMatrix(tuple):
 
     plan = None        # device buffer of the plan, or None
     plan_meta = None   # (virtual_rows, segment_elements, longest_row, split_rows, recommended)
-    windows = None     # device buffer of the column windows that `multiply_batched` walks, or None
-    windows_of = None  # write counts of deltas and row_indices when the windows were built
+    windows = None      # device buffer of the column windows that `multiply_batched` walks, or None
+    windows_of = None   # write counts and addresses of deltas and row_indices when the windows were built (None: not counted)
+    windows_batch = 0   # the largest batch for which the windows are the faster route
 
-    def __new__(cls, compressed, plan=None, plan_meta=None, windows=None, windows_of=None):
+    def __new__(cls, compressed, plan=None, plan_meta=None, windows=None, windows_of=None, windows_batch=0):
         self = super().__new__(cls, tuple(compressed[:5]))
         self.plan = plan
         self.plan_meta = plan_meta
         self.windows = windows
         self.windows_of = windows_of
+        self.windows_batch = windows_batch
         return self
 
 
 if _direct is not None:
     _direct.set_frozen_type(FrozenMatrix)
 _direct_multiply = _direct.multiply if _direct is not None else lambda compressed_M, V: None
+_direct_batched = _direct.multiply_batched if _direct is not None else lambda compressed_M, V: None
 _is_compiling = torch.compiler.is_compiling
 
 
@@ -214,33 +217,64 @@ def freeze(compressed_M, plan="auto", segment_elements=0):
     torch.cuda.synchronize(compressed_M[0].device)
     if plan is False or compressed_M[0].dtype != torch.float16:
         return FrozenMatrix(compressed_M)
-    windows, windows_of = _build_windows(compressed_M)   # before the plan, which waits for the device
+    windows = _build_windows(compressed_M)   # before the plan, which waits for the device
     buf, meta = torch.ops.macko_spmv.plan_build.default(
         compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], compressed_M[0].numel(), int(segment_elements))
     meta = [int(v) for v in meta.tolist()]
     info = (meta[3], meta[4], meta[5], meta[6], meta[7])
     if plan is True or info[4]:
-        return FrozenMatrix(compressed_M, buf, info, windows, windows_of)
-    return FrozenMatrix(compressed_M, None, info, windows, windows_of)
+        return FrozenMatrix(compressed_M, buf, info, *windows)
+    return FrozenMatrix(compressed_M, None, info, *windows)
 
 
-def _write_counts(deltas, row_indices):
-    """How often the two tensors have been written in place, or None where that is not counted (inference tensors)."""
+def _written(deltas, row_indices):
+    """What tells whether the two tensors have been written or moved in place, or None where writes are not counted (inference
+    tensors)."""
     if deltas.is_inference() or row_indices.is_inference():
         return None
-    return deltas._version, row_indices._version
+    return deltas._version, row_indices._version, deltas.data_ptr(), row_indices.data_ptr()
 
 
 def _build_windows(compressed_M):
-    """Column windows of an fp16 matrix (`macko_spmm_windows`) and what they were built from, or (None, None) where the rows are so
-    short that their 8 bytes per row and window would weigh more than 5 % of the matrix."""
+    """(column windows of an fp16 matrix, what they were built from, the largest batch that takes them), or (None, None, 0) where
+    the rows are so short that their 8 bytes per row and window would weigh more than 5 % of the matrix."""
     _, deltas, row_indices, rows, cols = compressed_M[:5]
     stored = 2 * deltas.numel()
     if rows == 0 or rows >= 1 << 30 or cols >= 1 << 24:
-        return None, None
-    if 20 * _core.macko_spmm_windows_bytes(rows, cols, stored) > 2.5 * stored:
-        return None, None
-    return torch.ops.macko_spmv.windows_build.default(deltas, row_indices, rows, cols), _write_counts(deltas, row_indices)
+        return None, None, 0
+    nbytes = _core.macko_spmm_windows_bytes(rows, cols, stored)
+    if 20 * nbytes > 2.5 * stored:
+        return None, None, 0
+    windows = torch.ops.macko_spmv.windows_build.default(deltas, row_indices, rows, cols)
+    return windows, _written(deltas, row_indices), _windows_batch(rows, cols, stored, nbytes // (8 * rows))
+
+
+# Beyond this many right-hand sides the windowed product has never been ahead of the dense copy.
+WINDOWED_BATCH_LIMIT = 64
+
+
+def _windows_batch(rows, cols, stored, windows) -> int:
+    """The largest batch that goes over the column windows of a frozen matrix (`macko_spmm_fp16_windowed`), of 8 or more.
+
+    3..8 vectors always do, where the other choice is one pass of the one-kernel product: 11008x4096 d = 0.5 8 vectors 25.0
+    against 42.4 us, 4 vectors 20.7 / 27.0; 8192x8192 d = 0.3 24.2 / 38.8; 512x512 d = 0.5 5.5 / 6.5 and, the only loss, 3 vectors
+    4.4 / 4.2. Two vectors are level or behind (11008x4096 20.7 / 19.3, 4096x4096 d = 0.7 12.8 / 11.1).
+    Larger batches take every 8 vectors through the matrix, against one dense copy and a GEMM: the two models below, in us, fit 18
+    shapes x 9..48 vectors with a standard deviation of 7 % and 21 %. 16 vectors, windows / copy: 4096x11008 d = 0.5 39.3 / 48.6,
+    d = 0.2 24.8 / 42.6, 4096x4096 d = 0.7 23.4 / 21.3, 16384x4096 d = 0.9 92.6 / 77.3; 24 vectors: 4096x11008 d = 0.2 35.9 / 42.9,
+    11008x4096 d = 0.5 57.4 / 44.0, 1024x16384 d = 0.3 18.9 / 26.9. The GEMM is slower where rows of the copy do not start on
+    16 bytes: 1500x5001 d = 0.15 16 vectors 8.5 / 21.5."""
+    blocks = (rows + 3) // 4
+    copy_us = (6.9 + 0.63e-6 * rows * cols + 0.52e-6 * stored) * (1.0 if cols % 8 == 0 else 1.7)
+    best = 8
+    for batch in range(16, WINDOWED_BATCH_LIMIT + 1, 8):
+        ctas = windows * batch // 8
+        warps = 32 * max(1, 148 // ctas)
+        rounds = 0.5 * (blocks / warps - blocks // -warps) * -(ctas // -148)
+        if 4.6 + 0.74 * rounds * (stored / (64.0 * rows * windows) + 1.5) + 3.7e-6 * windows * rows * batch >= copy_us:
+            break
+        best = batch
+    return best
 
 
 def multiply(compressed_M, V, out=None):
@@ -308,40 +342,16 @@ def decompress(compressed_M):
     return torch.ops.macko_spmv.decompress.default(*compressed_M[:5])
 
 
-# Beyond this many right-hand sides the windowed product has never been ahead of the dense copy.
-WINDOWED_BATCH_LIMIT = 64
-
-
 def _windows_pay(frozen, V) -> bool:
-    """Whether a batch goes over the column windows of a frozen matrix (`macko_spmm_fp16_windowed`).
-
-    3..8 vectors always do, where the other choice is one pass of the one-kernel product: 11008x4096 d = 0.5 8 vectors 25.0
-    against 42.4 us, 4 vectors 20.7 / 27.0; 8192x8192 d = 0.3 24.2 / 38.8; 512x512 d = 0.5 5.5 / 6.5 and, the only loss, 3 vectors
-    4.4 / 4.2. Two vectors are level or behind (11008x4096 20.7 / 19.3, 4096x4096 d = 0.7 12.8 / 11.1).
-    Larger batches take every 8 vectors through the matrix, against one dense copy and a GEMM: the two models below, in us, fit 18
-    shapes x 9..48 vectors with a standard deviation of 7 % and 21 %. 16 vectors, windows / copy: 4096x11008 d = 0.5 39.3 / 48.6,
-    d = 0.2 24.8 / 42.6, 4096x4096 d = 0.7 23.4 / 21.3, 16384x4096 d = 0.9 92.6 / 77.3; 24 vectors: 4096x11008 d = 0.2 35.9 / 42.9,
-    11008x4096 d = 0.5 57.4 / 44.0, 1024x16384 d = 0.3 18.9 / 26.9. The GEMM is slower where rows of the copy do not start on
-    16 bytes: 1500x5001 d = 0.15 16 vectors 8.5 / 21.5."""
+    """Whether a batch goes over the column windows of a frozen matrix."""
     batch = V.shape[0]
-    if frozen.windows is None or batch < 3 or batch > WINDOWED_BATCH_LIMIT or _is_compiling():
+    if batch < 3 or batch > frozen.windows_batch:
         return False
-    if frozen.windows_of != _write_counts(frozen[1], frozen[2]):
+    if frozen.windows_of is not None and frozen.windows_of != _written(frozen[1], frozen[2]):
         return False   # written since: the windows may be those of another matrix
-    if batch <= 8:
-        return True
-    # the dense copy goes through operators that can be differentiated and transformed
-    if (V.requires_grad and torch.is_grad_enabled()) or type(V) is not torch.Tensor or torch._C._functorch.peek_interpreter_stack() is not None \
-            or torch.autograd.forward_ad._current_level >= 0:
-        return False
-    rows, cols, stored = frozen[3], frozen[4], 2 * frozen[1].numel()
-    windows, groups, blocks = frozen.windows.numel() // (8 * rows), (batch + 7) // 8, (rows + 3) // 4
-    ctas = windows * groups
-    warps = 32 * max(1, 148 // ctas)
-    rounds = 0.5 * (blocks / warps - blocks // -warps) * -(ctas // -148)
-    windows_us = 4.6 + 0.74 * rounds * (stored / (64.0 * rows * windows) + 1.5) + 3.7e-6 * windows * rows * batch
-    copy_us = (6.9 + 0.63e-6 * rows * cols + 0.52e-6 * stored) * (1.0 if cols % 8 == 0 else 1.7)
-    return windows_us < copy_us
+    # above 8 vectors the other route is a dense copy and operators that can be differentiated and transformed
+    return batch <= 8 or not ((V.requires_grad and torch.is_grad_enabled()) or type(V) is not torch.Tensor
+                              or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0)
 
 
 def multiply_batched(compressed_M, V):
@@ -353,14 +363,20 @@ def multiply_batched(compressed_M, V):
     the route of the larger batches: decompress once and run a dense GEMM. A frozen matrix (`freeze`) has column windows, over
     which a pass is up to twice as fast, so more batches stay with the compressed matrix.
     """
+    windowed = type(compressed_M) is FrozenMatrix and compressed_M.windows_batch > 0 and not _is_compiling()
+    if windowed:
+        y = _direct_batched(compressed_M, V)   # None: not a plain call of 3..8 vectors
+        if y is not None:
+            return y
     assert compressed_M[0].is_cuda
     assert V.is_cuda
     assert V.is_contiguous()
     if V.dim() != 2:
         raise RuntimeError("V must have shape [batch, cols]")
-    if type(compressed_M) is FrozenMatrix and _windows_pay(compressed_M, V):
+    batch = V.shape[0]
+    if windowed and _windows_pay(compressed_M, V):
         return torch.ops.macko_spmv.multiply_windowed.default(*compressed_M[:5], compressed_M.windows, V, True)
-    if V.shape[0] > DENSE_BATCH_THRESHOLD or _dense_copy_pays(compressed_M, V.shape[0]):
+    if batch > DENSE_BATCH_THRESHOLD or (windowed and batch > compressed_M.windows_batch) or _dense_copy_pays(compressed_M, batch):
         return V @ decompress(compressed_M).t()
     return torch.ops.macko_spmv.multiply_batched.default(*compressed_M[:5], V)
 

@@ -249,6 +249,10 @@ at::Tensor windows_build_cuda(const at::Tensor &deltas, const at::Tensor &ri, in
     return windows;
 }
 
+}  // namespace
+
+namespace macko_torch {
+
 // Y[batch, rows] for V[batch, cols] over the matrix's column windows. The partial sums are scratch of this call alone.
 at::Tensor multiply_windowed_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
                                   int64_t rows, int64_t cols, const at::Tensor &windows, const at::Tensor &V, bool frozen)
@@ -271,6 +275,12 @@ at::Tensor multiply_windowed_cuda(const at::Tensor &values, const at::Tensor &de
                  "macko_spmm_fp16_windowed");
     return y;
 }
+
+}  // namespace macko_torch
+
+namespace {
+
+using macko_torch::multiply_windowed_cuda;
 
 at::Tensor decompress_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
                            int64_t rows, int64_t cols)

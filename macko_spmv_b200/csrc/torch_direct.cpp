@@ -1,4 +1,4 @@
-// `multiply` without the operator dispatcher, a Python module beside the operator library.
+// `multiply` and the batched product of a frozen matrix without the operator dispatcher, a Python module beside the operator library.
 //
 // A product of a small matrix takes less time on the GPU than the way of its arguments through the operator boundary
 // (Python asserts, schema matching, boxing). The module function below takes that way out for calls that only
@@ -20,7 +20,7 @@
 namespace {
 
 PyObject *g_frozen_type = nullptr;   // macko_spmv_b200.FrozenMatrix
-PyObject *g_plan_name = nullptr, *g_plan_meta_name = nullptr;
+PyObject *g_plan_name = nullptr, *g_plan_meta_name = nullptr, *g_windows_name = nullptr, *g_windows_of_name = nullptr;
 
 bool nobody_watches()
 {
@@ -91,6 +91,59 @@ PyObject *direct_multiply(PyObject *, PyObject *const *args, Py_ssize_t n_args)
     END_HANDLE_TH_ERRORS
 }
 
+// Attribute `name` of a frozen matrix; the new reference is dropped at once, the attribute outlives the call in the matrix.
+PyObject *attribute(PyObject *m, PyObject *name)
+{
+    PyObject *p = PyObject_GetAttr(m, name);
+    Py_XDECREF(p);
+    return p;
+}
+
+// Whether the tensors that the windows were built from are as they were: `of` = (write count of the deltas, of the row offsets, their
+// addresses), or None where writes are not counted.
+bool as_built(PyObject *of, const at::Tensor &deltas, const at::Tensor &ri)
+{
+    if (of == Py_None) return true;
+    if (!PyTuple_CheckExact(of) || PyTuple_GET_SIZE(of) != 4 || deltas.is_inference() || ri.is_inference()) return false;
+    const int64_t now[4] = {deltas._version(), ri._version(), reinterpret_cast<int64_t>(deltas.data_ptr()), reinterpret_cast<int64_t>(ri.data_ptr())};
+    for (int i = 0; i < 4; ++i) {
+        int64_t was;
+        if (!as_int64(PyTuple_GET_ITEM(of, i), was) || was != now[i]) return false;
+    }
+    return true;
+}
+
+// multiply_batched(compressed, V) -> y for 3..8 vectors of a frozen matrix with windows, or None where the call has to take another route
+PyObject *direct_multiply_batched(PyObject *, PyObject *const *args, Py_ssize_t n_args)
+{
+    HANDLE_TH_ERRORS
+    PyObject *m = n_args == 2 ? args[0] : nullptr;
+    if (!m || reinterpret_cast<PyObject *>(Py_TYPE(m)) != g_frozen_type || PyTuple_GET_SIZE(m) < 5) Py_RETURN_NONE;
+    const at::Tensor *V = plain_tensor(args[1]);
+    if (!V || V->dim() != 2 || V->size(0) < 3 || V->size(0) > 8 || !V->is_contiguous() || !nobody_watches()) Py_RETURN_NONE;
+    const at::Tensor *values = plain_tensor(PyTuple_GET_ITEM(m, 0)), *deltas = plain_tensor(PyTuple_GET_ITEM(m, 1)),
+                     *ri = plain_tensor(PyTuple_GET_ITEM(m, 2));
+    int64_t rows, cols;
+    if (!values || !deltas || !ri || !as_int64(PyTuple_GET_ITEM(m, 3), rows) || !as_int64(PyTuple_GET_ITEM(m, 4), cols))
+        Py_RETURN_NONE;
+    PyObject *w = attribute(m, g_windows_name);
+    if (!w) return nullptr;
+    const at::Tensor *windows = plain_tensor(w);
+    if (!windows) Py_RETURN_NONE;
+    PyObject *of = attribute(m, g_windows_of_name);
+    if (!of) return nullptr;
+    if (!as_built(of, *deltas, *ri)) Py_RETURN_NONE;
+    // own handles: another thread may drop the Python ones while the interpreter lock is released
+    const at::Tensor v = *values, d = *deltas, r = *ri, x = *V, win = *windows;
+    at::Tensor y;
+    {
+        struct NoGil { PyThreadState *s = PyEval_SaveThread(); ~NoGil() { PyEval_RestoreThread(s); } } no_gil;
+        y = macko_torch::multiply_windowed_cuda(v, d, r, rows, cols, win, x, true);
+    }
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
 // set_frozen_type(FrozenMatrix): the class that `freeze` returns
 PyObject *set_frozen_type(PyObject *, PyObject *type)
 {
@@ -101,6 +154,7 @@ PyObject *set_frozen_type(PyObject *, PyObject *type)
 
 PyMethodDef g_methods[] = {
     {"multiply", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&direct_multiply)), METH_FASTCALL, nullptr},
+    {"multiply_batched", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&direct_multiply_batched)), METH_FASTCALL, nullptr},
     {"set_frozen_type", &set_frozen_type, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_direct", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
@@ -111,5 +165,7 @@ PyMODINIT_FUNC PyInit__torch_direct()
 {
     g_plan_name = PyUnicode_InternFromString("plan");
     g_plan_meta_name = PyUnicode_InternFromString("plan_meta");
-    return g_plan_name && g_plan_meta_name ? PyModule_Create(&g_module) : nullptr;
+    g_windows_name = PyUnicode_InternFromString("windows");
+    g_windows_of_name = PyUnicode_InternFromString("windows_of");
+    return g_plan_name && g_plan_meta_name && g_windows_name && g_windows_of_name ? PyModule_Create(&g_module) : nullptr;
 }

@@ -16,4 +16,8 @@ at::Tensor multiply_planned_cuda(const at::Tensor &values, const at::Tensor &del
                                  const at::Tensor &plan, int64_t virtual_rows, int64_t segment_elements, int64_t split_rows,
                                  const at::Tensor &V, bool frozen);
 
+// y[batch, rows] for V[batch, cols] over the matrix's column windows.
+at::Tensor multiply_windowed_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri, int64_t rows, int64_t cols,
+                                  const at::Tensor &windows, const at::Tensor &V, bool frozen);
+
 }  // namespace macko_torch

@@ -68,17 +68,13 @@ class MackoLinear(nn.Module):
     def compressed(self):
         return (self.c_0, self.c_1, self.c_2, self.out_features, self.in_features)
 
-    def _frozen_as_is(self, x):
-        """The frozen matrix if it still holds this layer's buffers and they can be looked at (not in a traced or
-        transformed call, whose tensors stand for others)."""
-        fz = self._frozen
-        if fz is None or torch.compiler.is_compiling() or type(x) is not torch.Tensor or type(self.c_0) is not torch.Tensor:
+    def _frozen_as_is(self):
+        """The frozen matrix if its buffers are still this layer's (not where a traced or transformed call has put others in
+        their place)."""
+        fz, own = self._frozen, self._buffers
+        if torch.compiler.is_compiling():
             return None
-        try:
-            same = all(a.data_ptr() == b.data_ptr() for a, b in zip(fz, (self.c_0, self.c_1, self.c_2)))
-        except RuntimeError:   # a tensor without storage
-            return None
-        return fz if same else None
+        return fz if fz is not None and fz[0] is own["c_0"] and fz[1] is own["c_1"] and fz[2] is own["c_2"] else None
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         from . import multiply, multiply_batched
@@ -94,8 +90,7 @@ class MackoLinear(nn.Module):
                 fz = self._frozen = None   # the buffers were replaced since freeze(): back to the safe path
             y = multiply(fz if fz is not None else comp, flat[0].contiguous()).unsqueeze(0)
         else:
-            fz = self._frozen_as_is(flat)
-            y = multiply_batched(fz if fz is not None else comp, flat.contiguous())
+            y = multiply_batched(self._frozen_as_is() or comp, flat.contiguous())
         if self.bias is not None:
             y = y + self.bias
         return y.reshape(*lead, self.out_features)

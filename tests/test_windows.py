@@ -205,14 +205,14 @@ def test_layers_follow_their_buffers():
     x = torch.randn(7, 3000, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).half()
     _check(layer(x), W, x, "layer")
     _check(copy.deepcopy(layer)(x), W, x, "copied layer")
-    assert layer._frozen_as_is(x) is layer._frozen
+    assert layer._frozen_as_is() is layer._frozen
     W2 = W.roll(7, 0).contiguous()   # the same rows in another order: buffers of the same sizes
     two = MackoLinear(macko_spmv.compress(W2))
     assert two.c_0.shape == layer.c_0.shape
     layer.load_state_dict(two.state_dict())   # writes the frozen buffers in place, without another freeze()
     _check(layer(x), W2, x, "reloaded layer")
     layer.c_0, layer.c_1, layer.c_2 = (t.clone() for t in MackoLinear(macko_spmv.compress(W)).compressed[:3])
-    assert layer._frozen_as_is(x) is None
+    assert layer._frozen_as_is() is None
     _check(layer(x), W, x, "replaced buffers")
 
 
