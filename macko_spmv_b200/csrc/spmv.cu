@@ -226,9 +226,11 @@ struct Extra {
 // EARLY the caller has declared the matrix immutable: the first matrix loads are issued before the wait for the
 //       previous kernel of the stream and before x is staged (a separate instantiation, so that the default
 //       launch keeps the simpler code: wait, stage x, then walk the rows)
+// ROLL  a lane's next units are fetched one pair at a time as its units are worked on, not all at once at the top of an iteration:
+//       the loads of a long row stay in flight while it is walked (for the line see choose_launch)
 // TAIL  the last `tail_rows` rows are walked with a warp per row (see choose_tail)
 // T     threads of a CTA: 512, two CTAs on an SM, or 1024, one CTA and one copy of x (see choose_launch)
-template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads, bool TAIL = false>
+template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads, bool TAIL = false, bool ROLL = PLAN>
 __global__ void __launch_bounds__(T, kThreadsPerSm / T)
 spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
             const int *__restrict__ ri, const __half *__restrict__ x, __half *__restrict__ y,
@@ -384,6 +386,8 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
 #pragma unroll
         for (int b = 0; b < BV; ++b) accb[b][0] = accb[b][1] = 0.f;
 
+        uint4 v[D];
+        unsigned w[D];
         if constexpr (FIRST && !EARLY) stage_x();
         bool first_pass = EARLY && FIRST;
         for (;;) {
@@ -476,30 +480,28 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
                 if (done) break;
             }
 
-            // ---- issue the loads of the whole iteration ------------------------------------------------------
-            uint4 v[D];
-            unsigned w[D];
+            // ---- matrix loads: the units of the whole iteration (ROLL: of a row just taken; the others were issued when the units D in
+            //      front of them had been worked on) --------------------------------------------------------------------
             const int ord0 = (int)(pos + (unsigned)(lig * kGroup));   // not negative where it is used as an index
             const int rem0 = (int)(end - (unsigned)ord0);    // elements of the row from the lane's first unit on
             const int lo0 = (int)(begin - (unsigned)ord0);   // > 0: leading elements of sub-step 0 belong to the previous row
-            {
-                const uint4 *vp = values + (ord0 >> 3);
-                const unsigned *dp = deltas + (ord0 >> 3);
-#pragma unroll
-                for (int s = 0; s < D; ++s) {
-                    v[s] = make_uint4(0u, 0u, 0u, 0u);
-                    w[s] = 0u;
-                    if (s * STEP < rem0) {
-                        if constexpr (VT == kI8) {
-                            const uint2 t = ldg_stream_v2(reinterpret_cast<const uint2 *>(values) + (ord0 >> 3) + s * LN);
-                            v[s].x = t.x;
-                            v[s].y = t.y;
-                        } else {
-                            v[s] = ldg_stream_v4(vp + s * LN);
-                        }
-                        w[s] = ldg_stream_u32(dp + s * LN);
+            auto load_unit = [&](int s, int step) {
+                v[s] = make_uint4(0u, 0u, 0u, 0u);
+                w[s] = 0u;
+                if (step * STEP < rem0) {
+                    if constexpr (VT == kI8) {
+                        const uint2 t = ldg_stream_v2(reinterpret_cast<const uint2 *>(values) + (ord0 >> 3) + step * LN);
+                        v[s].x = t.x;
+                        v[s].y = t.y;
+                    } else {
+                        v[s] = ldg_stream_v4(values + (ord0 >> 3) + step * LN);
                     }
+                    w[s] = ldg_stream_u32(deltas + (ord0 >> 3) + step * LN);
                 }
+            };
+            if (!ROLL || (needmask != 0u && need)) {
+#pragma unroll
+                for (int s = 0; s < D; ++s) load_unit(s, s);
             }
 
             // ---- first pass only: with the first matrix loads in flight, wait for the previous kernel of the
@@ -627,6 +629,7 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
                         acc2 = fma_h<0, VT == kBF16 ? kBF16 : kF16>(acc2, vw[3], xe[3]);
                         acc3 = fma_h<1, VT == kBF16 ? kBF16 : kF16>(acc3, vw[3], xo[3]);
                     }
+                    if constexpr (ROLL) load_unit(s, s + D);
                 }
             }
             // every sub-step that was skipped lies behind the end of all rows of the warp: `run` is not used again before the next row resets it
@@ -774,27 +777,27 @@ __global__ void peer_wait_kernel(unsigned *flags, int world, unsigned spin_limit
     flags[world + 2] = 1u + (unsigned)p;   // gave up: the host can read which rank never arrived
 }
 
-template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T, bool TAIL>
+template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T, bool TAIL, bool ROLL>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra);
 
 // The instantiation with or without early matrix loads, by the immutable-matrix flag of the call.
-template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads, bool TAIL = false>
+template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads, bool TAIL = false, bool ROLL = PLAN>
 int launch(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
            const void *x, void *y, float alpha, float beta, cudaStream_t stream,
            const DeviceInfo &dev, int ctas_per_sm, const Peers &peers = Peers{}, int batch = 1, const Extra &extra = Extra{})
 {
     if constexpr (BV == 1) {
         if (extra.flags & MACKO_SPMV_MATRIX_IMMUTABLE)
-            return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, true, T, TAIL>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
+            return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, true, T, TAIL, ROLL && (L == 8 || PLAN)>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
                                                                          stream, dev, ctas_per_sm, peers, batch, extra);
     }
-    return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, false, T, TAIL>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
+    return launch_variant<L, NPAIR, XS, PEER, BV, PLAN, VT, false, T, TAIL, ROLL && (L == 32 || PLAN)>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta,
                                                                   stream, dev, ctas_per_sm, peers, batch, extra);
 }
 
-template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T, bool TAIL>
+template <int L, int NPAIR, bool XS, bool PEER, int BV, bool PLAN, int VT, bool EARLY, int T, bool TAIL, bool ROLL>
 int launch_variant(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
                    const void *x, void *y, float alpha, float beta, cudaStream_t stream,
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra)
@@ -805,7 +808,7 @@ int launch_variant(const void *values, const void *deltas, const int32_t *ri, in
     if (smem > (size_t)dev.max_smem_optin)
         return fail(MACKO_ERR_INVALID_ARGUMENT, "the launch needs %lld bytes of shared memory, the device offers %d (cols=%d)",
                     (long long)smem, dev.max_smem_optin, cols);
-    auto kernel = spmv_kernel<L, NPAIR, XS, PEER, BV, PLAN, VT, EARLY, T, TAIL>;
+    auto kernel = spmv_kernel<L, NPAIR, XS, PEER, BV, PLAN, VT, EARLY, T, TAIL, ROLL>;
     if (smem > 48 * 1024) {
         // Idempotent and cheap; set on every call so that every device is covered.
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -910,7 +913,7 @@ Shape choose_shape(long long rows, long long cols, long long padded, int residen
 // pipe of the SM well enough that nothing is gained (28000x3000 d = 0.5, 1.48 rounds: 24.2 / 24.0), and a matrix of less than one round
 // would only lose the compact groups' fewer bank conflicts. With / without (B200, graph of products, immutable, us):
 // 22016x4096 (1.16 rounds) d = 0.5 26.3 / 29.3, d = 0.9 38.6 / 44.4, d = 0.1 11.5 / 11.5, 21000x9000 d = 0.4 (1.11) 44.1 / 50.0, 42000x4096
-// d = 0.3 (2.22) 31.6 / 33.2; 16 lanes: 10000x8192 d = 0.5 (1.06) 28.2 / 30.6, 12288x11008 (1.30) 38.0 / 40.6. A kernel of its own: with the
+// d = 0.3 (2.22) 31.6 / 33.2; walked with 16 lanes, 10000x8192 d = 0.5 (1.06) 28.2 / 30.6, 12288x11008 (1.30) 38.0 / 40.6. A kernel of its own: with the
 // second walk in the code, launches that do not need it took up to 3 % longer.
 int choose_tail(int64_t rows, int block, int64_t warps)
 {
@@ -935,10 +938,15 @@ int choose_tail(int64_t rows, int block, int64_t warps)
 //           and need the room earlier: 8 lanes, 1024 / 512 threads: 11623x14035 63.1 / 67.0, 12623x8247 38.0 / 37.5; 16 lanes: 8192x24576 55.4 /
 //           55.7, 6681x46940 53.9 / 58.5, 8234x14855 39.6 / 39.4; a warp per row: 3000x40000 37.8 / 40.1, 4096x28672 35.5 / 35.5, 4096x11008 16.1 /
 //           15.2. Few long rows, less than half a row per warp, take it as well: 1143x29165 18.9 / 21.4, 1286x5290 7.9 / 9.0.
+//   roll    loads that stay in flight while a row is walked: from five iterations a row on with 8 lanes, 32000x4096 d = 0.5 35.1 / 36.3, 12288x4096
+//           15.9 / 16.4, d = 0.9 51.7 / 52.3, and with a warp per row where fewer than half of the warps have one and the matrix may
+//           change (no loads in front of the wait): 838x15588 d = 0.74 14.4 / 16.9, 520x11301 d = 0.37 6.7 / 7.6. Elsewhere the extra
+//           instructions cost up to 8 % (4096x4096 plain 8.9 / 8.2, int8 11008x4096 14.7 / 14.2). The planned launch rolls as well: 46.5 / 46.9.
 struct Launch {
     int L;          // 0: none, the rows are too short
     int threads;
     int tail_rows;
+    bool roll;      // built for 8 lanes of 16-bit values of an immutable matrix and for a warp per row of any other
 };
 Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, bool immutable)
 {
@@ -946,9 +954,10 @@ Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, b
     // rows from which on there are blocks enough for 16 lanes; for 8 lanes twice as many
     const int64_t from = immutable ? warps + 1 : (55 * 2 * warps + 99) / 100;
     const int L = rows < from ? 32 : rows < 2 * from || cols >= 38000 ? 16 : 8;
-    if (avg_row <= 3LL * L * kGroup) return {0, kThreads, 0};
+    if (avg_row <= 3LL * L * kGroup) return {0, kThreads, 0, false};
     const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384 : cols > 33088 || (2 * rows <= warps && avg_row >= 4600);
-    return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps)};
+    return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps),
+            immutable ? L == 8 && avg_row >= 1900 : L == 32 && 2 * rows <= warps && avg_row >= 3600};
 }
 
 // One launch for up to BV vectors. Lanes per row as in the single-vector product; fewer units in flight with
@@ -1005,8 +1014,9 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
         const Launch best = choose_launch(rows, cols, padded_count, dev->sm_count, (flags & MACKO_SPMV_MATRIX_IMMUTABLE) != 0);
         extra.tail_rows = best.tail_rows;
         const int r = (int)rows, c = (int)cols;
-#define MACKO_LAUNCH(LL, T, TAIL) \
-    launch<LL, 3, true, false, 1, false, VT, T, TAIL>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, 0, Peers{}, 1, extra)
+#define MACKO_LAUNCH_R(LL, T, TAIL, ROLL) \
+    launch<LL, 3, true, false, 1, false, VT, T, TAIL, ROLL>(values, deltas, row_indices, r, c, padded_count, x, y, alpha, beta, s, *dev, 0, Peers{}, 1, extra)
+#define MACKO_LAUNCH(LL, T, TAIL) (best.roll ? MACKO_LAUNCH_R(LL, T, TAIL, LL == 32 || (LL == 8 && VT != kI8)) : MACKO_LAUNCH_R(LL, T, TAIL, false))
 #define MACKO_LAUNCH_T(LL, T) (best.tail_rows > 0 ? MACKO_LAUNCH(LL, T, true) : MACKO_LAUNCH(LL, T, false))
         switch (best.L * 10 + (best.threads == kThreads ? 0 : 1)) {
             case 80: return MACKO_LAUNCH_T(8, kThreads);
@@ -1019,6 +1029,7 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
         }
 #undef MACKO_LAUNCH_T
 #undef MACKO_LAUNCH
+#undef MACKO_LAUNCH_R
     }
     if (xs)
         return launch_l<true, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);

@@ -8,8 +8,8 @@
 // rows; the sums of a row over the windows are added by a second small kernel, in window order, so y is reproducible.
 //
 // Measured (B200, graph of products of rotating matrices, us, one kernel for all columns / windows): 8 vectors, 11008x4096 d = 0.5
-// 42.4 / 25.0, 4096x11008 d = 0.5 47.6 / 23.9, 16384x4096 d = 0.9 106.5 / 50.4, 4096x4096 d = 0.3 17.9 / 10.9, skewed 8192x28672 339.6 /
-// 111.8; 4 vectors, 11008x4096 27.0 / 20.7, 32000x4096 d = 0.5 64.4 / 47.0. What bounds it: the four passes of a 16-byte gather, 32 of
+// 42.4 / 24.5, 4096x11008 d = 0.5 47.6 / 23.9, 16384x4096 d = 0.9 106.5 / 49.2, 4096x4096 d = 0.3 17.9 / 10.7, skewed 8192x28672 339.6 /
+// 111.8; 4 vectors, 11008x4096 27.0 / 20.7, 32000x4096 d = 0.5 64.4 / 44.6. What bounds it: the four passes of a 16-byte gather, 32 of
 // about 44 passes of the load/store pipe per 8 x 32 elements, then the walk of the few blocks of rows that a warp gets.
 #include "common.cuh"
 #include "unit.cuh"
@@ -115,8 +115,10 @@ __device__ __forceinline__ float group_sums(float (&a)[BV], int lane)
 // of blocks of four rows and walks the rows of a block in step: they reach their ends together, so that the sums, the stores
 // and the next block's set-up run once per block for all four (rows that differ in length wait for the longest; a walk in
 // which every group fetched its own next row, as in spmv.cu, took 27.0 us instead of 24.6). The next block's section is
-// fetched while this one is walked; the first sub-steps of the first block are in flight while x is staged and, for an
-// immutable matrix, before the wait for the kernel in front.
+// fetched while this one is walked, and its first units while this one's sums are formed: a unit's registers take the unit D sub-steps on
+// as soon as it has been worked on, so a warp always has D of them in flight (8 vectors, all units of an iteration at its top /
+// like this: 32000x4096 d = 0.5 58.1 / 55.5 us, 2048x2048 7.8 / 7.0, 11008x4096 25.0 / 24.5; 16384x1024 9.0 / 9.2). The first units of the
+// first block are in flight while x is staged and, for an immutable matrix, before the wait for the kernel in front.
 template <int BV>
 __global__ void __launch_bounds__(kThreads, 1)
 windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas, const uint2 *__restrict__ sections,
@@ -169,42 +171,44 @@ windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ de
     const int x_base = (int)smem0 + (BV == 4 ? 8 * (lane & 15) : 16 * (lane & 7));
     const unsigned lane_const = (unsigned)(2 * lig);
     const unsigned a_max = (unsigned)(2 * (kWindowFront + here));
-    bool staged = false;
-    do {   // a warp without rows comes through once as well, for the staging
+    // where the rows of the block stand: first unit of the next sub-step, elements left from there, their columns
+    unsigned run = 0u, pos = 0u;
+    int rem = 0, lo = 0, left = 0;
+    bool masks = false;
+    auto take_block = [&]() {
         const unsigned begin = min(section.x, (unsigned)stored), end = min(begin + (section.y >> kWindowColBits), (unsigned)stored);
         // twice the column in front of the row's next unit, less 14 per lane below in the group (see spmv.cu)
-        unsigned run = lane_const + 2u * (section.y & ((1u << kWindowColBits) - 1u)) - 2u * (begin & (unsigned)(kGroup - 1));
-        unsigned pos = (begin & ~(unsigned)(kGroup - 1)) + (unsigned)(kGroup * lig);
-        int rem = (int)(end - pos);
-        int left = (int)__reduce_max_sync(0xffffffffu, end - (begin & ~(unsigned)(kGroup - 1)));
-        const bool masks = __any_sync(0xffffffffu, ((begin | end) & (unsigned)(kGroup - 1)) != 0u);   // not in a window inside the rows
-        int lo = (int)(begin - pos);   // elements of the row before in the lane's first unit
-        const unsigned row = block * K + (unsigned)(lane / L);
-        const bool live = block < block_hi;
+        run = lane_const + 2u * (section.y & ((1u << kWindowColBits) - 1u)) - 2u * (begin & (unsigned)(kGroup - 1));
+        pos = (begin & ~(unsigned)(kGroup - 1)) + (unsigned)(kGroup * lig);
+        rem = (int)(end - pos);
+        lo = (int)(begin - pos);   // elements of the row before in the lane's first unit
+        left = (int)__reduce_max_sync(0xffffffffu, end - (begin & ~(unsigned)(kGroup - 1)));
+        masks = __any_sync(0xffffffffu, ((begin | end) & (unsigned)(kGroup - 1)) != 0u);   // not in a window inside the rows
         ++block;
         fetch_section();
+    };
+    uint4 v[D];
+    unsigned w[D];
+    auto load_unit = [&](int s, int step) {
+        v[s] = make_uint4(0u, 0u, 0u, 0u);
+        w[s] = 0u;
+        if (step * STEP < rem) {
+            v[s] = ldg_stream_v4(values + (pos >> 3) + step * L);
+            w[s] = ldg_stream_u32(deltas + (pos >> 3) + step * L);
+        }
+    };
+    const bool any_rows = block < block_hi;
+    take_block();
+#pragma unroll
+    for (int s = 0; s < D; ++s) load_unit(s, s);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    stage_x();
+    if (!any_rows) return;
+    for (;;) {
         float acc[BV];
 #pragma unroll
         for (int b = 0; b < BV; ++b) acc[b] = 0.f;
         do {
-            uint4 v[D];
-            unsigned w[D];
-            const uint4 *vp = values + (pos >> 3);
-            const unsigned *dp = deltas + (pos >> 3);
-#pragma unroll
-            for (int s = 0; s < D; ++s) {
-                v[s] = make_uint4(0u, 0u, 0u, 0u);
-                w[s] = 0u;
-                if (s * STEP < rem) {
-                    v[s] = ldg_stream_v4(vp + s * L);
-                    w[s] = ldg_stream_u32(dp + s * L);
-                }
-            }
-            if (!staged) {
-                staged = true;
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                stage_x();
-            }
             // byte-wise prefix sums of the deltas and one scan over the group for two sub-steps, as in spmv.cu
             unsigned ce[D], co[D];
 #pragma unroll
@@ -252,6 +256,7 @@ windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ de
                 element_pair(Int<1>{});
                 element_pair(Int<2>{});
                 element_pair(Int<3>{});
+                load_unit(s, s + D);   // the unit D sub-steps on takes its place
             }
             lo = 0;
             run += (unsigned)(2 * L * D);
@@ -259,8 +264,15 @@ windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ de
             rem -= D * STEP;
             left -= D * STEP;
         } while (left > 0);
+        const unsigned row = (block - 1u) * K + (unsigned)(lane / L);
+        const bool more = block < block_hi;
+        if (more) {   // the first units of the next block are on their way while this one is added up
+            take_block();
+#pragma unroll
+            for (int s = 0; s < D; ++s) load_unit(s, s);
+        }
         const float total = group_sums<BV>(acc, lane);
-        if (live && row < (unsigned)rows && lig < BV) {
+        if (row < (unsigned)rows && lig < BV) {
             if (windows > 1) {
                 partial[((size_t)(grp * windows + win) * rows + row) * BV + lig] = total;
             } else if (grp * BV + lig < batch) {
@@ -270,7 +282,8 @@ windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ de
                 *out = __float2half_rn(r);
             }
         }
-    } while (block < block_hi);
+        if (!more) break;
+    }
 }
 
 // y = fp16(alpha * (sum over the windows, in their order) + beta * y). A CTA takes 256 / BV rows of a group of BV vectors: the
