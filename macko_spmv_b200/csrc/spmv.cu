@@ -915,11 +915,16 @@ Shape choose_shape(long long rows, long long cols, long long padded, int residen
 // 22016x4096 (1.16 rounds) d = 0.5 26.3 / 29.3, d = 0.9 38.6 / 44.4, d = 0.1 11.5 / 11.5, 21000x9000 d = 0.4 (1.11) 44.1 / 50.0, 42000x4096
 // d = 0.3 (2.22) 31.6 / 33.2; walked with 16 lanes, 10000x8192 d = 0.5 (1.06) 28.2 / 30.6, 12288x11008 (1.30) 38.0 / 40.6. A kernel of its own: with the
 // second walk in the code, launches that do not need it took up to 3 % longer.
-int choose_tail(int64_t rows, int block, int64_t warps)
+// A row of the tail costs its warp about as much again as 1150 elements of it (set-up, a last iteration mostly empty), so rows have to
+// be long enough for the one or two that a warp gets: 24000x3000 d = 0.4 int8 (1184 a row, two rows) 19.1 / 21.7, 42000x1500 d = 0.9 int8
+// (1331, one) 27.2 / 28.7, but 43502x1771 d = 0.6 (1062, two) 27.4 / 26.5, 42000x900 d = 0.6 (539, one) 16.3 / 16.1, 22000x1000 d = 0.25 (252,
+// one) 7.7 / 6.9.
+int choose_tail(int64_t rows, int block, int64_t warps, int64_t avg_row)
 {
     const int64_t blocks = (rows + block - 1) / block, rounds = blocks / warps, left = blocks - rounds * warps;
     if (rounds == 0 || left == 0 || 2 * left > warps) return 0;
-    return (int)(rows - rounds * warps * block);
+    const int64_t tail = rows - rounds * warps * block, per_warp = (tail + warps - 1) / warps;
+    return avg_row >= (block == 4 ? 575 : 1150) * per_warp ? (int)tail : 0;
 }
 
 // The default launch of one vector with x in shared memory and rows long enough for six units in flight. Against choose_shape, the
@@ -937,7 +942,8 @@ int choose_tail(int64_t rows, int block, int64_t warps)
 //           through it; from 57408 columns on only one CTA of 512 threads fits at all. Fewer lanes per row touch more lines at a time
 //           and need the room earlier: 8 lanes, 1024 / 512 threads: 11623x14035 63.1 / 67.0, 12623x8247 38.0 / 37.5; 16 lanes: 8192x24576 55.4 /
 //           55.7, 6681x46940 53.9 / 58.5, 8234x14855 39.6 / 39.4; a warp per row: 3000x40000 37.8 / 40.1, 4096x28672 35.5 / 35.5, 4096x11008 16.1 /
-//           15.2. Few long rows, less than half a row per warp, take it as well: 1143x29165 18.9 / 21.4, 1286x5290 7.9 / 9.0.
+//           15.2. Few long rows, a fifth to half a row per warp, take it as well: 1143x29165 18.9 / 21.4, 1286x5290 7.9 / 9.0 (but
+//           572x7730 9.1 / 8.7).
 //   roll    loads that stay in flight while a row is walked: from five iterations a row on with 8 lanes, 32000x4096 d = 0.5 35.1 / 36.3, 12288x4096
 //           15.9 / 16.4, d = 0.9 51.7 / 52.3, and with a warp per row where fewer than half of the warps have one and the matrix may
 //           change (no loads in front of the wait): 838x15588 d = 0.74 14.4 / 16.9, 520x11301 d = 0.37 6.7 / 7.6. Elsewhere the extra
@@ -955,8 +961,8 @@ Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, b
     const int64_t from = immutable ? warps + 1 : (55 * 2 * warps + 99) / 100;
     const int L = rows < from ? 32 : rows < 2 * from || cols >= 38000 ? 16 : 8;
     if (avg_row <= 3LL * L * kGroup) return {0, kThreads, 0, false};
-    const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384 : cols > 33088 || (2 * rows <= warps && avg_row >= 4600);
-    return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps),
+    const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384 : cols > 33088 || (2 * rows <= warps && 5 * rows >= warps && avg_row >= 4600);
+    return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps, avg_row),
             immutable ? L == 8 && avg_row >= 1900 : L == 32 && 2 * rows <= warps && avg_row >= 3600};
 }
 

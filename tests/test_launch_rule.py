@@ -19,7 +19,7 @@ DEV = "cuda:0"
     (5209, 3000, 0.3), (5210, 3000, 0.3), (10419, 2000, 0.3), (10420, 2000, 0.3),        # the same for a matrix that may change
     (4800, 16383, 0.03), (4800, 16384, 0.03), (9473, 9999, 0.03), (9473, 10000, 0.03),   # 1024 threads with 16 and 8 lanes
     (9473, 37999, 0.02), (2368, 6000, 0.85), (2369, 6000, 0.85), (2368, 6000, 0.7),      # few long rows
-    (4736, 1000, 0.75), (4737, 1000, 0.37), (9473, 600, 0.3), (9473, 600, 0.35),         # around three sub-steps a row
+    (947, 6000, 0.85), (948, 6000, 0.85), (4736, 1000, 0.75), (4737, 1000, 0.37), (9473, 600, 0.3), (9473, 600, 0.35),         # around three sub-steps a row
 ])
 def test_product_against_float64(rows, cols, d):
     M = workloads.bernoulli_matrix(rows, cols, d, seed=rows + cols, device=DEV)

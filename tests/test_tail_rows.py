@@ -16,9 +16,11 @@ DEV = "cuda:0"
 OPS = torch.ops.macko_spmv
 
 
-# 8 lanes: blocks of four rows, 4736 of them a round; 16 lanes: of two, from 38000 columns on
-@pytest.mark.parametrize("rows,cols,d", [(18944, 500, 0.5), (18945, 500, 0.5), (18951, 500, 0.5), (28416, 500, 0.5), (28417, 500, 0.5), (37889, 407, 0.6),
-                                         (18947, 10000, 0.03), (9473, 38000, 0.02), (14208, 38000, 0.02)])
+# 8 lanes: blocks of four rows, 4736 of them a round, rows of 575 elements for a tail of one row per warp, 1150 for two; 16 lanes: of
+# two, from 38000 columns on, 1150 elements
+@pytest.mark.parametrize("rows,cols,d", [(18944, 900, 0.7), (18945, 900, 0.7), (18951, 900, 0.7), (18951, 900, 0.5), (23681, 1700, 0.7), (28416, 1700, 0.7), (28417, 1700, 0.7),
+                                         (37889, 900, 0.7),
+                                         (18947, 10000, 0.06), (9473, 38000, 0.03), (14208, 38000, 0.03)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.int8])
 def test_product_against_float64(rows, cols, d, dtype):
     if rows * cols > 100 << 20 and dtype is not torch.float16:
