@@ -36,7 +36,9 @@ constexpr int kWin = 1024;       // fp16 slots of a warp's window of the dense r
 // is twice the column of element 2j / 2j+1 relative to the unit's base, and the top byte of `co` plus 2 is twice the
 // columns the unit advances), the units' bases from a warp scan. A step that reaches beyond the window stays in
 // registers: what lies inside is stored, the window leaves, and the rest goes to the next one. Pads and everything
-// else that is +-0 stay +0. The loads of the next step are issued before a step is scattered.
+// else that is +-0 stay +0. The loads of the next step are issued before a step is scattered, and the second-level cache is asked for
+// the stream four steps ahead: with one step of loads alone a warp waits for memory in every step (4096x11008 at density 0.5 33.1 us
+// without). More loads in flight take registers that the fifth CTA needs.
 // Bound by the load/store pipe (a 2-byte shared store of 32 elements takes 3.8 passes: random columns, random banks) and
 // close behind it HBM: 11003x4093 at density 0.2 (113 MB) in 21.5 us = 5.2 TB/s, 4096x11008 at 0.5 (146 MB) in 29.3 us
 // = 5.0 TB/s; a CTA per row takes 32.8 and 31.8 us. With the window flushed and cleared by the same 16-byte loads and
@@ -102,14 +104,26 @@ decompress_rows_kernel(const uint4 *__restrict__ values, const unsigned *__restr
             w = __ldcs(deltas + (first >> 3));
         }
     };
+    // Asks the second-level cache for `steps` steps of 256 stored elements from `from` on: lanes [0, 4 * steps) the lines of the values,
+    // the next `steps` those of the deltas.
+    auto prefetch = [&](unsigned from, unsigned steps) {
+        const unsigned l = (unsigned)lane;
+        const bool value_line = l < 4u * steps;
+        const unsigned e = from + (value_line ? 64u * l : 256u * (l - 4u * steps));
+        if (l < 5u * steps && e < end)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(value_line ? reinterpret_cast<const char *>(values) + 2 * (size_t)e : reinterpret_cast<const char *>(deltas) + (e >> 1)));
+    };
     unsigned first = (begin & ~7u) + (unsigned)(lane * 8);   // first element of the lane's unit
     uint4 v;
     unsigned w;
     fetch(first, v, w);
+    const bool far = end > begin + 768u;   // shorter rows are over before it helps: 16000x1001 d = 0.7 15.0 us with it, 14.6 without
+    if (far) prefetch((begin & ~7u) + 256u, 3u);
     for (unsigned pos = begin & ~7u; pos < end && start < hi; pos += 256u, first += 256u) {
         uint4 v_next;
         unsigned w_next;
         fetch(first + 256u, v_next, w_next);
+        if (far) prefetch(pos + 1024u, 1u);
         if (first < begin || (first < end && first + 8u > end)) keep_elements(v, w, (int)(begin - first), (int)(end - first));
         const unsigned ev = w & 0x0f0f0f0fu, od = (w >> 4) & 0x0f0f0f0fu;
         const unsigned pe = ev * 0x02020202u + 0x0c080400u, po = od * 0x02020202u;
