@@ -230,7 +230,7 @@ struct Extra {
 //       the loads of a long row stay in flight while it is walked (for the line see choose_launch)
 // TAIL  the last `tail_rows` rows are walked with a warp per row (see choose_tail)
 // T     threads of a CTA: 512, two CTAs on an SM, or 1024, one CTA and one copy of x (see choose_launch)
-template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads, bool TAIL = false, bool ROLL = PLAN>
+template <int L, int NPAIR, bool XS, bool PEER, int BV = 1, bool PLAN = false, int VT = kF16, bool EARLY = false, int T = kThreads, bool TAIL = false, bool ROLL = false>
 __global__ void __launch_bounds__(T, kThreadsPerSm / T)
 spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ deltas,
             const int *__restrict__ ri, const __half *__restrict__ x, __half *__restrict__ y,
@@ -783,7 +783,7 @@ int launch_variant(const void *values, const void *deltas, const int32_t *ri, in
                    const DeviceInfo &dev, int ctas_per_sm, const Peers &peers, int batch, const Extra &extra);
 
 // The instantiation with or without early matrix loads, by the immutable-matrix flag of the call.
-template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads, bool TAIL = false, bool ROLL = PLAN>
+template <int L, int NPAIR, bool XS, bool PEER = false, int BV = 1, bool PLAN = false, int VT = kF16, int T = kThreads, bool TAIL = false, bool ROLL = false>
 int launch(const void *values, const void *deltas, const int32_t *ri, int rows, int cols, long long padded,
            const void *x, void *y, float alpha, float beta, cudaStream_t stream,
            const DeviceInfo &dev, int ctas_per_sm, const Peers &peers = Peers{}, int batch = 1, const Extra &extra = Extra{})
@@ -947,7 +947,7 @@ int choose_tail(int64_t rows, int block, int64_t warps, int64_t avg_row)
 //   roll    loads that stay in flight while a row is walked: from five iterations a row on with 8 lanes, 32000x4096 d = 0.5 35.1 / 36.3, 12288x4096
 //           15.9 / 16.4, d = 0.9 51.7 / 52.3, and with a warp per row where fewer than half of the warps have one and the matrix may
 //           change (no loads in front of the wait): 838x15588 d = 0.74 14.4 / 16.9, 520x11301 d = 0.37 6.7 / 7.6. Elsewhere the extra
-//           instructions cost up to 8 % (4096x4096 plain 8.9 / 8.2, int8 11008x4096 14.7 / 14.2). The planned launch rolls as well: 46.5 / 46.9.
+//           instructions cost up to 8 % (4096x4096 plain 8.9 / 8.2, int8 11008x4096 14.7 / 14.2). For the planned launch see macko_spmv_fp16_planned.
 struct Launch {
     int L;          // 0: none, the rows are too short
     int threads;
@@ -1140,8 +1140,14 @@ int macko_spmv_fp16_planned(const void *values, const void *deltas, const int32_
     if (info->split_rows < 0 || info->split_rows > rows)
         return fail(MACKO_ERR_INVALID_ARGUMENT, "the plan info is inconsistent (%d cut rows of %lld)", info->split_rows, (long long)rows);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    st = launch<8, 3, true, false, 1, true>(values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y,
-                                            alpha, beta, s, *dev, 0, Peers{}, 1, extra);
+    // loads roll through segments of two iterations and more (plans of some size): skewed 9600x5000 14.2 / 15.5 us, 5662x10772 18.3 / 19.2,
+    // 32000x8192 46.4 / 47.1; with segments of 512 elements they lose more often than they gain: 3939x9142 15.1 / 14.0, 12968x2442 12.2 /
+    // 11.9, 6000x6000 13.6 / 14.4
+    const bool roll = info->segment_elements > 512;
+    st = roll ? launch<8, 3, true, false, 1, true, kF16, kThreads, false, true>(values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y,
+                                                                               alpha, beta, s, *dev, 0, Peers{}, 1, extra)
+              : launch<8, 3, true, false, 1, true, kF16, kThreads, false, false>(values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y,
+                                                                                alpha, beta, s, *dev, 0, Peers{}, 1, extra);
     if (st != MACKO_OK || info->split_rows == 0) return st;
     // the segments of the cut rows are added up by a second, tiny kernel that starts when the first has finished
     cudaLaunchConfig_t cfg = {};
