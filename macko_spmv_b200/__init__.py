@@ -365,7 +365,7 @@ def multiply_batched(compressed_M, V):
     """
     windowed = type(compressed_M) is FrozenMatrix and compressed_M.windows_batch > 0 and not _is_compiling()
     if windowed:
-        y = _direct_batched(compressed_M, V)   # None: not a plain call of 3..8 vectors
+        y = _direct_batched(compressed_M, V)   # None: not a plain call of three vectors or more
         if y is not None:
             return y
     assert compressed_M[0].is_cuda

@@ -956,11 +956,12 @@ struct Launch {
 };
 Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, bool immutable)
 {
-    const int64_t warps = (int64_t)sm_count * (kThreadsPerSm / 32), avg_row = padded / rows;
+    const int64_t warps = (int64_t)sm_count * (kThreadsPerSm / 32);
     // rows from which on there are blocks enough for 16 lanes; for 8 lanes twice as many
     const int64_t from = immutable ? warps + 1 : (55 * 2 * warps + 99) / 100;
     const int L = rows < from ? 32 : rows < 2 * from || cols >= 38000 ? 16 : 8;
-    if (avg_row <= 3LL * L * kGroup) return {0, kThreads, 0, false};
+    if (padded < (3LL * L * kGroup + 1) * rows) return {0, kThreads, 0, false};
+    const int64_t avg_row = padded / rows;
     const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384 : cols > 33088 || (2 * rows <= warps && 5 * rows >= warps && avg_row >= 4600);
     return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps, avg_row),
             immutable ? L == 8 && avg_row >= 1900 : L == 32 && 2 * rows <= warps && avg_row >= 3600};
@@ -1010,8 +1011,6 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
 
     const size_t smem = (size_t)(kXPadFront + cols + kXPadBack) * sizeof(__half);
     const int ctas = smem * 2 + 2048 <= (size_t)dev->max_smem_optin ? 2 : 1;
-    const Shape shape = choose_shape(rows, cols, padded_count, dev->sm_count * ctas * kWarpsPerCta);
-    const int L = shape.L, D = shape.D;
     const bool xs = smem <= (size_t)dev->max_smem_optin;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Extra extra = {};
@@ -1037,6 +1036,8 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
 #undef MACKO_LAUNCH
 #undef MACKO_LAUNCH_R
     }
+    const Shape shape = choose_shape(rows, cols, padded_count, dev->sm_count * ctas * kWarpsPerCta);
+    const int L = shape.L, D = shape.D;
     if (xs)
         return launch_l<true, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);
     return launch_l<false, VT>(L, D, values, deltas, row_indices, (int)rows, (int)cols, padded_count, x, y, alpha, beta, s, *dev, 0, extra);

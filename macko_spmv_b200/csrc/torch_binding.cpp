@@ -276,12 +276,6 @@ at::Tensor multiply_windowed_cuda(const at::Tensor &values, const at::Tensor &de
     return y;
 }
 
-}  // namespace macko_torch
-
-namespace {
-
-using macko_torch::multiply_windowed_cuda;
-
 at::Tensor decompress_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
                            int64_t rows, int64_t cols)
 {
@@ -295,6 +289,13 @@ at::Tensor decompress_cuda(const at::Tensor &values, const at::Tensor &deltas, c
                  "macko_decompress_fp16");
     return dense;
 }
+
+}  // namespace macko_torch
+
+namespace {
+
+using macko_torch::decompress_cuda;
+using macko_torch::multiply_windowed_cuda;
 
 // Counts the stored elements of M's rows into `ri` and returns their sum, which sizes the outputs. The sum comes through a word of
 // pinned host memory (from PyTorch's pool, given back on return) that the counting kernel writes and this thread watches: the

@@ -20,7 +20,7 @@
 namespace {
 
 PyObject *g_frozen_type = nullptr;   // macko_spmv_b200.FrozenMatrix
-PyObject *g_plan_name = nullptr, *g_plan_meta_name = nullptr, *g_windows_name = nullptr, *g_windows_of_name = nullptr;
+PyObject *g_plan_name = nullptr, *g_plan_meta_name = nullptr, *g_windows_name = nullptr, *g_windows_of_name = nullptr, *g_windows_batch_name = nullptr;
 
 bool nobody_watches()
 {
@@ -113,32 +113,42 @@ bool as_built(PyObject *of, const at::Tensor &deltas, const at::Tensor &ri)
     return true;
 }
 
-// multiply_batched(compressed, V) -> y for 3..8 vectors of a frozen matrix with windows, or None where the call has to take another route
+// multiply_batched(compressed, V) -> y for 3 vectors and more of a frozen matrix with windows: over the windows up to the batch that
+// `freeze` found them faster for, else a dense copy and a GEMM. None where the call has to take another route.
 PyObject *direct_multiply_batched(PyObject *, PyObject *const *args, Py_ssize_t n_args)
 {
     HANDLE_TH_ERRORS
     PyObject *m = n_args == 2 ? args[0] : nullptr;
     if (!m || reinterpret_cast<PyObject *>(Py_TYPE(m)) != g_frozen_type || PyTuple_GET_SIZE(m) < 5) Py_RETURN_NONE;
     const at::Tensor *V = plain_tensor(args[1]);
-    if (!V || V->dim() != 2 || V->size(0) < 3 || V->size(0) > 8 || !V->is_contiguous() || !nobody_watches()) Py_RETURN_NONE;
+    if (!V || V->dim() != 2 || V->size(0) < 3 || !V->is_contiguous() || V->scalar_type() != at::kHalf || V->_fw_grad(0).defined() || !nobody_watches())
+        Py_RETURN_NONE;
     const at::Tensor *values = plain_tensor(PyTuple_GET_ITEM(m, 0)), *deltas = plain_tensor(PyTuple_GET_ITEM(m, 1)),
                      *ri = plain_tensor(PyTuple_GET_ITEM(m, 2));
     int64_t rows, cols;
-    if (!values || !deltas || !ri || !as_int64(PyTuple_GET_ITEM(m, 3), rows) || !as_int64(PyTuple_GET_ITEM(m, 4), cols))
+    if (!values || !deltas || !ri || values->_fw_grad(0).defined() || !as_int64(PyTuple_GET_ITEM(m, 3), rows) ||
+        !as_int64(PyTuple_GET_ITEM(m, 4), cols))
         Py_RETURN_NONE;
     PyObject *w = attribute(m, g_windows_name);
     if (!w) return nullptr;
     const at::Tensor *windows = plain_tensor(w);
     if (!windows) Py_RETURN_NONE;
-    PyObject *of = attribute(m, g_windows_of_name);
-    if (!of) return nullptr;
-    if (!as_built(of, *deltas, *ri)) Py_RETURN_NONE;
+    PyObject *limit = attribute(m, g_windows_batch_name);
+    if (!limit) return nullptr;
+    int64_t windows_batch;
+    if (!as_int64(limit, windows_batch) || V->size(1) != cols) Py_RETURN_NONE;
+    const bool dense = V->size(0) > windows_batch;
+    if (!dense) {
+        PyObject *of = attribute(m, g_windows_of_name);
+        if (!of) return nullptr;
+        if (!as_built(of, *deltas, *ri)) Py_RETURN_NONE;
+    }
     // own handles: another thread may drop the Python ones while the interpreter lock is released
     const at::Tensor v = *values, d = *deltas, r = *ri, x = *V, win = *windows;
     at::Tensor y;
     {
         struct NoGil { PyThreadState *s = PyEval_SaveThread(); ~NoGil() { PyEval_RestoreThread(s); } } no_gil;
-        y = macko_torch::multiply_windowed_cuda(v, d, r, rows, cols, win, x, true);
+        y = dense ? at::matmul(x, macko_torch::decompress_cuda(v, d, r, rows, cols).t()) : macko_torch::multiply_windowed_cuda(v, d, r, rows, cols, win, x, true);
     }
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
@@ -167,5 +177,6 @@ PyMODINIT_FUNC PyInit__torch_direct()
     g_plan_meta_name = PyUnicode_InternFromString("plan_meta");
     g_windows_name = PyUnicode_InternFromString("windows");
     g_windows_of_name = PyUnicode_InternFromString("windows_of");
-    return g_plan_name && g_plan_meta_name && g_windows_name && g_windows_of_name ? PyModule_Create(&g_module) : nullptr;
+    g_windows_batch_name = PyUnicode_InternFromString("windows_batch");
+    return g_plan_name && g_plan_meta_name && g_windows_name && g_windows_of_name && g_windows_batch_name ? PyModule_Create(&g_module) : nullptr;
 }

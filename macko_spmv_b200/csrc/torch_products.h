@@ -20,4 +20,7 @@ at::Tensor multiply_planned_cuda(const at::Tensor &values, const at::Tensor &del
 at::Tensor multiply_windowed_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri, int64_t rows, int64_t cols,
                                   const at::Tensor &windows, const at::Tensor &V, bool frozen);
 
+// Dense [rows, cols] of a compressed matrix.
+at::Tensor decompress_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri, int64_t rows, int64_t cols);
+
 }  // namespace macko_torch

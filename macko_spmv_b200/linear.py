@@ -83,14 +83,13 @@ class MackoLinear(nn.Module):
             raise RuntimeError(f"expected last dimension {self.in_features}, got {tuple(x.shape)}")
         lead = x.shape[:-1]
         flat = x.reshape(-1, self.in_features)
-        comp = self.compressed
         if flat.shape[0] == 1:
             fz = self._frozen
             if fz is not None and fz[0].data_ptr() != self.c_0.data_ptr():
                 fz = self._frozen = None   # the buffers were replaced since freeze(): back to the safe path
-            y = multiply(fz if fz is not None else comp, flat[0].contiguous()).unsqueeze(0)
+            y = multiply(fz if fz is not None else self.compressed, flat[0].contiguous()).unsqueeze(0)
         else:
-            y = multiply_batched(self._frozen_as_is() or comp, flat.contiguous())
+            y = multiply_batched(self._frozen_as_is() or self.compressed, flat.contiguous())
         if self.bias is not None:
             y = y + self.bias
         return y.reshape(*lead, self.out_features)

@@ -184,6 +184,19 @@ def test_route_of_a_frozen_matrix(monkeypatch):
     assert not pay(frozen, V(9, grad=True)) and pay(frozen, V(8, grad=True))
     with torch.autograd.forward_ad.dual_level():
         assert not pay(frozen, V(9))
+    # what the direct calls answer is what the operators give; above the limit the dense copy
+    assert frozen.windows_batch >= 16
+    for b in (3, 8, 9, 16, 65, 80):
+        want = OPS.multiply_windowed.default(*comp[:5], frozen.windows, V(b), True) if b <= frozen.windows_batch else V(b) @ macko_spmv.decompress(comp).t()
+        assert torch.equal(macko_spmv.multiply_batched(frozen, V(b)), want)
+    with pytest.raises(RuntimeError):
+        macko_spmv.multiply_batched(frozen, V(9)[:, :4000].contiguous())
+    with pytest.raises(RuntimeError):
+        macko_spmv.multiply_batched(frozen, V(9).float())
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(V(70), V(71)[:70])
+        tangent = torch.autograd.forward_ad.unpack_dual(macko_spmv.multiply_batched(frozen, dual)).tangent
+        assert tangent is not None and float((tangent.float() - V(71)[:70].float() @ M.float().t()).norm()) < 5e-3 * float(tangent.float().norm())
     # gradients and batching rules of the dense copy are still there
     x = V(17, grad=True)
     macko_spmv.multiply_batched(frozen, x).sum().backward()
