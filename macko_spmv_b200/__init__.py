@@ -184,7 +184,7 @@ class FrozenMatrix(tuple):
     plan = None        # device buffer of the plan, or None
     plan_meta = None   # (virtual_rows, segment_elements, longest_row, split_rows, recommended)
     windows = None      # device buffer of the column windows that `multiply_batched` walks, or None
-    windows_of = None   # write counts and addresses of deltas and row_indices when the windows were built (None: not counted)
+    windows_of = None   # write counts and addresses of deltas, row_indices and values at `freeze` (see `_written`; None: not counted)
     windows_batch = 0   # the largest batch for which the windows are the faster route
 
     def __new__(cls, compressed, plan=None, plan_meta=None, windows=None, windows_of=None, windows_batch=0):
@@ -210,9 +210,16 @@ def freeze(compressed_M, plan="auto", segment_elements=0):
     Waits once for the device work that produced the buffers (they must be complete before a kernel may read
     them ahead of stream order). `plan`: "auto" builds the plan and keeps it only if the row statistics
     recommend it (rows far longer than the average, e.g. skewed matrices), True keeps it always, False builds
-    none. Unless it is False, an fp16 matrix also gets its column windows, which `multiply_batched` walks (8 bytes per row and
-    window of up to 1408 columns, at most 5 % of the matrix). The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
-    (from several streams, order them or freeze once per stream). The reference has no counterpart (src/macko_spmv/__init__.py has only compress / multiply)."""
+    none. The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
+    (from several streams, order them or freeze once per stream).
+
+    Unless `plan` is False, an fp16 matrix also gets its column windows, which `multiply_batched` walks (8 bytes per row and
+    window of up to 1408 columns), if they take at most 5 % of the matrix and PyTorch counts writes to the buffers (not for
+    inference tensors): windows describe the deltas and row offsets that they were built from, and `multiply_batched` leaves them
+    alone once those have been written. Writes that PyTorch does not count (through `.data`, DLPack or a raw pointer) need
+    another `freeze`.
+
+    The reference has no counterpart (src/macko_spmv/__init__.py has only compress / multiply)."""
     assert compressed_M[0].is_cuda and compressed_M[1].is_cuda and compressed_M[2].is_cuda
     torch.cuda.synchronize(compressed_M[0].device)
     if plan is False or compressed_M[0].dtype != torch.float16:
@@ -227,26 +234,29 @@ def freeze(compressed_M, plan="auto", segment_elements=0):
     return FrozenMatrix(compressed_M, None, info, *windows)
 
 
-def _written(deltas, row_indices):
-    """What tells whether the two tensors have been written or moved in place, or None where writes are not counted (inference
-    tensors)."""
-    if deltas.is_inference() or row_indices.is_inference():
+def _written(compressed_M):
+    """What tells whether the buffers have been written or moved since: write counts of deltas and row_indices, their addresses, and
+    both of values. None where PyTorch does not count writes (inference tensors)."""
+    values, deltas, row_indices = compressed_M[:3]
+    if deltas.is_inference() or row_indices.is_inference() or values.is_inference():
         return None
-    return deltas._version, row_indices._version, deltas.data_ptr(), row_indices.data_ptr()
+    return deltas._version, row_indices._version, deltas.data_ptr(), row_indices.data_ptr(), values._version, values.data_ptr()
 
 
 def _build_windows(compressed_M):
     """(column windows of an fp16 matrix, what they were built from, the largest batch that takes them), or (None, None, 0) where
-    the rows are so short that their 8 bytes per row and window would weigh more than 5 % of the matrix."""
+    they cannot index the matrix, where the rows are so short that their 8 bytes per row and window would weigh more than 5 % of the
+    matrix, and where nobody would notice a write to it."""
     _, deltas, row_indices, rows, cols = compressed_M[:5]
     stored = 2 * deltas.numel()
     if rows == 0 or rows >= 1 << 30 or cols >= 1 << 24:
         return None, None, 0
     nbytes = _core.macko_spmm_windows_bytes(rows, cols, stored)
-    if 20 * nbytes > 2.5 * stored:
+    written = _written(compressed_M)
+    if 20 * nbytes > 2.5 * stored or written is None:
         return None, None, 0
     windows = torch.ops.macko_spmv.windows_build.default(deltas, row_indices, rows, cols)
-    return windows, _written(deltas, row_indices), _windows_batch(rows, cols, stored, nbytes // (8 * rows))
+    return windows, written, _windows_batch(rows, cols, stored, nbytes // (8 * rows))
 
 
 # Beyond this many right-hand sides the windowed product has never been ahead of the dense copy.
@@ -347,11 +357,18 @@ def _windows_pay(frozen, V) -> bool:
     batch = V.shape[0]
     if batch < 3 or batch > frozen.windows_batch:
         return False
-    if frozen.windows_of is not None and frozen.windows_of != _written(frozen[1], frozen[2]):
-        return False   # written since: the windows may be those of another matrix
+    if frozen.windows_of is not None:
+        now = _written(frozen)
+        if now is None or frozen.windows_of[:4] != now[:4]:
+            return False   # written since: the windows may be those of another matrix
     # above 8 vectors the other route is a dense copy and operators that can be differentiated and transformed
     return batch <= 8 or not ((V.requires_grad and torch.is_grad_enabled()) or type(V) is not torch.Tensor
                               or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0)
+
+
+def _values_as_frozen(frozen) -> bool:
+    """Whether the windowed product may fetch the values ahead of stream order: nobody has written them since `freeze`."""
+    return frozen.windows_of is None or frozen.windows_of == _written(frozen)
 
 
 def multiply_batched(compressed_M, V):
@@ -375,7 +392,7 @@ def multiply_batched(compressed_M, V):
         raise RuntimeError("V must have shape [batch, cols]")
     batch = V.shape[0]
     if windowed and _windows_pay(compressed_M, V):
-        return torch.ops.macko_spmv.multiply_windowed.default(*compressed_M[:5], compressed_M.windows, V, True)
+        return torch.ops.macko_spmv.multiply_windowed.default(*compressed_M[:5], compressed_M.windows, V, _values_as_frozen(compressed_M))
     if batch > DENSE_BATCH_THRESHOLD or (windowed and batch > compressed_M.windows_batch) or _dense_copy_pays(compressed_M, batch):
         return V @ decompress(compressed_M).t()
     return torch.ops.macko_spmv.multiply_batched.default(*compressed_M[:5], V)

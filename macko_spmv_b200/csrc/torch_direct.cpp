@@ -99,14 +99,15 @@ PyObject *attribute(PyObject *m, PyObject *name)
     return p;
 }
 
-// Whether the tensors that the windows were built from are as they were: `of` = (write count of the deltas, of the row offsets, their
-// addresses), or None where writes are not counted.
-bool as_built(PyObject *of, const at::Tensor &deltas, const at::Tensor &ri)
+// Whether the matrix is as `freeze` found it: `of` = (write count of the deltas, of the row offsets, their addresses, write count and
+// address of the values), or None where the caller has promised that nobody writes it.
+bool as_frozen(PyObject *of, const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri)
 {
     if (of == Py_None) return true;
-    if (!PyTuple_CheckExact(of) || PyTuple_GET_SIZE(of) != 4 || deltas.is_inference() || ri.is_inference()) return false;
-    const int64_t now[4] = {deltas._version(), ri._version(), reinterpret_cast<int64_t>(deltas.data_ptr()), reinterpret_cast<int64_t>(ri.data_ptr())};
-    for (int i = 0; i < 4; ++i) {
+    if (!PyTuple_CheckExact(of) || PyTuple_GET_SIZE(of) != 6 || deltas.is_inference() || ri.is_inference() || values.is_inference()) return false;
+    const int64_t now[6] = {deltas._version(), ri._version(), reinterpret_cast<int64_t>(deltas.data_ptr()), reinterpret_cast<int64_t>(ri.data_ptr()),
+                            values._version(), reinterpret_cast<int64_t>(values.data_ptr())};
+    for (int i = 0; i < 6; ++i) {
         int64_t was;
         if (!as_int64(PyTuple_GET_ITEM(of, i), was) || was != now[i]) return false;
     }
@@ -141,7 +142,7 @@ PyObject *direct_multiply_batched(PyObject *, PyObject *const *args, Py_ssize_t 
     if (!dense) {
         PyObject *of = attribute(m, g_windows_of_name);
         if (!of) return nullptr;
-        if (!as_built(of, *deltas, *ri)) Py_RETURN_NONE;
+        if (!as_frozen(of, *values, *deltas, *ri)) Py_RETURN_NONE;
     }
     // own handles: another thread may drop the Python ones while the interpreter lock is released
     const at::Tensor v = *values, d = *deltas, r = *ri, x = *V, win = *windows;

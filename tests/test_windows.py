@@ -230,10 +230,57 @@ def test_layers_follow_their_buffers():
 
 
 def test_inference_mode():
+    """Nobody counts writes to inference tensors: no windows, so a layer that is reloaded without another freeze() stays right."""
     with torch.inference_mode():
         W = workloads.magnitude_pruned_matrix(640, 2500, 0.5, 7, device=DEV)
         layer = MackoLinear(macko_spmv.compress(W)).freeze()
         x = torch.randn(8, 2500, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).half()
-        assert layer._frozen.windows is not None
+        assert layer._frozen.windows is None
         _check(layer(x), W, x, "inference tensors")
         _check(layer(x.repeat(2, 1)), W, x.repeat(2, 1), "inference tensors, two groups")
+        W2 = W.roll(7, 0).contiguous()   # the same rows in another order: buffers of the same sizes
+        layer.load_state_dict(MackoLinear(macko_spmv.compress(W2)).state_dict())
+        _check(layer(x), W2, x, "reloaded inference tensors")
+
+
+class _WindowedCalls(torch.utils._python_dispatch.TorchDispatchMode):
+    """Records the `frozen` argument of every windowed product."""
+
+    def __init__(self):
+        super().__init__()
+        self.frozen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        if func is OPS.multiply_windowed.default:
+            self.frozen.append(args[7])
+        return func(*args, **(kwargs or {}))
+
+
+def test_values_written_after_freeze():
+    """The windows do not depend on the values: a write to them alone keeps the windows, but no longer lets a product fetch them ahead
+    of stream order."""
+    rows, cols = 900, 3000
+    W = workloads.magnitude_pruned_matrix(rows, cols, 0.4, 31, device=DEV)
+    layer = MackoLinear(macko_spmv.compress(W)).freeze()
+    x = torch.randn(8, cols, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).half()
+    assert macko_spmv._direct_batched(layer._frozen, x) is not None
+    with _WindowedCalls() as calls:
+        layer(x)
+    assert calls.frozen == [True]
+    layer.c_0.mul_(2.0)
+    _check(layer(x), 2 * W, x, "scaled values")
+    assert macko_spmv._direct_batched(layer._frozen, x) is None
+    with _WindowedCalls() as calls:
+        layer(x)
+    assert calls.frozen == [False]
+    # values that the kernel in front is still writing: y of a product that lets its successor start early
+    stored = layer.c_0.numel()
+    A = workloads.bernoulli_matrix(stored, 64, 0.5, seed=5, device=DEV)
+    v = torch.randn(64, generator=torch.Generator(device=DEV).manual_seed(6), device=DEV).half()
+    frozen_A = macko_spmv.freeze(macko_spmv.compress(A), plan=False)
+    torch.autograd.graph.increment_version(layer.c_0)   # the operator's `out` argument is not counted
+    for _ in range(3):
+        layer.c_0.fill_(float("nan"))
+        macko_spmv.multiply(frozen_A, v, out=layer.c_0)
+        y = layer(x)
+        _check(y, macko_spmv.decompress(layer.compressed), x, "values written by the kernel in front")
