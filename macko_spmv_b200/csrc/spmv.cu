@@ -313,7 +313,7 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
             const __half *xb = x + (size_t)b * cols;
 #pragma unroll 4
             for (int c = tid; c < cols; c += T)
-                xs[(size_t)(kXPadFront + c) * BV + b] = b < batch ? xb[c] : __ushort_as_half(0);
+                xs[(size_t)(kXPadFront + c) * BV + b] = __ushort_as_half(b < batch ? ldg_fresh_u16(xb + c) : (unsigned short)0);
         }
         __syncthreads();
     } else if (XS) {
@@ -333,12 +333,12 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
             for (int i = tid; i < n_vec; i += T)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + 16u * (unsigned)i), "l"(src0 + 16 * (size_t)i) : "memory");
 #pragma unroll 1
-            for (int i = (n_vec << 3) + tid; i < cols; i += T) xs[kXPadFront + i] = x[i];
+            for (int i = (n_vec << 3) + tid; i < cols; i += T) xs[kXPadFront + i] = __ushort_as_half(ldg_fresh_u16(x + i));
             asm volatile("cp.async.commit_group;" ::: "memory");
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else {
 #pragma unroll 1
-            for (int i = tid; i < cols; i += T) xs[kXPadFront + i] = x[i];
+            for (int i = tid; i < cols; i += T) xs[kXPadFront + i] = __ushort_as_half(ldg_fresh_u16(x + i));
         }
         __syncthreads();
     }
@@ -609,7 +609,7 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
                             const unsigned short *xg = reinterpret_cast<const unsigned short *>(x);
                             const int cmax = cols - 1;
                             auto gather = [&](int off2) -> unsigned {
-                                return (unsigned)__ldg(xg + min(max((off2 >> 1) - kXPadFront, 0), cmax));
+                                return (unsigned)ldg_fresh_u16(xg + min(max((off2 >> 1) - kXPadFront, 0), cmax));
                             };
                             xe[0] = gather(add_byte<0>(ce[hs], (int)a0));
                             xo[0] = gather(add_byte<0>(co[hs], (int)a0));

@@ -53,6 +53,23 @@ __device__ __forceinline__ unsigned ldg_stream_u32(const unsigned *p)
     return r;
 }
 
+// Loads of what the kernel in front in the stream may have written while this one was already resident (programmatic dependent
+// launch): not the read-only path (ld.global.nc, which __ldg and const __restrict__ pointers become), whose data must not change
+// while a kernel lives, and volatile, so that they stay behind griddepcontrol.wait.
+__device__ __forceinline__ unsigned short ldg_fresh_u16(const void *p)
+{
+    unsigned short r;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(r) : "l"(p));
+    return r;
+}
+
+__device__ __forceinline__ uint2 ldg_fresh_v2(const uint2 *p)
+{
+    uint2 r;
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    return r;
+}
+
 // c + byte `J` of a: one integer dot-product instruction extracts the byte and adds the base, and it
 // does not run on the (half-rate) integer ALU pipe the rest of the index arithmetic competes for.
 template <int J, int M = 1>

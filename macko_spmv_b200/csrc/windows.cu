@@ -148,7 +148,7 @@ windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ de
                 const __half *xc = x + (size_t)grp * BV * cols + col0 + c;
 #pragma unroll
                 for (int b = 0; b < BV; ++b)
-                    if (grp * BV + b < batch) q[b >> 1] |= (unsigned)__half_as_ushort(__ldg(xc + (size_t)b * cols)) << (16 * (b & 1));
+                    if (grp * BV + b < batch) q[b >> 1] |= (unsigned)ldg_fresh_u16(xc + (size_t)b * cols) << (16 * (b & 1));
                 if (BV == 4) { q[2] = q[0]; q[3] = q[1]; }
             }
             const unsigned at = smem0 + (unsigned)(c + kWindowFront) * (unsigned)kWindowColBytes;
@@ -163,7 +163,7 @@ windows_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ de
     auto fetch_section = [&]() {
         const unsigned row = block * K + (unsigned)(lane / L);
         section = make_uint2(0u, 0u);
-        if (block < block_hi && row < (unsigned)rows) section = __ldg(sections + (size_t)win * rows + row);
+        if (block < block_hi && row < (unsigned)rows) section = ldg_fresh_v2(sections + (size_t)win * rows + row);
     };
     fetch_section();
     // byte address of the lane's copy; offsets into x are kept doubled (bytes of fp16), as the prefix sums come, and a column

@@ -165,6 +165,37 @@ def test_graph_and_streams_side_by_side():
         assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("frozen", [True, False])
+def test_x_written_by_the_kernel_in_front_is_seen(frozen):
+    """y of one batched product is x of the next, whose CTAs are already resident while it is written: eager and as one graph.
+
+    Every stage is checked against float64 of what it read, so the bound does not grow along the chain."""
+    n = 2000
+    M = workloads.bernoulli_matrix(n, n, 0.3, seed=77, device=DEV, scale=0.04)
+    comp = macko_spmv.compress(M)
+    windows = OPS.windows_build.default(comp[1], comp[2], n, n)
+    V = torch.randn(8, n, generator=torch.Generator(device=DEV).manual_seed(4), device=DEV).half()
+
+    def chain():
+        out = [V]
+        for _ in range(6):
+            out.append(OPS.multiply_windowed.default(*comp[:5], windows, out[-1], frozen))
+        return out
+
+    eager = chain()
+    for a, b in zip(eager, eager[1:]):
+        _check(b, M, a, "chain")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain()
+    for _ in range(3):
+        for y in out[1:]:
+            y.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(out, eager))
+
+
 def test_route_of_a_frozen_matrix(monkeypatch):
     """Which batches take the windows, and what makes a call take the other routes."""
     M = workloads.magnitude_pruned_matrix(1500, 5000, 0.3, 3, device=DEV)
