@@ -301,15 +301,34 @@ using macko_torch::multiply_windowed_cuda;
 // pinned host memory (from PyTorch's pool, given back on return) that the counting kernel writes and this thread watches: the
 // copy, the synchronisation and the operators of ri[rows].item() left the GPU idle for some 20 us between counting and emitting
 // (11008x4096 d = 0.5: 93.5 us a call, 69.5 of them kernels). The stream is asked now and then, so that a failed kernel ends the wait.
+//
+// The word until the device has written it: given back to the pool only when no kernel can write it any more.
+struct CountWord {
+    c10::DataPtr memory = at::cuda::getCachingHostAllocator()->allocate(sizeof(int32_t));
+    cudaStream_t stream;
+    bool arrived = false;
+
+    explicit CountWord(cudaStream_t s) : stream(s) { *value() = -1; }
+    CountWord(const CountWord &) = delete;
+    ~CountWord()
+    {
+        // an exception on the way: wait for the kernels, or, where not even that works, leave the four bytes to them
+        if (!arrived && cudaStreamSynchronize(stream) != cudaSuccess) {
+            (void)cudaGetLastError();
+            (void)memory.release_context();
+        }
+    }
+    volatile int32_t *value() const { return static_cast<volatile int32_t *>(memory.get()); }
+};
+
 int64_t count_stored(const at::Tensor &M, at::Tensor &ri, cudaStream_t stream)
 {
     const int64_t rows = M.size(0), cols = M.size(1);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     TORCH_CHECK(cudaStreamIsCapturing(stream, &capture) == cudaSuccess, "cudaStreamIsCapturing failed");
     if (capture != cudaStreamCaptureStatusNone) return ri[rows].item<int32_t>();   // refuses, as any read-back in a capture
-    const c10::DataPtr word = at::cuda::getCachingHostAllocator()->allocate(sizeof(int32_t));
-    volatile int32_t *total = static_cast<volatile int32_t *>(word.get());
-    *total = -1;
+    CountWord word(stream);
+    volatile int32_t *total = word.value();
     check_status(macko_compress_count_total(M.data_ptr(), rows, cols, (int32_t)M.element_size(), ri.data_ptr<int32_t>(),
                                             const_cast<int32_t *>(total), stream),
                  M.element_size() == 1 ? "macko_compress_count_int8" : "macko_compress_count");
@@ -323,6 +342,7 @@ int64_t count_stored(const at::Tensor &M, at::Tensor &ri, cudaStream_t stream)
             TORCH_CHECK(*total >= 0, "compress: the stored count did not arrive");
         }
     }
+    word.arrived = true;
     return *total;
 }
 

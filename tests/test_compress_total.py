@@ -1,6 +1,10 @@
 """The stored count that the compressor leaves in pinned host memory (`macko_compress_count_total`), against the last row offset: row
 counts around the 512 that a warp and the 16384 that the CTA of the prefix sum takes at a time, empty matrices, both value
 widths, several threads at once."""
+import os
+import shutil
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -58,3 +62,53 @@ def test_threads_and_streams_at_once():
     for w, g in zip(want, got):
         for c in g:
             assert all(torch.equal(a, b) for a, b in zip(w[:3], c[:3]))
+
+
+# cudaStreamQuery and, on request, cudaStreamSynchronize that answer an error (999) and nothing else, while `fail` says so
+_FAKE = """
+#define _GNU_SOURCE
+#include <dlfcn.h>
+int fail_query, fail_synchronize;
+typedef int (*call)(void *);
+int cudaStreamQuery(void *s) { return fail_query ? 999 : ((call)dlsym(RTLD_NEXT, "cudaStreamQuery"))(s); }
+int cudaStreamSynchronize(void *s) { return fail_synchronize ? 999 : ((call)dlsym(RTLD_NEXT, "cudaStreamSynchronize"))(s); }
+"""
+
+_CHILD = """
+import ctypes, sys
+import torch
+import macko_spmv_b200 as macko_spmv
+from macko_spmv_b200 import workloads
+
+fake = ctypes.CDLL(sys.argv[1])
+M = workloads.bernoulli_matrix(300, 500, 0.4, seed=1, device="cuda")
+want = macko_spmv.compress(M)
+torch.cuda.synchronize()
+torch.cuda._sleep(400_000_000)   # the count is still to come when the query fails
+ctypes.c_int.in_dll(fake, "fail_query").value = 1
+ctypes.c_int.in_dll(fake, "fail_synchronize").value = int(sys.argv[2])
+try:
+    macko_spmv.compress(M)
+    raise SystemExit("compress did not notice the failing query")
+except RuntimeError as e:
+    assert "compress" in str(e), e
+ctypes.c_int.in_dll(fake, "fail_query").value = ctypes.c_int.in_dll(fake, "fail_synchronize").value = 0
+words = [torch.full((1,), 12345, dtype=torch.int32).pin_memory() for _ in range(4)]
+torch.cuda.synchronize()
+assert all(int(w) == 12345 for w in words), [int(w) for w in words]
+assert all(torch.equal(a, b) for a, b in zip(want[:3], macko_spmv.compress(M)[:3]))
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="needs a C compiler")
+@pytest.mark.parametrize("synchronize_fails", [0, 1])
+def test_word_is_not_reused_while_the_count_is_pending(tmp_path, synchronize_fails):
+    """A query that fails ends the call with the count still on its way: the pinned word must not go to somebody else."""
+    (tmp_path / "fake.c").write_text(_FAKE)
+    fake = tmp_path / "fake.so"
+    subprocess.run(["gcc", "-shared", "-fPIC", str(tmp_path / "fake.c"), "-o", str(fake), "-ldl"], check=True)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, LD_PRELOAD=str(fake), PYTHONPATH=root)
+    r = subprocess.run([sys.executable, "-c", _CHILD, str(fake), str(synchronize_fails)], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
