@@ -112,3 +112,31 @@ def test_word_is_not_reused_while_the_count_is_pending(tmp_path, synchronize_fai
     env = dict(os.environ, LD_PRELOAD=str(fake), PYTHONPATH=root)
     r = subprocess.run([sys.executable, "-c", _CHILD, str(fake), str(synchronize_fails)], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+_BLOCKING = """
+import ctypes, time
+import torch
+cudart = ctypes.CDLL("libcudart.so.12")   # torch's
+assert cudart.cudaSetDeviceFlags(4) == 0   # cudaDeviceScheduleBlockingSync
+import macko_spmv_b200 as macko_spmv
+from macko_spmv_b200 import workloads
+
+M = workloads.bernoulli_matrix(300, 500, 0.4, seed=1, device="cuda")
+want = macko_spmv.compress(M)
+torch.cuda.synchronize()
+torch.cuda._sleep(1_000_000_000)   # about half a second
+wall, cpu = time.perf_counter(), time.thread_time()
+got = macko_spmv.compress(M)
+wall, cpu = time.perf_counter() - wall, time.thread_time() - cpu
+assert wall > 0.3 and cpu < 0.2 * wall, (wall, cpu)
+assert all(torch.equal(a, b) for a, b in zip(want[:3], got[:3]))
+"""
+
+
+@pytest.mark.gpu
+def test_blocking_synchronisation_is_respected():
+    """A program that asked CUDA to put its threads to sleep while they wait does not find one of them spinning in compress()."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _BLOCKING], env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
