@@ -256,7 +256,13 @@ def _build_windows(compressed_M):
     if 20 * nbytes > 2.5 * stored or written is None:
         return None, None, 0
     windows = torch.ops.macko_spmv.windows_build.default(deltas, row_indices, rows, cols)
-    return windows, written, _windows_batch(rows, cols, stored, nbytes // (8 * rows))
+    limit = _windows_batch(rows, cols, stored, nbytes // (8 * rows))
+    if limit < DENSE_BATCH_THRESHOLD and not _dense_copy_pays(compressed_M, DENSE_BATCH_THRESHOLD):
+        # 9..16 vectors that take two passes of the one-kernel product where nothing is frozen: the sums stay in fp32 (the GEMM may
+        # add parts in fp16), at about the time of the copy. 16 vectors, windows / copy / passes: 2048x2048 d = 0.7 11.8 / 12.2 / 21.9 us,
+        # d = 0.9 12.8 / 12.3 / 26.8, 2000x5000 d = 0.8 18.4 / 20.8 / 47.2, 4096x1024 d = 0.9 11.1 / 9.8 / 28.0
+        limit = DENSE_BATCH_THRESHOLD
+    return windows, written, limit
 
 
 # Beyond this many right-hand sides the windowed product has never been ahead of the dense copy.

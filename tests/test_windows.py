@@ -242,6 +242,21 @@ def test_route_of_a_frozen_matrix(monkeypatch):
     _check(macko_spmv.multiply_batched(frozen, V(8)), turned, V(8), "written after freeze()")
 
 
+@pytest.mark.parametrize("rows,cols,d", [(2048, 2048, 0.7), (2048, 2048, 0.9), (4096, 1024, 0.9)])
+def test_sums_of_a_frozen_matrix_stay_in_fp32(rows, cols, d):
+    """9..16 vectors of a matrix for which no dense copy pays: compressed passes before `freeze` and after it, never a GEMM whose sums
+    may be fp16."""
+    M = workloads.magnitude_pruned_matrix(rows, cols, d, 3, device=DEV)
+    comp = macko_spmv.compress(M)
+    frozen = macko_spmv.freeze(comp)
+    assert not macko_spmv._dense_copy_pays(comp, 9) and not macko_spmv._dense_copy_pays(comp, 16)
+    for batch in (9, 16):
+        V = torch.randn(batch, cols, generator=torch.Generator(device=DEV).manual_seed(batch), device=DEV).half()
+        Y = macko_spmv.multiply_batched(frozen, V)
+        assert torch.equal(Y, OPS.multiply_windowed.default(*comp[:5], frozen.windows, V, True))
+        _check(Y, M, V, f"batch {batch}")
+
+
 def test_layers_follow_their_buffers():
     """MackoLinear batches over the windows while they are those of its buffers; copies and reloaded layers stay right."""
     W = workloads.magnitude_pruned_matrix(900, 3000, 0.4, 31, device=DEV)
