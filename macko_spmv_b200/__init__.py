@@ -204,7 +204,7 @@ _direct_batched = _direct.multiply_batched if _direct is not None else lambda co
 _is_compiling = torch.compiler.is_compiling
 
 
-def freeze(compressed_M, plan="auto", segment_elements=0):
+def freeze(compressed_M, plan="auto", segment_elements=0, windows="auto"):
     """Declare a compressed CUDA matrix immutable and, if it pays, build its launch plan.
 
     Waits once for the device work that produced the buffers (they must be complete before a kernel may read
@@ -213,25 +213,28 @@ def freeze(compressed_M, plan="auto", segment_elements=0):
     none. The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
     (from several streams, order them or freeze once per stream).
 
-    Unless `plan` is False, an fp16 matrix also gets its column windows, which `multiply_batched` walks (8 bytes per row and
-    window of up to 1408 columns), if they take at most 5 % of the matrix and PyTorch counts writes to the buffers (not for
+    `windows`: "auto" gives an fp16 matrix its column windows, which `multiply_batched` walks (8 bytes per row and window of up to
+    1408 columns), if they take at most 5 % of the matrix, `plan` is not False, and PyTorch counts writes to the buffers (not for
     inference tensors): windows describe the deltas and row offsets that they were built from, and `multiply_batched` leaves them
     alone once those have been written. Writes that PyTorch does not count (through `.data`, DLPack or a raw pointer) need
-    another `freeze`.
+    another `freeze`. False builds none, for a matrix that only ever meets single vectors. True builds them for every fp16 matrix
+    that they can index, also where writes are not counted (the caller promises that there are none).
 
     The reference has no counterpart (src/macko_spmv/__init__.py has only compress / multiply)."""
     assert compressed_M[0].is_cuda and compressed_M[1].is_cuda and compressed_M[2].is_cuda
     torch.cuda.synchronize(compressed_M[0].device)
-    if plan is False or compressed_M[0].dtype != torch.float16:
-        return FrozenMatrix(compressed_M)
-    windows = _build_windows(compressed_M)   # before the plan, which waits for the device
+    half = compressed_M[0].dtype == torch.float16
+    wanted = half and (windows is True or (windows == "auto" and plan is not False))
+    built = _build_windows(compressed_M, windows is True) if wanted else (None, None, 0)   # before the plan, which waits for the device
+    if plan is False or not half:
+        return FrozenMatrix(compressed_M, None, None, *built)
     buf, meta = torch.ops.macko_spmv.plan_build.default(
         compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], compressed_M[0].numel(), int(segment_elements))
     meta = [int(v) for v in meta.tolist()]
     info = (meta[3], meta[4], meta[5], meta[6], meta[7])
     if plan is True or info[4]:
-        return FrozenMatrix(compressed_M, buf, info, *windows)
-    return FrozenMatrix(compressed_M, None, info, *windows)
+        return FrozenMatrix(compressed_M, buf, info, *built)
+    return FrozenMatrix(compressed_M, None, info, *built)
 
 
 def _written(compressed_M):
@@ -243,17 +246,17 @@ def _written(compressed_M):
     return deltas._version, row_indices._version, deltas.data_ptr(), row_indices.data_ptr(), values._version, values.data_ptr()
 
 
-def _build_windows(compressed_M):
+def _build_windows(compressed_M, always):
     """(column windows of an fp16 matrix, what they were built from, the largest batch that takes them), or (None, None, 0) where
-    they cannot index the matrix, where the rows are so short that their 8 bytes per row and window would weigh more than 5 % of the
-    matrix, and where nobody would notice a write to it."""
+    they cannot index the matrix. Unless `always`, also where the rows are so short that their 8 bytes per row and window would
+    weigh more than 5 % of the matrix, and where nobody would notice a write to it."""
     _, deltas, row_indices, rows, cols = compressed_M[:5]
     stored = 2 * deltas.numel()
     if rows == 0 or rows >= 1 << 30 or cols >= 1 << 24:
         return None, None, 0
     nbytes = _core.macko_spmm_windows_bytes(rows, cols, stored)
     written = _written(compressed_M)
-    if 20 * nbytes > 2.5 * stored or written is None:
+    if not always and (20 * nbytes > 2.5 * stored or written is None):
         return None, None, 0
     windows = torch.ops.macko_spmv.windows_build.default(deltas, row_indices, rows, cols)
     limit = _windows_batch(rows, cols, stored, nbytes // (8 * rows))

@@ -33,15 +33,15 @@ class MackoLinear(nn.Module):
         self.bias = nn.Parameter(bias, requires_grad=False) if bias is not None else None
         self._frozen = None   # FrozenMatrix after freeze(): immutable weights, optional launch plan
 
-    def freeze(self, plan="auto") -> "MackoLinear":
+    def freeze(self, plan="auto", windows="auto") -> "MackoLinear":
         """Declare the weight buffers final (call after loading / moving the module, before serving): products may
         then read them ahead of stream order, matrices with very uneven rows get a launch plan, and batches go over
-        column windows (see `macko_spmv_b200.freeze`). Writing c_0 / c_1 / c_2 afterwards
+        column windows (see `macko_spmv_b200.freeze` for both arguments). Writing c_0 / c_1 / c_2 afterwards
         (load_state_dict, .to(...)) requires another freeze(): until then the single-vector product still reads ahead,
         and batches leave windows alone that PyTorch has counted a write for."""
         from . import freeze
 
-        self._frozen = freeze(self.compressed, plan=plan)
+        self._frozen = freeze(self.compressed, plan=plan, windows=windows)
         return self
 
     @classmethod

@@ -289,6 +289,31 @@ def test_inference_mode():
         _check(layer(x), W2, x, "reloaded inference tensors")
 
 
+def test_windows_argument():
+    """False: no windows, the plan as ever; True: also with plan=False, for inference tensors and where they are heavy."""
+    M = workloads.magnitude_pruned_matrix(640, 2500, 0.5, 7, device=DEV)
+    comp = macko_spmv.compress(M)
+    V = torch.randn(8, 2500, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).half()
+    none = macko_spmv.freeze(comp, windows=False)
+    assert none.windows is None and none.plan_meta == macko_spmv.freeze(comp).plan_meta
+    assert torch.equal(macko_spmv.multiply_batched(none, V), macko_spmv.multiply_batched(comp, V))
+    assert MackoLinear(comp).freeze(windows=False)._frozen.windows is None
+    want = macko_spmv.multiply_batched(macko_spmv.freeze(comp), V)
+    for frozen in (macko_spmv.freeze(comp, windows=True), macko_spmv.freeze(comp, plan=False, windows=True)):
+        assert torch.equal(macko_spmv.multiply_batched(frozen, V), want)
+    with torch.inference_mode():
+        frozen = macko_spmv.freeze(macko_spmv.compress(M), windows=True)
+        assert frozen.windows is not None and frozen.windows_of is None
+        assert torch.equal(macko_spmv.multiply_batched(frozen, V.clone()), want)
+    sparse = torch.zeros(2000, 5000, dtype=torch.float16, device=DEV)
+    sparse[::7, 3] = 1.0
+    frozen = macko_spmv.freeze(macko_spmv.compress(sparse), windows=True)
+    V = V.repeat(1, 2)
+    assert frozen.windows is not None
+    _check(macko_spmv.multiply_batched(frozen, V), sparse, V, "heavy windows")
+    assert macko_spmv.freeze(macko_spmv.compress(M.bfloat16()), windows=True).windows is None
+
+
 class _WindowedCalls(torch.utils._python_dispatch.TorchDispatchMode):
     """Records the `frozen` argument of every windowed product."""
 
