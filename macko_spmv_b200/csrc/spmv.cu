@@ -913,8 +913,9 @@ Shape choose_shape(long long rows, long long cols, long long padded, int residen
 // pipe of the SM well enough that nothing is gained (28000x3000 d = 0.5, 1.48 rounds: 24.2 / 24.0), and a matrix of less than one round
 // would only lose the compact groups' fewer bank conflicts. With / without (B200, graph of products, immutable, us):
 // 22016x4096 (1.16 rounds) d = 0.5 26.3 / 29.3, d = 0.9 38.6 / 44.4, d = 0.1 11.5 / 11.5, 21000x9000 d = 0.4 (1.11) 44.1 / 50.0, 42000x4096
-// d = 0.3 (2.22) 31.6 / 33.2; walked with 16 lanes, 10000x8192 d = 0.5 (1.06) 28.2 / 30.6, 12288x11008 (1.30) 38.0 / 40.6. A kernel of its own: with the
-// second walk in the code, launches that do not need it took up to 3 % longer.
+// d = 0.3 (2.22) 31.6 / 33.2; walked with 16 lanes (nothing declared), 10000x8192 d = 0.5 (1.06) 30.4 / 33.8, 9800x5000 (1.03) 20.7 / 22.1, 10400x6000
+// (1.10) 24.3 / 27.2; rows of very uneven length 40.5 / 49.0, 26.6 / 31.1, 31.5 / 37.1. A kernel of its own: with the second walk in the code, launches
+// that do not need it took up to 3 % longer.
 // A row of the tail costs its warp about as much again as 1150 elements of it (set-up, a last iteration mostly empty), so rows have to
 // be long enough for the one or two that a warp gets: 24000x3000 d = 0.4 int8 (1184 a row, two rows) 19.1 / 21.7, 42000x1500 d = 0.9 int8
 // (1331, one) 27.2 / 28.7, but 43502x1771 d = 0.6 (1062, two) 27.4 / 26.5, 42000x900 d = 0.6 (539, one) 16.3 / 16.1, 22000x1000 d = 0.25 (252,
@@ -1026,7 +1027,7 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
         switch (best.L * 10 + (best.threads == kThreads ? 0 : 1)) {
             case 80: return MACKO_LAUNCH_T(8, kThreads);
             case 81: return MACKO_LAUNCH_T(8, 2 * kThreads);
-            case 160: return MACKO_LAUNCH(16, kThreads, false);   // up to two rows per warp: one round at most
+            case 160: return MACKO_LAUNCH_T(16, kThreads);
             case 161: return MACKO_LAUNCH_T(16, 2 * kThreads);
             case 320: return MACKO_LAUNCH(32, kThreads, false);
             case 321: return MACKO_LAUNCH(32, 2 * kThreads, false);

@@ -17,10 +17,11 @@ OPS = torch.ops.macko_spmv
 
 
 # 8 lanes: blocks of four rows, 4736 of them a round, rows of 575 elements for a tail of one row per warp, 1150 for two; 16 lanes: of
-# two, from 38000 columns on, 1150 elements
+# two, 1150 elements a row: from 38000 columns on, and up to 10419 rows where nothing is declared (CTAs of 512 threads)
 @pytest.mark.parametrize("rows,cols,d", [(18944, 900, 0.7), (18945, 900, 0.7), (18951, 900, 0.7), (18951, 900, 0.5), (23681, 1700, 0.7), (28416, 1700, 0.7), (28417, 1700, 0.7),
                                          (37889, 900, 0.7),
-                                         (18947, 10000, 0.06), (9473, 38000, 0.03), (14208, 38000, 0.03)])
+                                         (18947, 10000, 0.06), (9473, 38000, 0.03), (14208, 38000, 0.03),
+                                         (9473, 2000, 0.7), (10001, 2000, 0.7), (10419, 2000, 0.7), (10001, 1600, 0.7)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.int8])
 def test_product_against_float64(rows, cols, d, dtype):
     if rows * cols > 100 << 20 and dtype is not torch.float16:
