@@ -187,6 +187,14 @@ def capture_step_graphs(fn, two_halves: bool):
 
 # --------------------------------------------------------------------------- workload
 
+def weight_flags(comp):
+    """Flag bits of a product whose matrix is a weight: compressed at set-up, looked at once, never written again."""
+    import macko_spmv_b200 as macko_spmv
+    from macko_spmv_b200 import cabi
+
+    return cabi.SPMV_MATRIX_IMMUTABLE | (cabi.SPMV_ROWS_EVEN if macko_spmv.rows_are_even(comp) else 0)
+
+
 def build_sweep(device, rank: int, world: int):
     """The 36 compressed matrices of the sweep (this rank's row block of each), their x, and the dense
     block (kept for the checks and, at N == 1, for the cuBLAS comparison)."""
@@ -211,7 +219,7 @@ def build_sweep(device, rank: int, world: int):
             x = workloads.dense_vector(cols, seed + 500, device)
             cases.append({
                 "rows": rows, "cols": cols, "density": d, "comp": comp, "x": x,
-                "lo": lo, "hi": hi, "dense": block,
+                "lo": lo, "hi": hi, "dense": block, "flags": weight_flags(comp),
                 "bytes": workloads.algorithmic_bytes(comp[0].numel(), hi - lo, cols),
                 "dense_bytes": workloads.dense_bytes(hi - lo, cols),
             })
@@ -235,7 +243,7 @@ def per_case_numbers(cases, lib, peak_gbs):
 
         def mk(cc, xx, yy):
             args = (cc[0].data_ptr(), cc[1].data_ptr(), cc[2].data_ptr(), rows_l, c["cols"], cc[0].numel(),
-                    xx.data_ptr(), yy.data_ptr(), 1.0, 0.0, cabi.SPMV_MATRIX_IMMUTABLE, stream)
+                    xx.data_ptr(), yy.data_ptr(), 1.0, 0.0, c["flags"], stream)
             return lambda: cabi.check(lib, lib.macko_spmv_fp16_ex(*args))
 
         reps = max(30, min(300, int(1.5e9 / c["bytes"])))
@@ -291,12 +299,11 @@ def sharded_large_leg(device, rank, world, lib, peer, peak_gbs, reps=40):
                 torch.cuda.synchronize()
                 gemv_us = e0.elapsed_time(e1) * 100.0
             cases.append({"rows": rows, "cols": cols, "density": d, "x": x, "gemv_us": gemv_us, "lo": lo, "hi": hi,
-                          "shard": sharded.RowShard(comp, lo, hi, rows, blocks), "block": block,
+                          "shard": sharded.RowShard(comp, lo, hi, rows, blocks), "block": block, "flags": weight_flags(comp),
                           "frozen": macko_spmv.freeze(comp, plan=True) if world == 1 else None,
                           "y": torch.empty(rows, dtype=torch.float16, device=device) if world == 1 else None,
                           "bytes": workloads.algorithmic_bytes(comp[0].numel(), hi - lo, cols)})
     torch.cuda.empty_cache()
-    flag = cabi.SPMV_MATRIX_IMMUTABLE
 
     def step(planned=False):
         if peer is not None:
@@ -311,7 +318,7 @@ def sharded_large_leg(device, rank, world, lib, peer, peak_gbs, reps=40):
             else:
                 comp = c["shard"].compressed
                 cabi.check(lib, lib.macko_spmv_fp16_ex(comp[0].data_ptr(), comp[1].data_ptr(), comp[2].data_ptr(), comp[3], comp[4],
-                                                       comp[0].numel(), c["x"].data_ptr(), c["y"].data_ptr(), 1.0, 0.0, flag, stream))
+                                                       comp[0].numel(), c["x"].data_ptr(), c["y"].data_ptr(), 1.0, 0.0, c["flags"], stream))
         return [c["y"] for c in cases]
 
     # ---- check every full y (outside any timed region)
@@ -364,7 +371,7 @@ def sharded_large_leg(device, rank, world, lib, peer, peak_gbs, reps=40):
             else:
                 comp = c["shard"].compressed
                 cabi.check(lib, lib.macko_spmv_fp16_ex(comp[0].data_ptr(), comp[1].data_ptr(), comp[2].data_ptr(), comp[3], comp[4],
-                                                       comp[0].numel(), c["x"].data_ptr(), c["y"].data_ptr(), 1.0, 0.0, flag,
+                                                       comp[0].numel(), c["x"].data_ptr(), c["y"].data_ptr(), 1.0, 0.0, c["flags"],
                                                        torch.cuda.current_stream().cuda_stream))
             marks[r][i + 1].record()
         if peer is not None:
@@ -477,7 +484,7 @@ def single_4096_leg(device, lib, peak_gbs):
 
     def plain(c, xx, y):
         args = (c[0].data_ptr(), c[1].data_ptr(), c[2].data_ptr(), 4096, 4096, c[0].numel(), xx.data_ptr(), y.data_ptr(),
-                1.0, 0.0, cabi.SPMV_MATRIX_IMMUTABLE, stream)
+                1.0, 0.0, weight_flags(comp), stream)
         return lambda: cabi.check(lib, lib.macko_spmv_fp16_ex(*args))
 
     us, nbytes, y = time_one_matrix(plain, comp, x)
@@ -552,8 +559,8 @@ def value_types_leg(device, peak_gbs):
         value_bytes = 1 if name == "int8" else 2
         nbytes = (value_bytes + 0.5) * stored + 4 * (rows + 1) + 2 * cols + 2 * rows
         ncopy = max(2, int(300e6 / nbytes) + 1)
-        copies = [macko_spmv.freeze(comp, plan=False)] + [
-            macko_spmv.freeze((comp[0].clone(), comp[1].clone(), comp[2].clone(), rows, cols), plan=False) for _ in range(ncopy - 1)]
+        copies = [macko_spmv.freeze(comp, windows=False)] + [
+            macko_spmv.freeze((comp[0].clone(), comp[1].clone(), comp[2].clone(), rows, cols), windows=False) for _ in range(ncopy - 1)]
         ys = [torch.empty(rows, dtype=x.dtype, device=device) for _ in range(ncopy)]
 
         def step():
@@ -750,7 +757,6 @@ def run_own_arm(args):
                                   overlap_forward=(args.exchange == "peer"))
     ys_local = [torch.empty(c["hi"] - c["lo"], dtype=torch.float16, device=device) for c in cases]
     ys_full = [torch.empty(c["rows"], dtype=torch.float16, device=device) for c in cases] if world > 1 else ys_local
-    flag = cabi.SPMV_MATRIX_IMMUTABLE   # the matrices are weights: compressed at set-up, never written again
 
     def step_device():
         """One step on the device: N == 1 the C ABI product per matrix; N > 1 the product with the exchange fused
@@ -766,7 +772,7 @@ def run_own_arm(args):
             comp = c["comp"]
             cabi.check(lib, lib.macko_spmv_fp16_ex(comp[0].data_ptr(), comp[1].data_ptr(), comp[2].data_ptr(),
                                                    c["hi"] - c["lo"], c["cols"], comp[0].numel(),
-                                                   c["x"].data_ptr(), yl.data_ptr(), 1.0, 0.0, flag, stream))
+                                                   c["x"].data_ptr(), yl.data_ptr(), 1.0, 0.0, c["flags"], stream))
             if world > 1:
                 dist.all_gather_into_tensor(yf, yl)
         return ys_full
@@ -850,7 +856,7 @@ def run_own_arm(args):
     x_dev = torch.empty(x_off[-1], dtype=torch.float16, device=device)
     y_dev = torch.zeros(y_off[-1], dtype=torch.float16, device=device)
     y_host = torch.zeros(max(y_off[-1], step_rows), dtype=torch.float16).pin_memory()
-    frozen = [macko_spmv.freeze(c["comp"], plan=False) for c in cases]
+    frozen = [macko_spmv.freeze(c["comp"], windows=False) for c in cases]
 
     def step_e2e():
         x_dev.copy_(x_host, non_blocking=True)
@@ -1144,7 +1150,7 @@ def run_single_case(args):
     if kind == "plain":
         run = lambda: macko_spmv.multiply(comp, x)
     elif kind == "frozen":
-        fz0 = macko_spmv.freeze(comp, plan=False)
+        fz0 = macko_spmv.freeze(comp, windows=False)
         run = lambda: macko_spmv.multiply(fz0, x)
     elif kind == "planned":
         fz = macko_spmv.freeze(comp, plan=True)

@@ -40,6 +40,10 @@ extern "C" {
 /* macko_spmv_fp16_scatter_ex only: publish this rank's slice and return without waiting for the other
  * ranks; the caller enqueues macko_peer_wait before the full y is read. */
 #define MACKO_SCATTER_DEFERRED_WAIT 2u
+/* macko_spmv_fp16_ex, _bf16 and _int8 only: the caller has looked at row_indices and knows that no row holds more stored elements
+ * than 9/8 of the mean (P / rows) plus 64. The product may then walk a row with fewer lanes, which is faster for such rows (and
+ * slower for others: y is right either way) and adds a row's products in another order. */
+#define MACKO_SPMV_ROWS_EVEN 16u
 
 enum macko_status {
     MACKO_OK = 0,
@@ -79,8 +83,9 @@ int macko_spmv_fp16(const void *values, const void *deltas, const int32_t *row_i
                     const void *x, void *y, float alpha, float beta, void *stream);
 
 /*
- * macko_spmv_fp16 with flag bits (MACKO_SPMV_MATRIX_IMMUTABLE). Same kernel, same result bits; the flag
- * only moves the first matrix loads in front of the wait for the previous kernel of the stream.
+ * macko_spmv_fp16 with flag bits (MACKO_SPMV_MATRIX_IMMUTABLE, MACKO_SPMV_ROWS_EVEN). The first changes no bit of the
+ * result: it only moves matrix loads, the first of them in front of the wait for the previous kernel of the stream. The second
+ * may change the order in which a row is added up in fp32.
  * Replaces the same reference launcher (kernels_torch_launchers.cuh:3-48), which has no such option.
  */
 int macko_spmv_fp16_ex(const void *values, const void *deltas, const int32_t *row_indices,
@@ -130,6 +135,14 @@ int macko_spmv_fp16_tuned(const void *values, const void *deltas, const int32_t 
  */
 int macko_spmv_shape(int64_t rows, int64_t cols, int64_t padded_count, int sm_count,
                      int *lanes_per_row, int *steps_in_flight);
+
+/*
+ * The launch that macko_spmv_fp16, _ex and _bf16 take for a matrix on a GPU with `sm_count` SMs and these flags: lanes per row, threads
+ * of a CTA (512 or 1024), how many rows at the end of the matrix are walked with a warp each, and whether matrix loads roll
+ * (macko_spmv_int8: the same, but they roll with 32 lanes only). Pure host arithmetic, as macko_spmv_shape.
+ */
+int macko_spmv_default_launch(int64_t rows, int64_t cols, int64_t padded_count, int sm_count, uint32_t flags,
+                              int *lanes_per_row, int *threads_per_cta, int *tail_rows, int *rolling);
 
 /*
  * Planned launch, for matrices whose rows are very long or very uneven. A plan is side metadata built once

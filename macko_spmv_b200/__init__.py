@@ -60,6 +60,8 @@ _core.macko_status_string.restype = ctypes.c_char_p
 _core.macko_status_string.argtypes = [ctypes.c_int]
 _core.macko_spmm_windows_bytes.restype = ctypes.c_int64
 _core.macko_spmm_windows_bytes.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int64]
+_core.macko_spmv_default_launch.restype = ctypes.c_int
+_core.macko_spmv_default_launch.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int, ctypes.c_uint32] + [ctypes.c_void_p] * 4
 
 
 def native_library_paths() -> tuple[str, str]:
@@ -109,7 +111,7 @@ def _decompress_fake(M_values, M_deltas, M_row_indices, M_rows, M_cols):
 
 
 @torch.library.register_fake("macko_spmv::multiply_frozen")
-def _multiply_frozen_fake(M_values, M_deltas, M_row_indices, M_rows, M_cols, V):
+def _multiply_frozen_fake(M_values, M_deltas, M_row_indices, M_rows, M_cols, V, even_rows=False):
     return torch.empty((M_rows,), device=M_values.device, dtype=V.dtype)
 
 
@@ -186,14 +188,16 @@ class FrozenMatrix(tuple):
     windows = None      # device buffer of the column windows that `multiply_batched` walks, or None
     windows_of = None   # write counts and addresses of deltas, row_indices and values at `freeze` (see `_written`; None: not counted)
     windows_batch = 0   # the largest batch for which the windows are the faster route
+    even_rows = False   # no row is much longer than the mean (see `rows_are_even`), where the launch asks for it
 
-    def __new__(cls, compressed, plan=None, plan_meta=None, windows=None, windows_of=None, windows_batch=0):
+    def __new__(cls, compressed, plan=None, plan_meta=None, windows=None, windows_of=None, windows_batch=0, even_rows=False):
         self = super().__new__(cls, tuple(compressed[:5]))
         self.plan = plan
         self.plan_meta = plan_meta
         self.windows = windows
         self.windows_of = windows_of
         self.windows_batch = windows_batch
+        self.even_rows = even_rows
         return self
 
 
@@ -210,8 +214,10 @@ def freeze(compressed_M, plan="auto", segment_elements=0, windows="auto"):
     Waits once for the device work that produced the buffers (they must be complete before a kernel may read
     them ahead of stream order). `plan`: "auto" builds the plan and keeps it only if the row statistics
     recommend it (rows far longer than the average, e.g. skewed matrices), True keeps it always, False builds
-    none. The partial sums of cut rows live in the plan: products of one planned matrix must not overlap on the GPU
-    (from several streams, order them or freeze once per stream).
+    none. Unless it is False, products of a matrix of any type whose rows are even (`rows_are_even`) may walk a row with fewer
+    lanes; with False `multiply` adds up every row as it does for the plain 5-tuple, bit for bit. The partial sums of cut rows
+    live in the plan: products of one planned matrix must not overlap on the GPU (from several streams, order them or freeze
+    once per stream).
 
     `windows`: "auto" gives an fp16 matrix its column windows, which `multiply_batched` walks (8 bytes per row and window of up to
     1408 columns), if they take at most 5 % of the matrix, `plan` is not False, and PyTorch counts writes to the buffers (not for
@@ -227,14 +233,42 @@ def freeze(compressed_M, plan="auto", segment_elements=0, windows="auto"):
     wanted = half and (windows is True or (windows == "auto" and plan is not False))
     built = _build_windows(compressed_M, windows is True) if wanted else (None, None, 0)   # before the plan, which waits for the device
     if plan is False or not half:
-        return FrozenMatrix(compressed_M, None, None, *built)
+        even = plan is not False and _lanes_depend_on_rows(compressed_M) and rows_are_even(compressed_M)
+        return FrozenMatrix(compressed_M, None, None, *built, even)
     buf, meta = torch.ops.macko_spmv.plan_build.default(
         compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], compressed_M[0].numel(), int(segment_elements))
     meta = [int(v) for v in meta.tolist()]
     info = (meta[3], meta[4], meta[5], meta[6], meta[7])
+    even = _even(info[2], compressed_M[0].numel(), compressed_M[3])
     if plan is True or info[4]:
-        return FrozenMatrix(compressed_M, buf, info, *built)
-    return FrozenMatrix(compressed_M, None, info, *built)
+        return FrozenMatrix(compressed_M, buf, info, *built, even)
+    return FrozenMatrix(compressed_M, None, info, *built, even)
+
+
+def _even(longest_row: int, stored: int, rows: int) -> bool:
+    """What MACKO_SPMV_ROWS_EVEN promises: no row above 9/8 of the mean and 64 elements more."""
+    return 8 * rows * (longest_row - 64) <= 9 * stored
+
+
+def _lanes_depend_on_rows(compressed_M) -> bool:
+    """Whether the product's launch is another one for rows known to be even (host arithmetic; saves the look at the rows if not)."""
+    launches = []
+    for flags in (1, 17):   # MACKO_SPMV_MATRIX_IMMUTABLE, the same and MACKO_SPMV_ROWS_EVEN
+        out = (ctypes.c_int * 4)()
+        at = ctypes.addressof(out)
+        status = _core.macko_spmv_default_launch(compressed_M[3], compressed_M[4], compressed_M[0].numel(),
+                                                 torch.cuda.get_device_properties(compressed_M[0].device).multi_processor_count,
+                                                 flags, at, at + 4, at + 8, at + 12)
+        launches.append((status, *out))
+    return launches[0] != launches[1]
+
+
+def rows_are_even(compressed_M) -> bool:
+    """Whether no row of a compressed matrix holds many more stored elements than the mean row (reads one number back from the
+    device). `freeze` asks this: products of such a matrix may walk a row with fewer lanes, which would make long rows of another
+    one take longer. The order of the fp32 sums of a row depends on it."""
+    row_indices, rows = compressed_M[2], compressed_M[3]
+    return rows > 0 and _even(int((row_indices[1:] - row_indices[:-1]).amax()), compressed_M[0].numel(), rows)
 
 
 def _written(compressed_M):
@@ -311,10 +345,11 @@ def multiply(compressed_M, V, out=None):
     assert V.is_cuda
     assert V.is_contiguous()
     if out is not None:
-        frozen = isinstance(compressed_M, FrozenMatrix)
+        flags = 0
+        if isinstance(compressed_M, FrozenMatrix):   # MACKO_SPMV_MATRIX_IMMUTABLE, MACKO_SPMV_ROWS_EVEN
+            flags = 17 if compressed_M.even_rows else 1
         torch.ops.macko_spmv.multiply_ex.default(
-            compressed_M[0], compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], V, out, 1.0, 0.0,
-            1 if frozen else 0)
+            compressed_M[0], compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], V, out, 1.0, 0.0, flags)
         return out
     if isinstance(compressed_M, FrozenMatrix):
         if compressed_M.plan is not None:
@@ -322,7 +357,7 @@ def multiply(compressed_M, V, out=None):
                 compressed_M[0], compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4],
                 compressed_M.plan, compressed_M.plan_meta[0], compressed_M.plan_meta[1], compressed_M.plan_meta[3], V, True)
         return torch.ops.macko_spmv.multiply_frozen.default(
-            compressed_M[0], compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], V)
+            compressed_M[0], compressed_M[1], compressed_M[2], compressed_M[3], compressed_M[4], V, compressed_M.even_rows)
     return torch.ops.macko_spmv.multiply.default(
         compressed_M[0],
         compressed_M[1],
@@ -407,5 +442,5 @@ def multiply_batched(compressed_M, V):
     return torch.ops.macko_spmv.multiply_batched.default(*compressed_M[:5], V)
 
 
-__all__ = ["compress", "multiply", "multiply_batched", "decompress", "move_to_device", "freeze", "FrozenMatrix",
+__all__ = ["compress", "multiply", "multiply_batched", "decompress", "move_to_device", "freeze", "rows_are_even", "FrozenMatrix",
            "native_library_paths", "native_version", "LIB_NAME"]

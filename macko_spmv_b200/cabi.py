@@ -29,6 +29,7 @@ _i32 = ctypes.c_int32
 # flag bits (include/macko_b200.h)
 SPMV_MATRIX_IMMUTABLE = 1
 SCATTER_DEFERRED_WAIT = 2
+SPMV_ROWS_EVEN = 16
 
 
 class PlanInfo(ctypes.Structure):
@@ -54,6 +55,7 @@ SIGNATURES = {
     "macko_spmv_fp16_planned": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, ctypes.POINTER(PlanInfo), _vp, _vp, _f, _f, _u32, _vp]),
     "macko_spmv_fp16_tuned": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _f, _f, _vp, _int, _int, _int, _int]),
     "macko_spmv_shape": (_int, [_i64, _i64, _i64, _int, _vp, _vp]),
+    "macko_spmv_default_launch": (_int, [_i64, _i64, _i64, _int, _u32, _vp, _vp, _vp, _vp]),
     "macko_spmm_fp16": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _i64, _f, _f, _vp]),
     "macko_spmm_windows_bytes": (_i64, [_i64, _i64, _i64]),
     "macko_spmm_windows": (_int, [_vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp]),

@@ -204,7 +204,7 @@ __device__ __forceinline__ int block_boundary(int rows, unsigned w, unsigned n_w
 
 // What a launch carries besides the reference's arguments.
 struct Extra {
-    unsigned flags;               // MACKO_SPMV_MATRIX_IMMUTABLE
+    unsigned flags;               // MACKO_SPMV_MATRIX_IMMUTABLE, MACKO_SPMV_ROWS_EVEN
     int tail_rows;                // TAIL kernels only
     PlanView plan;                // planned launch: virtual rows instead of row_indices (PLAN kernels only)
 };
@@ -929,43 +929,60 @@ int choose_tail(int64_t rows, int block, int64_t warps, int64_t avg_row)
 }
 
 // The default launch of one vector with x in shared memory and rows long enough for six units in flight. Against choose_shape, the
-// best shape of two CTAs of 512 threads whose last round may be mostly empty, it has the tail and CTAs of 1024 threads, and the rule is
-// simpler. 143 shapes (1024..49152 rows, 2048..49152 columns, d = 0.1..0.9, six launches each): within 0.3 % of the fastest on
-// average and at most 4 %, 2.1 % ahead of choose_shape on average (B200, graph of products, immutable, us, this / before):
-//   lanes   the fewest with which every warp still gets a block of rows: fewer bank conflicts, a shorter scan. 5139x12557 d = 0.15 10.2 / 12.4,
-//           5120x13824 d = 0.5 23.8 / 27.4, 10176x7155 d = 0.24 14.3 / 16.5, 14437x25305 d = 0.75 133.9 / 153.6, but 4693x9710 (not quite a row per
-//           warp) 7.2 with 32 lanes and 7.6 with 16. From 38000 columns on 16 at least: 12288x49152 d = 0.5 155.2, with eight lanes 162.4.
-//           Rows of very uneven length want more lanes; a matrix declared immutable has usually been looked at (such rows get a
-//           plan), any other takes the lower number only from 1.1 times as many rows on: skewed 9600x5000 21.9 with 16 lanes, 28.7
-//           with 8, 5000x6000 16.9 / 18.3.
-//   threads one CTA of 1024 threads and one copy of x, or two of 512. Two large copies leave the SM's first-level cache little room
-//           (28 KB from 41000 columns on), and the matrix data that 1024 threads keep in flight, 120 KB with six units a lane, passes
-//           through it; from 57408 columns on only one CTA of 512 threads fits at all. Fewer lanes per row touch more lines at a time
+// best shape of two CTAs of 512 threads whose last round may be mostly empty, it has the tail and CTAs of 1024 threads (B200, graph of
+// products, us):
+//   lanes   of rows known to be even (MACKO_SPMV_ROWS_EVEN): the fewest with which every warp still gets a block of rows: fewer bank
+//           conflicts, a shorter scan. 143 shapes (1024..49152 rows, 2048..49152 columns, d = 0.1..0.9, six launches each): within 0.3 % of
+//           the fastest on average and at most 4 %. 5139x12557 d = 0.15 10.2 / 12.4 (choose_shape), 5120x13824 d = 0.5 23.8 / 27.4, 10176x7155
+//           d = 0.24 14.3 / 16.5, 14437x25305 d = 0.75 133.9 / 153.6, but 4693x9710 (not quite a row per warp) 7.2 with 32 lanes and 7.6 with 16.
+//           From 38000 columns on 16 at least: 12288x49152 d = 0.5 155.2, with eight lanes 162.4.
+//           A long row is a serial chain that fewer lanes make longer. Where 2 % of the rows hold f times the others, fewest lanes / choose_shape:
+//           10000x9000 d = 0.5 f = 1.1 31.2 / 32.1, 1.2 33.1 / 33.5, 1.3 34.8 / 33.5; 14000x25000 d = 0.4 83.2 / 81.5, 88.0 / 83.5, 90.9 / 84.4; so "even" is
+//           an eighth above the mean and one sub-step of 64 elements (f = 1.3 on short rows, 9600x2500 d = 0.2: 6.7 / 6.8).
+//           Of any other rows: those of choose_shape, which bounds the chain of the average row. With the fewest lanes rows of very
+//           uneven length (mean density 0.2, 5 % dense) took up to 75 % longer: 9600x20000 103.9 / 59.8, 12000x20000 103.6 / 77.3, 11000x30000 149 / 104.
+//           But no row holds more than `cols` elements: from two thirds of that on average 16 lanes pay as soon as there are blocks
+//           for half the warps, and 8 from a full round on, whatever the rows look like: 11000x12000 d = 0.9 64.3 / 69.4, uneven 64.2 / 68.9, 14437x25305
+//           d = 0.75 141.2 / 158.4, uneven 158.5 / 170.5, 20000x12000 d = 0.8 94.4 / 98.0 (16 lanes) / 105.3, uneven 100.0 / 102.8 / 106.2.
+//   threads one CTA of 1024 threads and one copy of x, or two of 512. Shared memory and first-level cache share 256 KB: two copies of 98 KB
+//           (49000 columns) leave 28 KB of cache for the matrix data that 1024 threads keep in flight, 120 KB with six units a lane, to
+//           pass through, and from 57409 columns on only one CTA of 512 threads fits at all. Fewer lanes per row touch more lines at a time
 //           and need the room earlier: 8 lanes, 1024 / 512 threads: 11623x14035 63.1 / 67.0, 12623x8247 38.0 / 37.5; 16 lanes: 8192x24576 55.4 /
 //           55.7, 6681x46940 53.9 / 58.5, 8234x14855 39.6 / 39.4; a warp per row: 3000x40000 37.8 / 40.1, 4096x28672 35.5 / 35.5, 4096x11008 16.1 /
-//           15.2. Few long rows, a fifth to half a row per warp, take it as well: 1143x29165 18.9 / 21.4, 1286x5290 7.9 / 9.0 (but
+//           15.2; with more than a row per warp earlier if the matrix may change, 6000x20000 d = 0.3 27.8 / 28.7, 14000x25000 d = 0.4 78.7 / 80.4, 12000x20000
+//           uneven 76.1 / 78.4 (immutable and uneven 6000x20000 47.7 / 45.8, 9600x20000 63.2 / 59.9).
+//           Few long rows, a fifth to half a row per warp, take it as well: 1143x29165 18.9 / 21.4, 1286x5290 7.9 / 9.0 (but
 //           572x7730 9.1 / 8.7).
-//   roll    loads that stay in flight while a row is walked: from five iterations a row on with 8 lanes, 32000x4096 d = 0.5 35.1 / 36.3, 12288x4096
-//           15.9 / 16.4, d = 0.9 51.7 / 52.3, and with a warp per row where fewer than half of the warps have one and the matrix may
-//           change (no loads in front of the wait): 838x15588 d = 0.74 14.4 / 16.9, 520x11301 d = 0.37 6.7 / 7.6. Elsewhere the extra
+//   roll    loads that stay in flight while a row is walked: from five iterations an even row on with 8 lanes, 32000x4096 d = 0.5 35.1 / 36.3, 12288x4096
+//           15.9 / 16.4, d = 0.9 51.7 / 52.3 (uneven 12288x4096 d = 0.6 27.7 / 25.2, 2 % of the rows 1.3 times as long 21.7 / 21.5), and with a warp per
+//           row where fewer than half of the warps have one and the matrix may
+//           change (no loads in front of the wait): 838x15588 d = 0.74 14.4 / 16.9, 520x11301 d = 0.37 6.7 / 7.6, uneven 1500x20000 23.5 / 26.5. Elsewhere the extra
 //           instructions cost up to 8 % (4096x4096 plain 8.9 / 8.2, int8 11008x4096 14.7 / 14.2). For the planned launch see macko_spmv_fp16_planned.
+// Lanes and tail decide the order of the fp32 sums: they do not depend on MACKO_SPMV_MATRIX_IMMUTABLE, which promises the same bits.
 struct Launch {
     int L;          // 0: none, the rows are too short
     int threads;
     int tail_rows;
     bool roll;      // built for 8 lanes of 16-bit values of an immutable matrix and for a warp per row of any other
 };
-Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, bool immutable)
+Launch choose_launch(int64_t rows, int64_t cols, int64_t padded, int sm_count, uint32_t flags)
 {
+    const bool immutable = (flags & MACKO_SPMV_MATRIX_IMMUTABLE) != 0, even = (flags & MACKO_SPMV_ROWS_EVEN) != 0;
     const int64_t warps = (int64_t)sm_count * (kThreadsPerSm / 32);
-    // rows from which on there are blocks enough for 16 lanes; for 8 lanes twice as many
-    const int64_t from = immutable ? warps + 1 : (55 * 2 * warps + 99) / 100;
-    const int L = rows < from ? 32 : rows < 2 * from || cols >= 38000 ? 16 : 8;
+    const bool many = 100 * rows >= 110 * warps;   // blocks of two rows for 0.55 of the warps
+    int L;
+    if (even) {
+        L = rows <= warps ? 32 : rows <= 2 * warps + 1 || cols >= 38000 ? 16 : 8;
+    } else {
+        L = choose_shape(rows, cols, padded, (int)warps).L;
+        if (many && 2 * cols * rows <= 3 * padded) L = min(L, rows >= 4 * warps && cols < 38000 ? 8 : 16);
+    }
     if (padded < (3LL * L * kGroup + 1) * rows) return {0, kThreads, 0, false};
     const int64_t avg_row = padded / rows;
-    const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384 : cols > 33088 || (2 * rows <= warps && 5 * rows >= warps && avg_row >= 4600);
+    const bool wide = L == 8 ? cols >= 10000 : L == 16 ? cols >= 16384
+                      : cols > 33088 || (many && !immutable && cols >= 16384) || (2 * rows <= warps && 5 * rows >= warps && avg_row >= 4600);
     return {L, wide ? 2 * kThreads : kThreads, L == 32 ? 0 : choose_tail(rows, 32 / L, warps, avg_row),
-            immutable ? L == 8 && avg_row >= 1900 : L == 32 && 2 * rows <= warps && avg_row >= 3600};
+            L == 8 ? immutable && even && avg_row >= 1900 : L == 32 && !immutable && 2 * rows <= warps && avg_row >= 3600};
 }
 
 // One launch for up to BV vectors. Lanes per row as in the single-vector product; fewer units in flight with
@@ -989,9 +1006,9 @@ int launch_batched(const void *values, const void *deltas, const int32_t *ri, in
                 : launch<8, 1, true, false, BV>(values, deltas, ri, rows, cols, padded, x, y, alpha, beta, stream, dev, 0, Peers{}, batch);
 }
 
-int check_flags(uint32_t flags)
+int check_flags(uint32_t flags, uint32_t known)
 {
-    if (flags & ~(uint32_t)MACKO_SPMV_MATRIX_IMMUTABLE)
+    if (flags & ~known)
         return fail(MACKO_ERR_INVALID_ARGUMENT, "unknown flag bits 0x%x", flags);
     return MACKO_OK;
 }
@@ -1003,7 +1020,7 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
                  const void *x, void *y, float alpha, float beta, uint32_t flags, void *stream)
 {
     int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
-    if (st == MACKO_OK) st = check_flags(flags);
+    if (st == MACKO_OK) st = check_flags(flags, MACKO_SPMV_MATRIX_IMMUTABLE | MACKO_SPMV_ROWS_EVEN);
     if (st != MACKO_OK) return st;
     if (rows == 0) return MACKO_OK;
     const DeviceInfo *dev = nullptr;
@@ -1017,7 +1034,7 @@ int spmv_default(const void *values, const void *deltas, const int32_t *row_indi
     Extra extra = {};
     extra.flags = flags;
     if (xs) {
-        const Launch best = choose_launch(rows, cols, padded_count, dev->sm_count, (flags & MACKO_SPMV_MATRIX_IMMUTABLE) != 0);
+        const Launch best = choose_launch(rows, cols, padded_count, dev->sm_count, flags);
         extra.tail_rows = best.tail_rows;
         const int r = (int)rows, c = (int)cols;
 #define MACKO_LAUNCH_R(LL, T, TAIL, ROLL) \
@@ -1109,7 +1126,7 @@ int macko_spmv_fp16_planned(const void *values, const void *deltas, const int32_
 {
     using namespace macko;
     int st = check_product_args(values, deltas, row_indices, rows, cols, padded_count, x, y);
-    if (st == MACKO_OK) st = check_flags(flags);
+    if (st == MACKO_OK) st = check_flags(flags, MACKO_SPMV_MATRIX_IMMUTABLE);
     if (st != MACKO_OK) return st;
     if (!plan || !info) return fail(MACKO_ERR_INVALID_ARGUMENT, "null plan or plan info");
     if (!aligned(plan, 16)) return fail(MACKO_ERR_MISALIGNED, "plan must be 16-byte aligned");
@@ -1178,6 +1195,28 @@ int macko_spmv_shape(int64_t rows, int64_t cols, int64_t padded_count, int sm_co
     const Shape shape = choose_shape(rows, cols, padded_count, sm_count * ctas * kWarpsPerCta);
     *lanes_per_row = shape.L;
     *steps_in_flight = shape.D;
+    return MACKO_OK;
+}
+
+int macko_spmv_default_launch(int64_t rows, int64_t cols, int64_t padded_count, int sm_count, uint32_t flags,
+                              int *lanes_per_row, int *threads_per_cta, int *tail_rows, int *rolling)
+{
+    using namespace macko;
+    if (rows < 0 || cols < 0 || padded_count < 0 || sm_count <= 0 || sm_count > 65536 || !lanes_per_row || !threads_per_cta || !tail_rows || !rolling)
+        return fail(MACKO_ERR_INVALID_ARGUMENT, "bad argument to macko_spmv_default_launch");
+    if (rows >= (1LL << 31) - 64 || cols >= (1LL << 30) || padded_count >= (1LL << 31))
+        return fail(MACKO_ERR_SIZE_OVERFLOW, "rows=%lld cols=%lld P=%lld exceed 31-bit indexing", (long long)rows, (long long)cols, (long long)padded_count);
+    int st = check_flags(flags, MACKO_SPMV_MATRIX_IMMUTABLE | MACKO_SPMV_ROWS_EVEN);
+    Launch best = {0, kThreads, 0, false};
+    const size_t smem = (size_t)(kXPadFront + cols + kXPadBack) * sizeof(__half);
+    if (st == MACKO_OK && rows > 0 && smem <= (size_t)227 * 1024) best = choose_launch(rows, cols, padded_count, sm_count, flags);
+    int steps = 0;
+    if (st == MACKO_OK && best.L == 0) st = macko_spmv_shape(rows, cols, padded_count, sm_count, &best.L, &steps);
+    if (st != MACKO_OK) return st;
+    *lanes_per_row = best.L;
+    *threads_per_cta = best.threads;
+    *tail_rows = best.tail_rows;
+    *rolling = best.roll ? 1 : 0;
     return MACKO_OK;
 }
 

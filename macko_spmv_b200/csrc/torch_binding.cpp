@@ -92,11 +92,11 @@ at::Tensor multiply_cuda(const at::Tensor &values, const at::Tensor &deltas, con
 }
 
 // The same product for a matrix the caller has declared immutable (weights): the kernel may fetch matrix
-// data before the previous kernel of the stream has finished.
+// data before the previous kernel of the stream has finished. `even_rows`: no row is much longer than the mean.
 at::Tensor multiply_frozen_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
-                                int64_t rows, int64_t cols, const at::Tensor &V)
+                                int64_t rows, int64_t cols, const at::Tensor &V, bool even_rows)
 {
-    return multiply_flags(values, deltas, ri, rows, cols, V, MACKO_SPMV_MATRIX_IMMUTABLE);
+    return multiply_flags(values, deltas, ri, rows, cols, V, MACKO_SPMV_MATRIX_IMMUTABLE | (even_rows ? MACKO_SPMV_ROWS_EVEN : 0u));
 }
 
 // Plan of a compressed matrix: (plan buffer on the device, int64[8] on the host =
@@ -187,7 +187,7 @@ void multiply_out_cuda(const at::Tensor &values, const at::Tensor &deltas, const
                      "macko_spmv_fp16");
 }
 
-// multiply_out with flag bits (MACKO_SPMV_MATRIX_IMMUTABLE): the product into a caller-owned y.
+// multiply_out with flag bits (MACKO_SPMV_MATRIX_IMMUTABLE, MACKO_SPMV_ROWS_EVEN): the product into a caller-owned y.
 void multiply_ex_cuda(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri,
                       int64_t rows, int64_t cols, const at::Tensor &V, at::Tensor y, double alpha, double beta, int64_t flags)
 {
@@ -499,7 +499,8 @@ TORCH_LIBRARY(macko_spmv, m)
     m.def("decompress(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols) -> Tensor");
     m.def("multiply_ex(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor V, "
           "Tensor(a!) y, float alpha, float beta, int flags) -> ()");
-    m.def("multiply_frozen(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor V) -> Tensor");
+    m.def("multiply_frozen(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor V, "
+          "bool even_rows=False) -> Tensor");
     m.def("plan_build(Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, int padded_count, int segment_elements) -> (Tensor, Tensor)");
     m.def("multiply_planned(Tensor M_values, Tensor M_deltas, Tensor M_row_indices, int M_rows, int M_cols, Tensor plan, "
           "int virtual_rows, int segment_elements, int split_rows, Tensor V, bool frozen) -> Tensor");

@@ -20,7 +20,7 @@
 namespace {
 
 PyObject *g_frozen_type = nullptr;   // macko_spmv_b200.FrozenMatrix
-PyObject *g_plan_name = nullptr, *g_plan_meta_name = nullptr, *g_windows_name = nullptr, *g_windows_of_name = nullptr, *g_windows_batch_name = nullptr;
+PyObject *g_even_name = nullptr, *g_plan_name = nullptr, *g_plan_meta_name = nullptr, *g_windows_name = nullptr, *g_windows_of_name = nullptr, *g_windows_batch_name = nullptr;
 
 bool nobody_watches()
 {
@@ -65,6 +65,7 @@ PyObject *direct_multiply(PyObject *, PyObject *const *args, Py_ssize_t n_args)
         Py_RETURN_NONE;
     const at::Tensor *plan = nullptr;
     int64_t virtual_rows = 0, segment = 0, split_rows = 0;
+    uint32_t flags = frozen ? MACKO_SPMV_MATRIX_IMMUTABLE : 0u;
     if (frozen) {
         PyObject *p = PyObject_GetAttr(m, g_plan_name);   // new references; the attributes outlive the call in the matrix
         if (!p) return nullptr;
@@ -77,6 +78,11 @@ PyObject *direct_multiply(PyObject *, PyObject *const *args, Py_ssize_t n_args)
             if (!plan || !PyTuple_CheckExact(meta) || PyTuple_GET_SIZE(meta) < 4 || !as_int64(PyTuple_GET_ITEM(meta, 0), virtual_rows) ||
                 !as_int64(PyTuple_GET_ITEM(meta, 1), segment) || !as_int64(PyTuple_GET_ITEM(meta, 3), split_rows))
                 Py_RETURN_NONE;
+        } else {
+            PyObject *even = PyObject_GetAttr(m, g_even_name);
+            if (!even) return nullptr;
+            Py_DECREF(even);
+            if (even == Py_True) flags |= MACKO_SPMV_ROWS_EVEN;
         }
     }
     // own handles: another thread may drop the Python ones while the interpreter lock is released
@@ -85,7 +91,7 @@ PyObject *direct_multiply(PyObject *, PyObject *const *args, Py_ssize_t n_args)
     {
         struct NoGil { PyThreadState *s = PyEval_SaveThread(); ~NoGil() { PyEval_RestoreThread(s); } } no_gil;
         y = plan ? macko_torch::multiply_planned_cuda(v, d, r, rows, cols, pl, virtual_rows, segment, split_rows, x, true)
-                 : macko_torch::multiply_flags(v, d, r, rows, cols, x, frozen ? MACKO_SPMV_MATRIX_IMMUTABLE : 0u);
+                 : macko_torch::multiply_flags(v, d, r, rows, cols, x, flags);
     }
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
@@ -174,10 +180,11 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_direct", nullptr, -1, g_m
 
 PyMODINIT_FUNC PyInit__torch_direct()
 {
+    g_even_name = PyUnicode_InternFromString("even_rows");
     g_plan_name = PyUnicode_InternFromString("plan");
     g_plan_meta_name = PyUnicode_InternFromString("plan_meta");
     g_windows_name = PyUnicode_InternFromString("windows");
     g_windows_of_name = PyUnicode_InternFromString("windows_of");
     g_windows_batch_name = PyUnicode_InternFromString("windows_batch");
-    return g_plan_name && g_plan_meta_name && g_windows_name && g_windows_of_name && g_windows_batch_name ? PyModule_Create(&g_module) : nullptr;
+    return g_even_name && g_plan_name && g_plan_meta_name && g_windows_name && g_windows_of_name && g_windows_batch_name ? PyModule_Create(&g_module) : nullptr;
 }

@@ -8,7 +8,7 @@
 
 namespace macko_torch {
 
-// y[rows] for V[cols]. `flags`: MACKO_SPMV_MATRIX_IMMUTABLE or 0.
+// y[rows] for V[cols]. `flags`: MACKO_SPMV_MATRIX_IMMUTABLE, MACKO_SPMV_ROWS_EVEN.
 at::Tensor multiply_flags(const at::Tensor &values, const at::Tensor &deltas, const at::Tensor &ri, int64_t rows, int64_t cols,
                           const at::Tensor &V, uint32_t flags);
 
