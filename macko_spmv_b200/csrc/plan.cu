@@ -259,8 +259,8 @@ int macko_spmv_plan(const void *deltas, const int32_t *row_indices, int64_t rows
     st = current_device_info(&dev);
     if (st != MACKO_OK) return st;
     const bool x_fits = (kXPadFront + cols + kXPadBack) * 2 <= dev->max_smem_optin;
-    int lanes = 0, steps = 0;   // of the default launch
-    st = macko_spmv_shape(rows, cols, padded_count, dev->sm_count, &lanes, &steps);
+    int lanes = 0, threads = 0, tail = 0, rolling = 0;   // of the default launch (no plan is recommended for even rows)
+    st = macko_spmv_default_launch(rows, cols, padded_count, dev->sm_count, 0u, &lanes, &threads, &tail, &rolling);
     if (st != MACKO_OK) return st;
     const bool large = padded_count >= kPlanMinShare * plan_groups(cols);
     const bool long_row = (long long)info->longest_row >= kPlanMinChain * 8 * lanes;

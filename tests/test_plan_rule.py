@@ -57,6 +57,18 @@ def test_default_plans(rows, dense_rows, cols, planned, seg):
 
 
 @pytest.mark.gpu
+def test_chain_is_that_of_the_launch_that_would_run():
+    """Where one CTA per SM holds x the default launch has 1024 threads and a warp per row up to 5209 rows, `macko_spmv_shape` (two
+    CTAs of 512 threads) 16 lanes: 8000 elements are 31 sub-steps of a warp, too few for a plan, and would be 62 of 16 lanes."""
+    rows, cols = 3000, 60000
+    M = torch.zeros(rows, cols, dtype=torch.float16, device=DEV)
+    M[:, :800] = torch.randn(rows, 800, device=DEV).half()
+    M[70, :8000] = 0.5
+    frozen = macko_spmv.freeze(macko_spmv.compress(M))
+    assert frozen.plan_meta[2] == 8000 and frozen.plan is None
+
+
+@pytest.mark.gpu
 def test_no_plan_where_x_does_not_fit():
     """120 000 columns: the planned launch would refuse the matrix that `freeze` made."""
     rows, cols = 300, 120_000
