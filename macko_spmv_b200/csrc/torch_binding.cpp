@@ -327,21 +327,20 @@ int64_t count_stored(const at::Tensor &M, at::Tensor &ri, cudaStream_t stream)
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     TORCH_CHECK(cudaStreamIsCapturing(stream, &capture) == cudaSuccess, "cudaStreamIsCapturing failed");
     if (capture != cudaStreamCaptureStatusNone) return ri[rows].item<int32_t>();   // refuses, as any read-back in a capture
-    const char *what = M.element_size() == 1 ? "macko_compress_count_int8" : "macko_compress_count";
-    unsigned schedule = 0;
-    if (cudaGetDeviceFlags(&schedule) == cudaSuccess && (schedule & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync) {
-        // the program wants its threads to sleep while they wait for the GPU: no watching
-        check_status(M.element_size() == 1 ? macko_compress_count_int8(M.data_ptr(), rows, cols, ri.data_ptr<int32_t>(), stream)
-                                           : macko_compress_count(M.data_ptr(), rows, cols, ri.data_ptr<int32_t>(), stream), what);
-        return ri[rows].item<int32_t>();
-    }
     CountWord word(stream);
     volatile int32_t *total = word.value();
     check_status(macko_compress_count_total(M.data_ptr(), rows, cols, (int32_t)M.element_size(), ri.data_ptr<int32_t>(),
-                                            const_cast<int32_t *>(total), stream), what);
+                                            const_cast<int32_t *>(total), stream),
+                 M.element_size() == 1 ? "macko_compress_count_int8" : "macko_compress_count");
     for (unsigned spin = 1; *total < 0; ++spin) {
         if (spin % 4096u != 0u) continue;
-        const cudaError_t e = cudaStreamQuery(stream);
+        cudaError_t e = cudaErrorNotReady;
+        unsigned schedule = 0;
+        // a program that wants its threads to sleep while they wait for the GPU: no more watching after some microseconds
+        if (spin == 4096u && cudaGetDeviceFlags(&schedule) == cudaSuccess && (schedule & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync)
+            e = cudaStreamSynchronize(stream);
+        else
+            e = cudaStreamQuery(stream);
         if (e == cudaErrorNotReady) {
             (void)cudaGetLastError();
         } else {
