@@ -324,8 +324,6 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
     } else if (XS) {
         __half *xs = reinterpret_cast<__half *>(smem);
         const int n_total = kXPadFront + cols + kXPadBack;
-        // as ldg_fresh_u16; with the inline load the code around it came out 2 % slower for int8 values (11008x4096 14.9 / 14.65 us)
-        const volatile unsigned short *xv = reinterpret_cast<const volatile unsigned short *>(x);
 #pragma unroll 1
         for (int i = tid; i < kXPadFront; i += T) xs[i] = __ushort_as_half(0);
 #pragma unroll 1
@@ -340,18 +338,21 @@ spmv_kernel(const uint4 *__restrict__ values, const unsigned *__restrict__ delta
             for (int i = tid; i < n_vec; i += T)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + 16u * (unsigned)i), "l"(src0 + 16 * (size_t)i) : "memory");
 #pragma unroll 1
-            for (int i = (n_vec << 3) + tid; i < cols; i += T) xs[kXPadFront + i] = __ushort_as_half(xv[i]);
+            for (int i = (n_vec << 3) + tid; i < cols; i += T) xs[kXPadFront + i] = __ushort_as_half(ldg_fresh_u16(x + i));
             asm volatile("cp.async.commit_group;" ::: "memory");
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else {
+            // four loads in flight (one: 4096x4096 9.3 / 8.5 us, 1000x40000 21.5 / 18.2, int8 11008x4096 15.9 / 14.9). Planned: one,
+            // where x is aligned, four cost other code (32000x8192 48.4 / 49.1, 9600x5000 14.6 / 14.8, but 4992x10368 20.5 / 19.3)
+            constexpr int U = PLAN ? 1 : 4;
 #pragma unroll 1
-            for (int i = tid; i < cols; i += 4 * T) {   // four loads in flight (one: 4096x4096 9.3 / 9.1 us, 1000x40000 21.5 / 18.2)
-                unsigned short q[4] = {};
+            for (int i = tid; i < cols; i += U * T) {
+                unsigned short q[U] = {};
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (i + k * T < cols) q[k] = xv[i + k * T];
+                for (int k = 0; k < U; ++k)
+                    if (i + k * T < cols) q[k] = ldg_fresh_u16(x + i + k * T);
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
+                for (int k = 0; k < U; ++k)
                     if (i + k * T < cols) xs[kXPadFront + i + k * T] = __ushort_as_half(q[k]);
             }
         }
