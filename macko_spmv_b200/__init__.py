@@ -309,9 +309,9 @@ WINDOWED_BATCH_LIMIT = 64
 def _windows_batch(rows, cols, stored, windows) -> int:
     """The largest batch that goes over the column windows of a frozen matrix (`macko_spmm_fp16_windowed`), of 8 or more.
 
-    3..8 vectors always do, where the other choice is one pass of the one-kernel product: 11008x4096 d = 0.5 8 vectors 25.0
-    against 42.4 us, 4 vectors 20.7 / 27.0; 8192x8192 d = 0.3 24.2 / 38.8; 512x512 d = 0.5 5.5 / 6.5 and, the only loss, 3 vectors
-    4.4 / 4.2. Two vectors are level or behind (11008x4096 20.7 / 19.3, 4096x4096 d = 0.7 12.8 / 11.1).
+    3..8 vectors always do, where the other choice is one pass of the one-kernel product: 11008x4096 d = 0.5 8 vectors 25.1
+    against 41.2 us, 4 vectors 20.5 / 27.9; 8192x8192 d = 0.3 24.1 / 38.7; 512x512 d = 0.5 4.6 / 5.1 and, the only loss, 3 or 4 vectors
+    4.1 / 3.7. Two vectors are level or behind (11008x4096 20.3 / 20.0, 4096x4096 d = 0.7 12.6 / 10.9).
     Larger batches take every 8 vectors through the matrix, against one dense copy and a GEMM: the two models below, in us, fit 18
     shapes x 9..48 vectors with a standard deviation of 7 % and 21 %. 16 vectors, windows / copy: 4096x11008 d = 0.5 39.3 / 48.6,
     d = 0.2 24.8 / 42.6, 4096x4096 d = 0.7 23.4 / 21.3, 16384x4096 d = 0.9 92.6 / 77.3; 24 vectors: 4096x11008 d = 0.2 35.9 / 42.9,
@@ -378,9 +378,9 @@ def _dense_copy_pays(compressed_M, batch: int) -> bool:
 
     The line: ceil(batch / 8) passes at 1.3 TB/s of compressed bytes against the copy at 3.0 TB/s of compressed + dense bytes
     plus 19 us. The rates are those of an earlier decompressor; today's takes about 5 TB/s, so the line keeps to the passes where
-    the copy is already ahead. Measured (B200, us, passes / copy, * = chosen): 11008x4096 16 vectors d = 0.2 *47.5 / 39.4,
-    0.3 *59.7 / 42.5, 0.4 71.6 / *45.5, 0.5 85.4 / *47.6; 9 vectors 0.2 *32.8 / 39.4, 0.4 49.5 / *45.4; 4096x4096 16 vectors
-    0.5 *45.9 / 22.6, 0.7 52.3 / *24.9; 8192x8192 9 vectors 0.3 *54.1 / 73.1, 0.5 78.6 / *84.6, 16 vectors 0.3 *78.1 / 73.2."""
+    the copy is already ahead. Measured (B200, us, passes / copy, * = chosen): 11008x4096 16 vectors d = 0.2 *42.7 / 34.9,
+    0.3 *55.6 / 38.0, 0.4 68.8 / *41.6, 0.5 81.2 / *44.6; 9 vectors 0.2 *30.0 / 35.0, 0.4 47.6 / *41.3; 4096x4096 16 vectors
+    0.5 *38.3 / 20.2, 0.7 45.2 / *22.7; 8192x8192 9 vectors 0.3 *52.6 / 69.6, 0.5 77.2 / *79.7, 16 vectors 0.3 *75.7 / 69.7."""
     if batch <= 8 or compressed_M[0].dtype != torch.float16:
         return False
     stored_bytes = 2.5 * compressed_M[0].numel()

@@ -38,7 +38,8 @@ constexpr int kWin = 1024;       // fp16 slots of a warp's window of the dense r
 // registers: what lies inside is stored, the window leaves, and the rest goes to the next one. Pads and everything
 // else that is +-0 stay +0. The loads of the next step are issued before a step is scattered, and the second-level cache is asked for
 // the stream four steps ahead: with one step of loads alone a warp waits for memory in every step (4096x11008 at density 0.5 33.1 us
-// without). More loads in flight take registers that the fifth CTA needs.
+// without; at density 0.2 it matters less: a call of 11003x4093 24.6 us without, 23.7..24.3 with it). More loads in flight take
+// registers that the fifth CTA needs.
 // Bound by the load/store pipe (a 2-byte shared store of 32 elements takes 3.8 passes: random columns, random banks) and
 // close behind it HBM: 11003x4093 at density 0.2 (113 MB) in 21.5 us = 5.2 TB/s, 4096x11008 at 0.5 (146 MB) in 29.3 us
 // = 5.0 TB/s; a CTA per row takes 32.8 and 31.8 us. With the window flushed and cleared by the same 16-byte loads and

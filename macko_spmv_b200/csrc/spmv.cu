@@ -23,9 +23,10 @@
 //     fp16 x fp16 + fp32 fused multiply-add needs no conversions;
 //   * row boundaries that fall inside a unit are handled by masking that unit, only in warps
 //     that actually contain such a unit (one warp-wide reduction per iteration finds them);
-//   * the first matrix loads of every warp are in flight before x is staged, and, when the caller
-//     declares the matrix immutable, before the kernel waits for the previous kernel of the stream
-//     (programmatic dependent launch), so the first HBM round trip overlaps that kernel's tail;
+//   * when the caller declares the matrix immutable, the first matrix loads of every warp are in
+//     flight before the kernel waits for the previous kernel of the stream (programmatic dependent
+//     launch) and before x is staged, so the first HBM round trip overlaps that kernel's tail;
+//     otherwise they follow the wait and the staging;
 //   * a planned launch walks "virtual rows" (rows cut into segments of bounded length, sorted by
 //     length and dealt to the warps in serpentine order) from side metadata built once per matrix,
 //     which balances matrices with very uneven rows; the compressed buffers stay untouched.

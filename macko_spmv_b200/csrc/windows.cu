@@ -8,8 +8,8 @@
 // rows; the sums of a row over the windows are added by a second small kernel, in window order, so y is reproducible.
 //
 // Measured (B200, graph of products of rotating matrices, us, one kernel for all columns / windows): 8 vectors, 11008x4096 d = 0.5
-// 42.4 / 24.5, 4096x11008 d = 0.5 47.6 / 23.9, 16384x4096 d = 0.9 106.5 / 49.2, 4096x4096 d = 0.3 17.9 / 10.7, skewed 8192x28672 339.6 /
-// 111.8; 4 vectors, 11008x4096 27.0 / 20.7, 32000x4096 d = 0.5 64.4 / 44.6. What bounds it: the four passes of a 16-byte gather, 32 of
+// 41.2 / 25.1, 4096x11008 d = 0.5 43.5 / 24.1, 16384x4096 d = 0.9 107.3 / 51.3, 4096x4096 d = 0.3 14.8 / 10.2, skewed 8192x28672 325 /
+// 113; 4 vectors, 11008x4096 27.9 / 20.5, 32000x4096 d = 0.5 69.0 / 47.9. What bounds it: the four passes of a 16-byte gather, 32 of
 // about 44 passes of the load/store pipe per 8 x 32 elements, then the walk of the few blocks of rows that a warp gets.
 #include "common.cuh"
 #include "unit.cuh"
